@@ -14,7 +14,7 @@ OBJDIR = os.path.join(HERE, "_build")
 HEADER = os.path.join(ROOT, "include", "swdk.h")
 # source -> (extra flags, headers it includes)
 SOURCES = {
-    "swdk.cu": ([], ["swdk_core.cuh", "swdk_eigen.cuh"]),
+    "swdk.cu": ([], ["swdk_core.cuh", "swdk_coop.cuh", "swdk_eigen.cuh"]),
     "swdk_mlp.cu": ([], []),
     "swdk_fmst.cu": (["-fmad=false"], ["swdk_fmst_march.cuh"]),
     "swdk_lsmr.cu": ([], []),

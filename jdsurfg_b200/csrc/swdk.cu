@@ -7,7 +7,8 @@
 //              (surfdisp96.f:154-226); writes the REAL*4 layer model
 //              half-space first and column by column, so each secular
 //              evaluation streams its own column forward.
-//   k_roots  : one thread per (column, root chain); a chain is one
+//   k_roots_queue / k_roots_coop : one lane or a group of lanes per (column,
+//              root chain); a chain is one
 //              surfdisp96 call (wave, period list, modes 1..M) with the
 //              reference's retry (surfdisp.cpp:94-109); identical chains of
 //              different slot types are computed once.
@@ -583,16 +584,13 @@ __device__ __forceinline__ int ragged_find(const T* tab, int n, long long key, l
 // (chains in `order`, Rayleigh first, columns consecutive) whenever their
 // current chain is finished, so lanes stay busy while long chains run.
 // queue[0] is the next item; the launch covers the GPU once.
-// Dynamic shared memory of k_roots_queue and k_retry (128 threads): 55 KB,
+// Dynamic shared memory of k_roots_queue (128 threads): 55 KB,
 // above the 48 KB a launch gets without opting in; four blocks fit an SM's
 // 228 KB.
 constexpr size_t ROOTS_SMEM = 128 * (sizeof(ChainState) + sizeof(ChainParams) + sizeof(ChainIO));
 
 #ifndef SWDK_ROOTS_MINB
 #define SWDK_ROOTS_MINB 4  // 127 registers, no spill (shared memory allows 4 blocks too); 3 blocks measured slower
-#endif
-#ifndef SWDK_RETRY_MINB
-#define SWDK_RETRY_MINB 3  // retries, one record per warp: 168 registers (48 B of spill loads); 2 blocks (202 registers) measured 8 ms per step slower, 4 (128 registers, more spill) the same as 3
 #endif
 #ifndef SWDK_EIGEN_MINB
 #define SWDK_EIGEN_MINB 3  // Rayleigh passes: 168 registers, no spill (2: 183, 3: 171, 4: 180, 5: 227 ms of eigen per step)
@@ -734,6 +732,14 @@ __global__ void __launch_bounds__(128, SWDK_ROOTS_MINB) k_roots_queue(int ncol, 
   if (threadIdx.x < 5 && nevals && blk_ev[threadIdx.x]) atomicAdd(nevals + threadIdx.x, blk_ev[threadIdx.x]);
 }
 
+}  // namespace
+#include "swdk_coop.cuh"
+namespace {
+
+constexpr size_t RETRY_SMEM = ROOTS_SMEM + 4 * COOP_BUF;  // of k_retry: 68 KB, three blocks per SM
+#ifndef SWDK_RETRY_MINB
+#define SWDK_RETRY_MINB 3  // 2 blocks measured 8 ms per step slower, 4 (128 registers, spills) the same as 3
+#endif
 // One round of the getsol scan (surfdisp96.f:452-486) by a whole warp.  The
 // chain machine has just asked for f at the next scan point c2 = s.creq (the
 // point counted in s.nscan).  Lane j evaluates the point j steps further on,
@@ -781,8 +787,8 @@ __device__ int retry_scan(ChainState& s, const ChainParams& P, const LayerView& 
 // record per warp.  A retry re-runs the reference's search for one period
 // from its start value, a scan of often several hundred dc steps; the warp's
 // lanes hold the same chain state and take the scan 32 points at a time
-// (retry_scan), the other requests (start point, refinement) are evaluated
-// by all lanes alike.
+// (retry_scan); the other requests (start point, refinement) are evaluated by
+// the lanes together, 32 layers at a time (coop_rayleigh, coop_love).
 __global__ void __launch_bounds__(128, SWDK_RETRY_MINB) k_retry(int ncol, const int* __restrict__ order,
                                                                const ChainDesc* __restrict__ chains,
                                                                const double* __restrict__ periods,
@@ -797,12 +803,13 @@ __global__ void __launch_bounds__(128, SWDK_RETRY_MINB) k_retry(int ncol, const 
                                                                unsigned long long* __restrict__ nevals, RaggedMap rg,
                                                                const float4* __restrict__ nodes,
                                                                const DepthLayer* __restrict__ dl) {
-  // dynamic shared memory (ROOTS_SMEM): one copy of the warp's chain state,
-  // parameters and output addressing per lane
+  // dynamic shared memory (RETRY_SMEM): one copy of the warp's chain state,
+  // parameters and output addressing per lane, and the warps' layer rows
   extern __shared__ __align__(16) unsigned char roots_smem[];
   ChainState* sst = reinterpret_cast<ChainState*>(roots_smem);
   ChainParams* sprm = reinterpret_cast<ChainParams*>(sst + 128);
   ChainIO* sio = reinterpret_cast<ChainIO*>(sprm + 128);
+  double* rows = reinterpret_cast<double*>(roots_smem + ROOTS_SMEM + (threadIdx.x >> 5) * COOP_BUF);
   __shared__ unsigned long long blk_ev[3];  // evaluations, Rayleigh and Love layer evaluations
   if (threadIdx.x < 3) blk_ev[threadIdx.x] = 0ull;
   __syncthreads();
@@ -872,7 +879,13 @@ __global__ void __launch_bounds__(128, SWDK_RETRY_MINB) k_retry(int ncol, const 
         nev += retry_scan(s, P, V, lane);
         continue;
       }
-      s.last = secular_fast(V, P.iwave, P.refine, s.omega / s.creq, s.omega);
+      const double om = s.omega, wv = om / s.creq;
+      if (P.iwave == 2)
+        s.last = P.refine == 0 ? coop_rayleigh<1>(true, V, wv, om, 32, lane, rows)
+                               : coop_rayleigh<4>(true, V, wv, om, 32, lane, rows);
+      else
+        s.last = P.refine == 0 ? coop_love<1>(true, V, wv, om, 32, lane, rows)
+                               : coop_love<4>(true, V, wv, om, 32, lane, rows);
       nev++;
       s.phase = s.next;
     }
@@ -888,15 +901,81 @@ __global__ void __launch_bounds__(128, SWDK_RETRY_MINB) k_retry(int ncol, const 
   if (threadIdx.x == 0 && nevals && blk_ev[0]) atomicAdd(nevals + EV_BASE + EV_RETRY, blk_ev[0]);
 }
 
-// Opts k_roots_queue and k_retry in to ROOTS_SMEM on the current device and
-// returns k_roots_queue's resident blocks per SM.
+// Opts the root kernels in to their dynamic shared memory on the current
+// device and returns k_roots_queue's resident blocks per SM.
 cudaError_t roots_occupancy(int* per) {
   cudaError_t e = cudaFuncSetAttribute(k_roots_queue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROOTS_SMEM);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_retry, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROOTS_SMEM);
+  const int cs = (int)coop_smem(COOP_MIN_G);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_roots_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_retry, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RETRY_SMEM);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, k_roots_queue, 128, ROOTS_SMEM);
   return e;
 }
 
+// Lanes per chain (1: k_roots_queue) for a root search of nitems chains.  One
+// lane each needs about 75 000 chains to fill the GPU; a call's time is then
+// the longest chain's, about 30 ms whatever the size.  More lanes shorten the
+// chain and cost throughput (the products run in every lane of a group; groups
+// of one warp that evaluate different numbers of velocities take turns).  ms of
+// the search with 1 / 4 / 8 / 32 lanes, 20 periods of 41 nodes, Rayleigh:
+//   1188 chains 24.6 / 10.0 / 9.2 / 4.4     3840  29.5 / 18.7 / 12.6 / 23.2
+//   1500        28.7 / 17.7 / 10.3 / 10.2   10000 36.3 / 23.9 / 33.6 / 42.2
+//   2400        28.7 / 18.7 / 11.7 / 16.0   16384 27.3 / 27.8 / 38.2 / 92.7
+// (16 lanes lie between 8 and 32 and lead nowhere).  The lines are a device's
+// of 148 SMs and move with its size.
+int coop_lanes(long long nitems, int nsm) {
+  const long long n = nitems * 148 / std::max(1, nsm);
+  return n <= 1500 ? 32 : n <= 6000 ? 8 : n <= 14000 ? 4 : 1;
+}
+
+struct RootsCall {
+  int ncol;
+  long long nitems;
+  const int* order;
+  const ChainDesc* chains;
+  const double* periods;
+  const float4 *layR, *layL;
+  const ColInfo* info;
+  int refine;
+  double rtol;
+  int sngl;
+  double* croot;
+  int32_t* cstat;
+  unsigned int* queue;  // zeroed
+  const float2* prop;
+  int2* retry_list;
+  unsigned int* rctr;  // {records, next record}, zeroed
+  unsigned int rcap;
+  unsigned long long* nevals;
+  RaggedMap rg;
+  const float4* nodes;
+  const DepthLayer* dl;
+};
+
+// the root search and the retries of its failed periods; rblocks: blocks of
+// k_roots_queue; tuned: that count was asked for (swdk_autotune, or the
+// caller's configuration), so the one-lane kernel runs
+cudaError_t launch_roots(const RootsCall& c, int rblocks, int nsm, bool tuned, cudaStream_t st) {
+  const int G = tuned ? 1 : coop_lanes(c.nitems, nsm);
+  if (G > 1) {
+    const long long need = (c.nitems * G + 127) / 128;
+    k_roots_coop<<<(unsigned)std::max(1LL, std::min<long long>(need, 3LL * nsm)), 128, coop_smem(G), st>>>(
+        c.ncol, (int)c.nitems, G, c.order, c.chains, c.periods, c.layR, c.layL, c.info, c.refine, c.rtol, c.sngl,
+        RETRY_DEFERRED, c.croot, c.cstat, c.queue, c.prop, c.retry_list, c.rctr, c.rcap, c.nevals, c.rg, c.nodes,
+        c.dl);
+  } else {
+    k_roots_queue<<<(unsigned)std::max(1LL, std::min<long long>(rblocks, (c.nitems + 127) / 128)), 128, ROOTS_SMEM,
+                    st>>>(c.ncol, (int)c.nitems, c.order, c.chains, c.periods, c.layR, c.layL, c.info, c.refine,
+                          c.rtol, c.sngl, RETRY_DEFERRED, c.croot, c.cstat, c.queue, c.prop, c.retry_list, c.rctr,
+                          c.rcap, c.nevals, c.rg, c.nodes, c.dl);
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  k_retry<<<(unsigned)rblocks, 128, RETRY_SMEM, st>>>(c.ncol, c.order, c.chains, c.periods, c.layR, c.layL, c.info,
+                                                      c.refine, c.rtol, c.sngl, c.croot, c.cstat, c.retry_list, c.rctr,
+                                                      c.rcap, c.rctr + 1, c.nevals, c.rg, c.nodes, c.dl);
+  return cudaGetLastError();
+}
 
 // recip() on an array (its accuracy test)
 __global__ void k_recip(int n, const double* __restrict__ x, double* __restrict__ r) {
@@ -1333,7 +1412,7 @@ struct swdk_ctx {
   Plan plan[2];  // 0: get_1d_kernel, 1: get_2d_map
   DevBuf layR, layL, lay0, info, chainrule, croot, cstat, nevals, depth_d, ierr, queue;
   DevBuf nodes, dltab;  // grid nodes and the depth grid's flattening (node-source root search)
-  int roots_blocks = 0;
+  int roots_blocks = 0, nsm = 148;
   DevBuf in_vs, in_vp, in_rho, out_vc, out_vout, out_kernel, out_status, in_misc;
   // learned bracket proposals
   swdk_mlp* net[2] = {nullptr, nullptr};  // 0: Rayleigh, 1: Love
@@ -1643,6 +1722,7 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     CK(roots_occupancy(&per));
+    ctx->nsm = nsm;
     ctx->roots_blocks = std::max(1, nsm * std::max(1, per));
   }
   const int nitems = (int)P.chains.size() * ncol;
@@ -1654,21 +1734,30 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
   CK(cudaMemsetAsync(ctx->retry_ctr.p, 0, 2 * sizeof(unsigned int), st));
   unsigned int* rctr = ctx->retry_ctr.as<unsigned int>();
   ctx->launches += 2;
-  k_roots_queue<<<std::min(rblocks, (nitems + 127) / 128), 128, ROOTS_SMEM, st>>>(
-      ncol, nitems, P.d_order.as<int>(), P.d_chains.as<ChainDesc>(), P.d_periods.as<double>(), ctx->layR.as<float4>(),
-      ctx->layL.as<float4>(), ctx->info.as<ColInfo>(), ctx->cfg.refine, ctx->cfg.rtol, ctx->cfg.sngl, RETRY_DEFERRED,
-      ctx->croot.as<double>(), ctx->cstat.as<int32_t>(), ctx->queue.as<unsigned int>(),
-      useprop ? ctx->prop.as<float2>() : nullptr, ctx->retry_list.as<int2>(), rctr, rcap,
-      ctx->nevals.as<unsigned long long>(), RaggedMap{nullptr, nullptr, 0, Lmax},
-      use_nodes ? ctx->nodes.as<float4>() : nullptr, ctx->dltab.as<DepthLayer>());
-  CK(cudaGetLastError());
-  k_retry<<<rblocks, 128, ROOTS_SMEM, st>>>(ncol, P.d_order.as<int>(), P.d_chains.as<ChainDesc>(), P.d_periods.as<double>(),
-                                   ctx->layR.as<float4>(), ctx->layL.as<float4>(), ctx->info.as<ColInfo>(),
-                                   ctx->cfg.refine, ctx->cfg.rtol, ctx->cfg.sngl, ctx->croot.as<double>(),
-                                   ctx->cstat.as<int32_t>(), ctx->retry_list.as<int2>(), rctr, rcap, rctr + 1,
-                                   ctx->nevals.as<unsigned long long>(), RaggedMap{nullptr, nullptr, 0, Lmax},
-                                   use_nodes ? ctx->nodes.as<float4>() : nullptr, ctx->dltab.as<DepthLayer>());
-  CK(cudaGetLastError());
+  RootsCall rc;
+  rc.ncol = ncol;
+  rc.nitems = nitems;
+  rc.order = P.d_order.as<int>();
+  rc.chains = P.d_chains.as<ChainDesc>();
+  rc.periods = P.d_periods.as<double>();
+  rc.layR = ctx->layR.as<float4>();
+  rc.layL = ctx->layL.as<float4>();
+  rc.info = ctx->info.as<ColInfo>();
+  rc.refine = ctx->cfg.refine;
+  rc.rtol = ctx->cfg.rtol;
+  rc.sngl = ctx->cfg.sngl;
+  rc.croot = ctx->croot.as<double>();
+  rc.cstat = ctx->cstat.as<int32_t>();
+  rc.queue = ctx->queue.as<unsigned int>();
+  rc.prop = useprop ? ctx->prop.as<float2>() : nullptr;
+  rc.retry_list = ctx->retry_list.as<int2>();
+  rc.rctr = rctr;
+  rc.rcap = rcap;
+  rc.nevals = ctx->nevals.as<unsigned long long>();
+  rc.rg = RaggedMap{nullptr, nullptr, 0, Lmax};
+  rc.nodes = use_nodes ? ctx->nodes.as<float4>() : nullptr;
+  rc.dl = ctx->dltab.as<DepthLayer>();
+  CK(launch_roots(rc, rblocks, ctx->nsm, ctx->cfg.block_roots > 0, st));
   if (timing) CK(cudaEventRecord(ctx->ev[2], st));
   if (!roots_only) {
     if (!ho) {
@@ -2456,7 +2545,7 @@ struct swdk_ragged {
   std::vector<double> periods;
   std::vector<SlotDesc> slots;
   long long nitems = 0, ncol_tot = 0, lay_tot = 0, crs_tot = 0, root_tot = 0, slots_tot = 0;
-  int maxL = 0, maxnz = 0, roots_blocks = 0;
+  int maxL = 0, maxnz = 0, roots_blocks = 0, nsm = 148;
   bool useprop = false;
   DevBuf d_models, d_blocks, d_eb[4], d_chains, d_periods, d_slots;
   DevBuf layR, layL, lay0, info, chainrule, croot, cstat, prop, nodefeat, retry_list, retry_ctr, queue, nevals;
@@ -2524,23 +2613,31 @@ int ragged_enqueue(swdk_ragged* R, cudaStream_t st, bool timing) {
   const RaggedMap rg{R->d_blocks.as<RBlock>(), R->d_models.as<RModel>(), (int)R->blocks.size(), 0};
   const unsigned int rcap = (unsigned int)std::min<long long>(R->root_tot, 0x7fffffffLL);
   unsigned int* rctr = R->retry_ctr.as<unsigned int>();
-  const long long grid = std::min<long long>(R->roots_blocks, (R->nitems + 127) / 128);
   R->launches += 2;
-  k_roots_queue<<<(unsigned)std::max(1LL, grid), 128, ROOTS_SMEM, st>>>(
-      0, (int)R->nitems, nullptr, R->d_chains.as<ChainDesc>(), R->d_periods.as<double>(), R->layR.as<float4>(),
-      R->layL.as<float4>(), R->info.as<ColInfo>(), cfg.refine, cfg.rtol, cfg.sngl, RETRY_DEFERRED,
-      R->croot.as<double>(), R->cstat.as<int32_t>(), R->queue.as<unsigned int>(),
-      R->useprop ? R->prop.as<float2>() : nullptr, R->retry_list.as<int2>(), rctr, rcap,
-      R->nevals.as<unsigned long long>(), rg, use_nodes ? R->nodes.as<float4>() : nullptr,
-      R->dltab.as<DepthLayer>());
-  CK(cudaGetLastError());
-  k_retry<<<R->roots_blocks, 128, ROOTS_SMEM, st>>>(0, nullptr, R->d_chains.as<ChainDesc>(), R->d_periods.as<double>(),
-                                           R->layR.as<float4>(), R->layL.as<float4>(), R->info.as<ColInfo>(),
-                                           cfg.refine, cfg.rtol, cfg.sngl, R->croot.as<double>(),
-                                           R->cstat.as<int32_t>(), R->retry_list.as<int2>(), rctr, rcap, rctr + 1,
-                                           R->nevals.as<unsigned long long>(), rg,
-                                           use_nodes ? R->nodes.as<float4>() : nullptr, R->dltab.as<DepthLayer>());
-  CK(cudaGetLastError());
+  RootsCall rc;
+  rc.ncol = 0;
+  rc.nitems = R->nitems;
+  rc.order = nullptr;
+  rc.chains = R->d_chains.as<ChainDesc>();
+  rc.periods = R->d_periods.as<double>();
+  rc.layR = R->layR.as<float4>();
+  rc.layL = R->layL.as<float4>();
+  rc.info = R->info.as<ColInfo>();
+  rc.refine = cfg.refine;
+  rc.rtol = cfg.rtol;
+  rc.sngl = cfg.sngl;
+  rc.croot = R->croot.as<double>();
+  rc.cstat = R->cstat.as<int32_t>();
+  rc.queue = R->queue.as<unsigned int>();
+  rc.prop = R->useprop ? R->prop.as<float2>() : nullptr;
+  rc.retry_list = R->retry_list.as<int2>();
+  rc.rctr = rctr;
+  rc.rcap = rcap;
+  rc.nevals = R->nevals.as<unsigned long long>();
+  rc.rg = rg;
+  rc.nodes = use_nodes ? R->nodes.as<float4>() : nullptr;
+  rc.dl = R->dltab.as<DepthLayer>();
+  CK(launch_roots(rc, R->roots_blocks, R->nsm, false, st));
   if (timing) CK(cudaEventRecord(R->ev[2], st));
   if (R->path != 2) {
     using EigR = void (*)(const REBlock*, int, const RModel*, const float4*, const ColInfo*, const float2*,

@@ -431,88 +431,184 @@ struct LayerCoef {
   double a0, cpcq, cpy, cpz, cqw, cqx, xy, xz, wy, wz, gam, gammk, rho, irho;
 };
 
+// Sums of products in the Rayleigh evaluation are written with the rounding
+// they have: xmul / xadd round, xfma rounds once.  Left to the compiler, the
+// same expressions were contracted differently in the one-lane loop and in
+// the group kernel, and unrounded roots differed by 1e-15 km/s; written out,
+// every kernel gives the same bits, whatever surrounds the code.  (On the
+// host, for the test harnesses, plain multiplications and additions.)
+#ifdef __CUDA_ARCH__
+SWDK_HD double xmul(double a, double b) { return a * b; }
+SWDK_HD double xadd(double a, double b) { return __dadd_rn(a, b); }
+SWDK_HD double xfma(double a, double b, double c) { return fma(a, b, c); }
+#else
+SWDK_HD double xmul(double a, double b) { return a * b; }
+SWDK_HD double xadd(double a, double b) { return a + b; }
+SWDK_HD double xfma(double a, double b, double c) { return a * b + c; }
+#endif
+
 SWDK_HD LayerCoef layer_coef(const float4 ly, double wvno, double wvno2, double omega, double iom) {
   LayerCoef k;
   k.irho = recip((double)ly.w);
   const double dpth = ly.x;
   k.rho = ly.w;
-  const double xka = omega * recip((double)ly.y), xkb = omega * recip((double)ly.z);
-  const double t = (double)ly.z * iom;
-  k.gammk = 2.0 * t * t;
-  k.gam = k.gammk * wvno2;
-  const double Xa = (wvno + xka) * fabs(wvno - xka);
-  const double Xb = (wvno + xkb) * fabs(wvno - xkb);
+  const double xka = xmul(omega, recip((double)ly.y)), xkb = xmul(omega, recip((double)ly.z));
+  const double t = xmul((double)ly.z, iom);
+  k.gammk = xmul(2.0 * t, t);
+  k.gam = xmul(k.gammk, wvno2);
+  const double Xa = xmul(xadd(wvno, xka), fabs(xadd(wvno, -xka)));
+  const double Xb = xmul(xadd(wvno, xkb), fabs(xadd(wvno, -xkb)));
   // var (surfdisp96.f:901-1018); ep = exp(-pex), eq = exp(-sex)
+  // The vertical wavenumbers and their reciprocals are the same expressions in
+  // both kinds of layer and stand before the branches: lanes of a warp that
+  // differ in kind evaluate them once (0 * inf = NaN where X = 0 is not used).
   double w, x, cosp, y, z, cosq, ep = 1.0, eq = 1.0, pex = 0.0, sex = 0.0;
+  const double ira = rsqrt(Xa), irb = rsqrt(Xb), rva = xmul(Xa, ira), rvb = xmul(Xb, irb);
+  const double p = xmul(rva, dpth), q = xmul(rvb, dpth);
+  if (wvno < xka) {
+    double sp, cp;
+    sincos(p, &sp, &cp);
+    w = xmul(sp, ira); x = xmul(-rva, sp); cosp = cp;
+  } else if (wvno == xka) {
+    cosp = 1.0; w = dpth; x = 0.0;
+  } else {
+    pex = p;
+    ep = (p < 60.0) ? exp(-p) : 0.0;
+    const double fac = (p < 16.0) ? xmul(ep, ep) : 0.0;
+    cosp = xmul(xadd(1.0, fac), 0.5);
+    const double sp = xmul(xadd(1.0, -fac), 0.5);
+    w = xmul(sp, ira); x = xmul(rva, sp);
+  }
+  if (wvno < xkb) {
+    double sq, cq;
+    sincos(q, &sq, &cq);
+    y = xmul(sq, irb); z = xmul(-rvb, sq); cosq = cq;
+  } else if (wvno == xkb) {
+    cosq = 1.0; y = dpth; z = 0.0;
+  } else {
+    sex = q;
+    eq = (q < 60.0) ? exp(-q) : 0.0;
+    const double fac = (q < 16.0) ? xmul(eq, eq) : 0.0;
+    cosq = xmul(xadd(1.0, fac), 0.5);
+    const double sq = xmul(xadd(1.0, -fac), 0.5);
+    y = xmul(sq, irb); z = xmul(rvb, sq);
+  }
+  // a0 = exp(-(pex+sex)) when pex+sex < 60 (both factors then below 60)
+  k.a0 = (xadd(pex, sex) < 60.0) ? xmul(ep, eq) : 0.0;
+  k.cpcq = xmul(cosp, cosq); k.cpy = xmul(cosp, y); k.cpz = xmul(cosp, z);
+  k.cqw = xmul(cosq, w); k.cqx = xmul(cosq, x);
+  k.xy = xmul(x, y); k.xz = xmul(x, z); k.wy = xmul(w, y); k.wz = xmul(w, z);
+  return k;
+}
+
+// The entries of a layer's Dunkin matrix (surfdisp96.f:1051-1095) that its
+// product uses: rows 1:(c11..c15) 2:(c21,c22,c23,c24,c14) 3:(c31..c35)
+// 4:(c41,c42,c43,c22,c12) 5:(c51,c41,c53,c21,c11)
+struct Dunkin {
+  double c11, c12, c13, c14, c15, c21, c22, c23, c24, c31, c32, c33, c34, c35, c41, c42, c43, c51, c53;
+};
+
+SWDK_HD Dunkin dunkin_entries(const LayerCoef& k, double wvno2) {
+  const double gam = k.gam, gammk = k.gammk, rho = k.rho, irho = k.irho;
+  const double gamm1 = xadd(gam, -1.0);
+  const double twgm1 = xadd(gam, gamm1), gmgmk = xmul(gam, gammk), gmgm1 = xmul(gam, gamm1),
+               gm1sq = xmul(gamm1, gamm1);
+  const double rho2 = xmul(rho, rho), irho2 = xmul(irho, irho);
+  const double a0pq = xadd(k.a0, -k.cpcq);
+  Dunkin d;
+  d.c11 = xfma(-xmul(wvno2, gm1sq), k.wy, xfma(-gmgmk, k.xz, xfma(-xmul(2.0, gmgm1), a0pq, k.cpcq)));
+  d.c12 = xmul(xfma(wvno2, k.cpy, -k.cqx), irho);
+  d.c13 = -xmul(xfma(xmul(wvno2, gamm1), k.wy, xfma(gammk, k.xz, xmul(twgm1, a0pq))), irho);
+  d.c14 = xmul(xfma(-wvno2, k.cqw, k.cpz), irho);
+  d.c15 = -xmul(xfma(xmul(wvno2, wvno2), k.wy, xfma(xmul(2.0, wvno2), a0pq, k.xz)), irho2);
+  d.c21 = xmul(xfma(gmgmk, k.cpz, -xmul(gm1sq, k.cqw)), rho);
+  d.c22 = k.cpcq;
+  d.c23 = xfma(gammk, k.cpz, -xmul(gamm1, k.cqw));
+  d.c24 = -k.wz;
+  d.c41 = xmul(xfma(gm1sq, k.cpy, -xmul(gmgmk, k.cqx)), rho);
+  d.c42 = -k.xy;
+  d.c43 = xfma(gamm1, k.cpy, -xmul(gammk, k.cqx));
+  const double g2 = xmul(gmgmk, gmgmk), m4 = xmul(gm1sq, gm1sq), gkm1 = xmul(gammk, gamm1);
+  d.c51 = -xmul(xfma(m4, k.wy, xfma(g2, k.xz, xmul(xmul(xmul(2.0, gmgmk), gm1sq), a0pq))), rho2);
+  d.c53 = -xmul(xfma(xmul(gamm1, gm1sq), k.wy, xfma(xmul(gmgmk, gammk), k.xz, xmul(xmul(gkm1, twgm1), a0pq))), rho);
+  const double tt = -2.0 * wvno2;
+  d.c31 = xmul(tt, d.c53); d.c32 = xmul(tt, d.c43); d.c33 = xfma(2.0, xadd(k.cpcq, -d.c11), k.a0);
+  d.c34 = xmul(tt, d.c23); d.c35 = xmul(tt, d.c13);
+  return d;
+}
+
+// e <- e * d (dltar4's product, surfdisp96.f:868-876)
+SWDK_HD void dunkin_product(const Dunkin& d, double& e0, double& e1, double& e2, double& e3, double& e4) {
+  const double f0 = xfma(e4, d.c51, xfma(e3, d.c41, xfma(e2, d.c31, xfma(e1, d.c21, xmul(e0, d.c11)))));
+  const double f1 = xfma(e4, d.c41, xfma(e3, d.c42, xfma(e2, d.c32, xfma(e1, d.c22, xmul(e0, d.c12)))));
+  const double f2 = xfma(e4, d.c53, xfma(e3, d.c43, xfma(e2, d.c33, xfma(e1, d.c23, xmul(e0, d.c13)))));
+  const double f3 = xfma(e4, d.c21, xfma(e3, d.c22, xfma(e2, d.c34, xfma(e0, d.c14, xmul(e1, d.c24)))));
+  const double f4 = xfma(e4, d.c11, xfma(e3, d.c12, xfma(e2, d.c35, xfma(e1, d.c14, xmul(e0, d.c15)))));
+  e0 = f0; e1 = f1; e2 = f2; e3 = f3; e4 = f4;
+}
+
+SWDK_HD void apply_dunkin(const LayerCoef& k, double wvno2, double& e0, double& e1, double& e2, double& e3,
+                          double& e4) {
+  dunkin_product(dunkin_entries(k, wvno2), e0, e1, e2, e3, e4);
+}
+
+// the propagated vector of dltar4: its start at the half-space, the
+// max-normalisation (surfdisp96.f:1022-1047; NORM 1 divides, larger NORM
+// multiplies by the reciprocal) and the value under a fluid top layer
+struct RayVec {
+  double e0, e1, e2, e3, e4;
+};
+
+SWDK_HD RayVec rayleigh_start(const float4 h, double wvno, double wvno2, double omega, double iom) {
+  const double ia = recip((double)h.y), xkb = xmul(omega, recip((double)h.z));
+  const double ra = sqrt(xmul(xfma(omega, ia, wvno), fabs(xfma(-omega, ia, wvno))));
+  const double rb = sqrt(xmul(xadd(wvno, xkb), fabs(xadd(wvno, -xkb))));
+  const double t = xmul((double)h.z, iom);
+  const double gammk = xmul(2.0 * t, t);
+  const double gam = xmul(gammk, wvno2);
+  const double gamm1 = xadd(gam, -1.0);
+  const double rho1 = h.w;
+  RayVec e;
+  e.e0 = xmul(xmul(rho1, rho1), xfma(gamm1, gamm1, -xmul(xmul(xmul(gam, gammk), ra), rb)));
+  e.e1 = xmul(-rho1, ra);
+  e.e2 = xmul(rho1, xfma(-xmul(gammk, ra), rb, gamm1));
+  e.e3 = xmul(rho1, rb);
+  e.e4 = xfma(-ra, rb, wvno2);
+  return e;
+}
+
+template <int NORM>
+SWDK_HD void rayleigh_norm(double& e0, double& e1, double& e2, double& e3, double& e4) {
+  double t1 = fmax(fmax(fmax(fabs(e0), fabs(e1)), fmax(fabs(e2), fabs(e3))), fabs(e4));
+  if (t1 < 1.e-40) t1 = 1.0;
+  if (NORM == 1) {
+    e0 = e0 / t1; e1 = e1 / t1; e2 = e2 / t1; e3 = e3 / t1; e4 = e4 / t1;
+  } else {
+    const double it1 = 1.0 / t1;
+    e0 *= it1; e1 *= it1; e2 *= it1; e3 *= it1; e4 *= it1;
+  }
+}
+
+SWDK_HD double rayleigh_fluid_top(const float4 ly, double wvno, double omega, double e0, double e1) {
+  const double dpth = ly.x, rho = ly.w;
+  const double xka = omega * recip((double)ly.y);
+  const double Xa = (wvno + xka) * fabs(wvno - xka);
+  double w, cosp;
   if (wvno < xka) {
     const double ir = rsqrt(Xa), r = Xa * ir;
     double sp, cp;
     sincos(r * dpth, &sp, &cp);
-    w = sp * ir; x = -r * sp; cosp = cp;
+    w = sp * ir; cosp = cp;
   } else if (wvno == xka) {
-    cosp = 1.0; w = dpth; x = 0.0;
+    cosp = 1.0; w = dpth;
   } else {
     const double ir = rsqrt(Xa), r = Xa * ir, p = r * dpth;
-    pex = p;
-    ep = (p < 60.0) ? exp(-p) : 0.0;
-    const double fac = (p < 16.0) ? ep * ep : 0.0;
+    const double fac = (p < 16.0) ? exp(-2.0 * p) : 0.0;
     cosp = (1.0 + fac) * 0.5;
-    const double sp = (1.0 - fac) * 0.5;
-    w = sp * ir; x = r * sp;
+    w = ((1.0 - fac) * 0.5) * ir;
   }
-  if (wvno < xkb) {
-    const double ir = rsqrt(Xb), r = Xb * ir;
-    double sq, cq;
-    sincos(r * dpth, &sq, &cq);
-    y = sq * ir; z = -r * sq; cosq = cq;
-  } else if (wvno == xkb) {
-    cosq = 1.0; y = dpth; z = 0.0;
-  } else {
-    const double ir = rsqrt(Xb), r = Xb * ir, q = r * dpth;
-    sex = q;
-    eq = (q < 60.0) ? exp(-q) : 0.0;
-    const double fac = (q < 16.0) ? eq * eq : 0.0;
-    cosq = (1.0 + fac) * 0.5;
-    const double sq = (1.0 - fac) * 0.5;
-    y = sq * ir; z = r * sq;
-  }
-  // a0 = exp(-(pex+sex)) when pex+sex < 60 (both factors then below 60)
-  k.a0 = (pex + sex < 60.0) ? ep * eq : 0.0;
-  k.cpcq = cosp * cosq; k.cpy = cosp * y; k.cpz = cosp * z; k.cqw = cosq * w; k.cqx = cosq * x;
-  k.xy = x * y; k.xz = x * z; k.wy = w * y; k.wz = w * z;
-  return k;
-}
-
-// e <- e * Dunkin(k) (surfdisp96.f:1051-1095 and dltar4's product)
-SWDK_HD void apply_dunkin(const LayerCoef& k, double wvno2, double& e0, double& e1, double& e2, double& e3,
-                          double& e4) {
-  const double gam = k.gam, gammk = k.gammk, rho = k.rho, irho = k.irho;
-  const double gamm1 = gam - 1.0;
-  const double twgm1 = gam + gamm1, gmgmk = gam * gammk, gmgm1 = gam * gamm1, gm1sq = gamm1 * gamm1;
-  const double rho2 = rho * rho, irho2 = irho * irho;
-  const double a0pq = k.a0 - k.cpcq;
-  const double c11 = k.cpcq - 2.0 * gmgm1 * a0pq - gmgmk * k.xz - wvno2 * gm1sq * k.wy;
-  const double c12 = (wvno2 * k.cpy - k.cqx) * irho;
-  const double c13 = -(twgm1 * a0pq + gammk * k.xz + wvno2 * gamm1 * k.wy) * irho;
-  const double c14 = (k.cpz - wvno2 * k.cqw) * irho;
-  const double c15 = -(2.0 * wvno2 * a0pq + k.xz + wvno2 * wvno2 * k.wy) * irho2;
-  const double c21 = (gmgmk * k.cpz - gm1sq * k.cqw) * rho;
-  const double c22 = k.cpcq;
-  const double c23 = gammk * k.cpz - gamm1 * k.cqw;
-  const double c24 = -k.wz;
-  const double c41 = (gm1sq * k.cpy - gmgmk * k.cqx) * rho;
-  const double c42 = -k.xy;
-  const double c43 = gamm1 * k.cpy - gammk * k.cqx;
-  const double c51 = -(2.0 * gmgmk * gm1sq * a0pq + gmgmk * gmgmk * k.xz + gm1sq * gm1sq * k.wy) * rho2;
-  const double c53 = -(gammk * gamm1 * twgm1 * a0pq + gam * gammk * gammk * k.xz + gamm1 * gm1sq * k.wy) * rho;
-  const double tt = -2.0 * wvno2;
-  const double c31 = tt * c53, c32 = tt * c43, c33 = k.a0 + 2.0 * (k.cpcq - c11), c34 = tt * c23, c35 = tt * c13;
-  const double f0 = e0 * c11 + e1 * c21 + e2 * c31 + e3 * c41 + e4 * c51;
-  const double f1 = e0 * c12 + e1 * c22 + e2 * c32 + e3 * c42 + e4 * c41;
-  const double f2 = e0 * c13 + e1 * c23 + e2 * c33 + e3 * c43 + e4 * c53;
-  const double f3 = e0 * c14 + e1 * c24 + e2 * c34 + e3 * c22 + e4 * c21;
-  const double f4 = e0 * c15 + e1 * c14 + e2 * c35 + e3 * c12 + e4 * c11;
-  e0 = f0; e1 = f1; e2 = f2; e3 = f3; e4 = f4;
+  const double w0 = -rho * w;
+  return cosp * e0 + w0 * e1;
 }
 
 template <int NORM, bool NODES>
@@ -522,34 +618,15 @@ SWDK_HDI double dltar4_fast(const LayerView& V, double wvno, double omga) {
   const double wvno2 = wvno * wvno;
   const double iom = 1.0 / omega;
   const int hs = V.L - 1;  // the half-space
-  const float4 h = V.layer(hs);
-  double xka = omega * recip((double)h.y), xkb = omega * recip((double)h.z);
-  const double ra = sqrt((wvno + xka) * fabs(wvno - xka));
-  const double rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
-  const double t = (double)h.z * iom;
-  const double gammk = 2.0 * t * t;
-  const double gam = gammk * wvno2;
-  const double gamm1 = gam - 1.0;
-  const double rho1 = h.w;
-  double e0 = rho1 * rho1 * (gamm1 * gamm1 - gam * gammk * ra * rb);
-  double e1 = -rho1 * ra;
-  double e2 = rho1 * (gamm1 - gammk * ra * rb);
-  double e3 = rho1 * rb;
-  double e4 = wvno2 - ra * rb;
+  const RayVec st = rayleigh_start(V.layer(hs), wvno, wvno2, omega, iom);
+  double e0 = st.e0, e1 = st.e1, e2 = st.e2, e3 = st.e3, e4 = st.e4;
   const int mlo = V.llw - 1;
   int since = 0;
   LayerView::Walk wk;
   auto norm_e = [&](int m) {
     if (++since >= NORM || m == mlo) {
       since = 0;
-      double t1 = fmax(fmax(fmax(fabs(e0), fabs(e1)), fmax(fabs(e2), fabs(e3))), fabs(e4));
-      if (t1 < 1.e-40) t1 = 1.0;
-      if (NORM == 1) {
-        e0 = e0 / t1; e1 = e1 / t1; e2 = e2 / t1; e3 = e3 / t1; e4 = e4 / t1;
-      } else {
-        const double it1 = 1.0 / t1;
-        e0 *= it1; e1 *= it1; e2 *= it1; e3 *= it1; e4 *= it1;
-      }
+      rayleigh_norm<NORM>(e0, e1, e2, e3, e4);
     }
   };
   if (hs - 1 >= mlo) {
@@ -567,29 +644,61 @@ SWDK_HDI double dltar4_fast(const LayerView& V, double wvno, double omga) {
     apply_dunkin(cur, wvno2, e0, e1, e2, e3, e4);
     norm_e(m);
   }
-  if (V.llw != 1) {
-    const float4 ly = V.layer(0);
-    const double dpth = ly.x, rho = ly.w;
-    xka = omega * recip((double)ly.y);
-    const double Xa = (wvno + xka) * fabs(wvno - xka);
-    double w, cosp;
-    if (wvno < xka) {
-      const double ir = rsqrt(Xa), r = Xa * ir;
-      double sp, cp;
-      sincos(r * dpth, &sp, &cp);
-      w = sp * ir; cosp = cp;
-    } else if (wvno == xka) {
-      cosp = 1.0; w = dpth;
-    } else {
-      const double ir = rsqrt(Xa), r = Xa * ir, p = r * dpth;
-      const double fac = (p < 16.0) ? exp(-2.0 * p) : 0.0;
-      cosp = (1.0 + fac) * 0.5;
-      w = ((1.0 - fac) * 0.5) * ir;
-    }
-    const double w0 = -rho * w;
-    return cosp * e0 + w0 * e1;
-  }
+  if (V.llw != 1) return rayleigh_fluid_top(V.layer(0), wvno, omega, e0, e1);
   return e0;
+}
+
+// one layer of dltar1's recursion: what depends on the layer and the trial
+// velocity alone, and its product with the propagated pair
+struct LoveCoef {
+  double cosq, y, z, xmu, ixmu;
+};
+
+SWDK_HD LoveCoef love_coef(const float4 ly, double wvno, double omega) {
+  const double beta1 = ly.z, rho1 = ly.w;
+  const double dpth = ly.x;
+  LoveCoef k;
+  k.xmu = rho1 * beta1 * beta1;
+  k.ixmu = recip(k.xmu);
+  const double xkb = omega * recip(beta1);
+  const double Xb = (wvno + xkb) * fabs(wvno - xkb);
+  if (wvno < xkb) {
+    const double ir = rsqrt(Xb), r = Xb * ir;
+    double sq, cq;
+    sincos(dpth * r, &sq, &cq);
+    k.y = sq * ir; k.z = -r * sq; k.cosq = cq;
+  } else if (wvno == xkb) {
+    k.cosq = 1.0; k.y = dpth; k.z = 0.0;
+  } else {
+    const double ir = rsqrt(Xb), r = Xb * ir, q = dpth * r;
+    const double fac = (q < 16.0) ? exp(-2.0 * q) : 0.0;
+    k.cosq = (1.0 + fac) * 0.5;
+    const double sq = (1.0 - fac) * 0.5;
+    k.y = sq * ir; k.z = r * sq;
+  }
+  return k;
+}
+
+SWDK_HD void love_start(const float4 h, double wvno, double omega, double& e1, double& e2) {
+  const double beta1 = h.z, rho1 = h.w;
+  const double xkb = omega * recip(beta1);
+  const double rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
+  e1 = rho1 * rb;
+  e2 = 1.0 / (beta1 * beta1);
+}
+
+template <int NORM>
+SWDK_HD void love_product(const LoveCoef& k, bool norm, double& e1, double& e2) {
+  const double e10 = e1 * k.cosq + e2 * k.xmu * k.z;
+  const double e20 = e1 * k.y * k.ixmu + e2 * k.cosq;
+  if (norm) {
+    double xnor = fmax(fabs(e10), fabs(e20));
+    if (xnor < 1.e-40) xnor = 1.0;
+    if (NORM == 1) { e1 = e10 / xnor; e2 = e20 / xnor; }
+    else { const double ix2 = 1.0 / xnor; e1 = e10 * ix2; e2 = e20 * ix2; }
+  } else {
+    e1 = e10; e2 = e20;
+  }
 }
 
 // dltar1 with 1/b and 1/(rho b^2) from recip()
