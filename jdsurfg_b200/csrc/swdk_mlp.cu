@@ -75,34 +75,39 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 }
 
 // ---------------------------------------------------------------------------
-// C[M x N] = A[M x K] * B[N x K]^T  (A, B bf16 row-major, K % 64 == 0,
-// M % 128 == 0, N % 64 == 0), FP32 accumulate in TMEM, then
-//   out_f32 (optional) = C + bias (pre-activation)
-//   out_bf16 (optional) = act(C + bias) with act = GELU or identity
-// lda/ldb/ldc are row strides in elements.  *err is set when a wait times
-// out (the kernel then skips its epilogue and releases its TMEM).
+// C[128 x 64] += A[128 x K] * B[64 x K]^T over K = [k0, k1)  (A, B bf16
+// row-major, K-slices of 64), FP32 accumulate in TMEM; each thread then hands
+// its row's 64 values to the epilogue epi(row of the tile, v).  *err is set
+// when a wait times out (the epilogue is then skipped and the TMEM released).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float gelu(float x) {
   return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
 }
 
-__global__ void __launch_bounds__(128) k_gemm_tn(int M, int N, int K, const __nv_bfloat16* __restrict__ A, int lda,
-                                                 const __nv_bfloat16* __restrict__ B, int ldb,
-                                                 const float* __restrict__ bias, int act, float* __restrict__ outf,
-                                                 __nv_bfloat16* __restrict__ outb, int ldc, int* __restrict__ err) {
-  __shared__ __align__(1024) uint8_t sA[TM * TK * 2];
-  __shared__ __align__(1024) uint8_t sB[TN * TK * 2];
-  __shared__ __align__(8) uint64_t bar;
+// K-slices in flight per CTA: 24 KB each, so two CTAs fit an SM
+constexpr int GS = 4;
+constexpr size_t GEMM_SMEM = GS * (TM + TN) * TK * 2 + 1024;
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
+}
+
+template <class Epi>
+__device__ __forceinline__ void gemm_tile(const __nv_bfloat16* __restrict__ A, int lda,
+                                          const __nv_bfloat16* __restrict__ B, int ldb, int k0, int k1,
+                                          int* __restrict__ err, Epi epi) {
+  extern __shared__ uint8_t gsm_raw[];
+  uint8_t* gsm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gsm_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t bar[GS];
   __shared__ uint32_t tmem_base;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
                  "r"(TN));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    mbar_init(&bar, 1);
+    for (int i = 0; i < GS; ++i) mbar_init(&bar[i], 1);
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
@@ -111,29 +116,37 @@ __global__ void __launch_bounds__(128) k_gemm_tn(int M, int N, int K, const __nv
   const uint32_t tmem = tmem_base;
   constexpr uint32_t idesc = idesc_bf16(TM, TN);
   bool ok = true;
-  uint32_t phase = 0;
-  for (int k0 = 0; k0 < K; k0 += TK) {
-    // global -> shared, 16-byte chunks, 128B swizzle: chunk j of row r goes
-    // to r*128 + ((j ^ (r & 7)) << 4)
-    for (int c = tid; c < TM * 8; c += 128) {
-      const int r = c >> 3, j = c & 7;
-      const uint4 v = *reinterpret_cast<const uint4*>(A + (size_t)(m0 + r) * lda + k0 + j * 8);
-      *reinterpret_cast<uint4*>(sA + r * 128 + ((j ^ (r & 7)) << 4)) = v;
+  const int n = (k1 - k0) / TK;
+  // slice i into buffer i % GS: global -> shared in 16-byte chunks, 128B
+  // swizzle: chunk j of row r goes to r*128 + ((j ^ (r & 7)) << 4)
+  auto load = [&](int i) {
+    if (i < n) {
+      const uint32_t sa = smem_u32(gsm + (i % GS) * ((TM + TN) * TK * 2)), sb = sa + TM * TK * 2;
+      const int k = k0 + i * TK;
+      for (int c = tid; c < TM * 8; c += 128) {
+        const int r = c >> 3, j = c & 7;
+        cp_async16(sa + r * 128 + ((j ^ (r & 7)) << 4), A + (size_t)r * lda + k + j * 8);
+      }
+      for (int c = tid; c < TN * 8; c += 128) {
+        const int r = c >> 3, j = c & 7;
+        cp_async16(sb + r * 128 + ((j ^ (r & 7)) << 4), B + (size_t)r * ldb + k + j * 8);
+      }
     }
-    for (int c = tid; c < TN * 8; c += 128) {
-      const int r = c >> 3, j = c & 7;
-      const uint4 v = *reinterpret_cast<const uint4*>(B + (size_t)(n0 + r) * ldb + k0 + j * 8);
-      *reinterpret_cast<uint4*>(sB + r * 128 + ((j ^ (r & 7)) << 4)) = v;
-    }
+    asm volatile("cp.async.commit_group;");  // an empty group past the end keeps the count
+  };
+  for (int i = 0; i < GS - 1; ++i) load(i);
+  for (int i = 0; i < n; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(GS - 2));  // slice i has landed (this thread's part)
     asm volatile("fence.proxy.async.shared::cta;");
     __syncthreads();
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;");
-      const uint64_t da = sw128_desc(smem_u32(sA)), db = sw128_desc(smem_u32(sB));
+      const uint32_t sa = smem_u32(gsm + (i % GS) * ((TM + TN) * TK * 2));
+      const uint64_t da = sw128_desc(sa), db = sw128_desc(sa + TM * TK * 2);
 #pragma unroll
       for (int kk = 0; kk < TK / 16; ++kk) {
         const uint64_t a = da + (uint64_t)(kk * 2), b = db + (uint64_t)(kk * 2);  // +32 B per K=16 step
-        const uint32_t acc = (k0 > 0 || kk > 0) ? 1u : 0u;
+        const uint32_t acc = (i > 0 || kk > 0) ? 1u : 0u;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
@@ -141,18 +154,18 @@ __global__ void __launch_bounds__(128) k_gemm_tn(int M, int N, int K, const __nv
             ::"r"(tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc));
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(&bar)));
+          smem_u32(&bar[i % GS])));
     }
-    // every thread waits for the MMAs to finish reading shared memory
-    if (!mbar_wait(&bar, phase)) ok = false;
-    phase ^= 1u;
-    __syncthreads();
+    // the buffer of slice i - 1 takes slice i + GS - 1 once its MMAs have read it
+    if (i > 0 && !mbar_wait(&bar[(i - 1) % GS], ((i - 1) / GS) & 1)) ok = false;
     if (!__syncthreads_and(ok)) break;
+    load(i + GS - 1);
   }
+  asm volatile("cp.async.wait_group 0;");
+  if (ok && n > 0 && !mbar_wait(&bar[(n - 1) % GS], ((n - 1) / GS) & 1)) ok = false;
   asm volatile("tcgen05.fence::after_thread_sync;");
   if (__syncthreads_and(ok)) {
     // TMEM lane = row: warp w owns rows 32w..32w+31; 64 fp32 columns
-    const int row = m0 + warp * 32 + lane;
     uint32_t v[64];
     const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
     asm volatile(
@@ -172,21 +185,118 @@ __global__ void __launch_bounds__(128) k_gemm_tn(int M, int N, int K, const __nv
           "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]), "=r"(v[62]), "=r"(v[63])
         : "r"(taddr + 32u));
     asm volatile("tcgen05.wait::ld.sync.aligned;");
-    if (row < M) {
-#pragma unroll 8
-      for (int j = 0; j < 64; ++j) {
-        const int col = n0 + j;
-        float x = __uint_as_float(v[j]) + (bias ? bias[col] : 0.0f);
-        if (outf) outf[(size_t)row * ldc + col] = x;
-        if (outb) outb[(size_t)row * ldc + col] = __float2bfloat16_rn(act ? gelu(x) : x);
-      }
-    }
+    epi(warp * 32 + lane, v);
   } else if (tid == 0) {
     atomicExch(err, 1);
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN));
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi) {
+  return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
+}
+
+// C[M x N] = A[M x K] * B[N x K]^T (M % 128 == 0, N % 64 == 0, K % 64 == 0):
+//   out_f32 (optional) = C + bias (pre-activation)
+//   out_bf16 (optional) = act(C + bias) with act = GELU or identity
+//   outt (optional) = the transpose of out_bf16 (N x M, row stride ldt)
+// lda/ldb/ldc are row strides in elements.  A thread holds a row of the tile:
+// its values leave in 16-byte stores, the transpose in stores of 64
+// contiguous bytes per warp.
+__global__ void __launch_bounds__(128) k_gemm_tn(int M, int N, int K, const __nv_bfloat16* __restrict__ A, int lda,
+                                                 const __nv_bfloat16* __restrict__ B, int ldb,
+                                                 const float* __restrict__ bias, int act, float* __restrict__ outf,
+                                                 __nv_bfloat16* __restrict__ outb, int ldc,
+                                                 __nv_bfloat16* __restrict__ outt, int ldt, int* __restrict__ err) {
+  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
+  const bool vec = (reinterpret_cast<uintptr_t>(outf) & 15) == 0 && (ldc & 3) == 0;  // a caller's output may be neither
+  gemm_tile(A + (size_t)m0 * lda, lda, B + (size_t)n0 * ldb, ldb, 0, K, err, [&](int r, const uint32_t (&v)[64]) {
+    const int row = m0 + r;
+#pragma unroll
+    for (int j = 0; j < 64; j += 8) {
+      float x[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = __uint_as_float(v[j + e]) + (bias ? bias[n0 + j + e] : 0.0f);
+      if (outf && vec) {
+        float4* o = reinterpret_cast<float4*>(outf + (size_t)row * ldc + n0 + j);
+        o[0] = make_float4(x[0], x[1], x[2], x[3]);
+        o[1] = make_float4(x[4], x[5], x[6], x[7]);
+      } else if (outf) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) outf[(size_t)row * ldc + n0 + j + e] = x[e];
+      }
+      if (outb) {
+        __nv_bfloat16 h[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16_rn(act ? gelu(x[e]) : x[e]);
+        *reinterpret_cast<uint4*>(outb + (size_t)row * ldc + n0 + j) =
+            make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
+        if (outt)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) outt[(size_t)(n0 + j + e) * ldt + row] = h[e];
+      }
+    }
+  });
+}
+
+// dZ = (dZ' W) GELU'(Z) of the layer below (A = dZ' (M x K), B = W^T (N x K)):
+// the product rounded to bf16 (dH), times GELU'(z) (M x N floats), as bf16 rows
+// (dz, row stride N) and transposed (dzt, row stride ldt)
+__global__ void __launch_bounds__(128) k_gemm_dx(int K, int N, const __nv_bfloat16* __restrict__ A,
+                                                 const __nv_bfloat16* __restrict__ B, const float* __restrict__ z,
+                                                 __nv_bfloat16* __restrict__ dz, __nv_bfloat16* __restrict__ dzt,
+                                                 int ldt, int* __restrict__ err) {
+  const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
+  gemm_tile(A + (size_t)m0 * K, K, B + (size_t)n0 * K, K, 0, K, err, [&](int r, const uint32_t (&v)[64]) {
+    const int row = m0 + r;
+#pragma unroll
+    for (int j = 0; j < 64; j += 8) {
+      const float4* zp = reinterpret_cast<const float4*>(z + (size_t)row * N + n0 + j);
+      const float4 za = zp[0], zb = zp[1];
+      const float zz[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
+      __nv_bfloat16 h[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float x = zz[e];
+        const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
+        const float pdf = 0.39894228040143268f * expf(-0.5f * x * x);
+        const float dh = __bfloat162float(__float2bfloat16_rn(__uint_as_float(v[j + e])));
+        h[e] = __float2bfloat16_rn(dh * (cdf + x * pdf));
+      }
+      *reinterpret_cast<uint4*>(dz + (size_t)row * N + n0 + j) =
+          make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
+#pragma unroll
+      for (int e = 0; e < 8; ++e) dzt[(size_t)(n0 + j + e) * ldt + row] = h[e];
+    }
+  });
+}
+
+// dW of every layer in one launch: dW[nl x kl] = dZ^T[nl x M] X^T[kl x M]^T, a
+// tile per block over the whole batch (split over the batch the sums would
+// round differently: 7e-5 of the gradients' norm at 16 384 rows), K-slices in
+// flight behind one another.  Rows padded to 128 go to `out`, k_grad's input.
+struct DwJob {
+  const __nv_bfloat16 *dzt, *xt;  // (rows padded to 128) x M, kl x M
+  int tile0, ntn, kl;             // first block, tiles along kl
+  int off;                        // of the layer's block in out
+};
+struct DwJobs {
+  DwJob j[MLP_LAYERS];
+};
+__global__ void __launch_bounds__(128) k_gemm_dw(DwJobs jobs, int M, float* __restrict__ out, int* __restrict__ err) {
+  int l = MLP_LAYERS - 1;
+  while (l > 0 && (int)blockIdx.x < jobs.j[l].tile0) --l;
+  const DwJob J = jobs.j[l];
+  const int t = blockIdx.x - J.tile0, m0 = (t / J.ntn) * TM, n0 = (t % J.ntn) * TN;
+  gemm_tile(J.dzt + (size_t)m0 * M, M, J.xt + (size_t)n0 * M, M, 0, M, err, [&](int r, const uint32_t (&v)[64]) {
+    float4* o = reinterpret_cast<float4*>(out + J.off + (size_t)(m0 + r) * J.kl + n0);
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      o[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]),
+                         __uint_as_float(v[4 * j + 3]));
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -457,13 +567,32 @@ __global__ void k_transpose_bf16(int rows, int cols, const __nv_bfloat16* __rest
   }
 }
 
+// the transposed bf16 weights (kin x nout) of layers 1 .. 4, one layer per z
+struct WtJobs {
+  size_t off[MLP_LAYERS];
+  int kin[MLP_LAYERS], nout[MLP_LAYERS];
+};
+__global__ void k_transpose_weights(WtJobs J, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ wt) {
+  __shared__ __nv_bfloat16 t[32][33];
+  const int l = blockIdx.z + 1, rows = J.nout[l], cols = J.kin[l];
+  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
+  if (r0 >= rows || c0 >= cols) return;
+  const __nv_bfloat16* x = w + J.off[l];
+  __nv_bfloat16* y = wt + J.off[l];
+  for (int i = threadIdx.y; i < 32; i += blockDim.y) t[i][threadIdx.x] = x[(size_t)(r0 + i) * cols + c0 + threadIdx.x];
+  __syncthreads();
+  for (int i = threadIdx.y; i < 32; i += blockDim.y) y[(size_t)(c0 + i) * rows + r0 + threadIdx.x] = t[threadIdx.x][i];
+}
+
 // Gaussian NLL of (mu, log sigma) against y on rows < M (rows of the padded
-// batch beyond M get zero gradient); dOut is the bf16 gradient w.r.t. the
-// 16-wide output (columns 0,1), loss accumulates the batch mean.
-__global__ void k_nll(int M, int Mpad, const float* __restrict__ out, const float* __restrict__ y,
-                      __nv_bfloat16* __restrict__ dout, float* __restrict__ loss) {
+// batch beyond M get zero gradient); dout is the bf16 gradient w.r.t. the
+// 64-wide output (columns 0,1) and doutt its transpose's rows 0 and 1 (the
+// others stay zero); lossp gets each block's sum of the batch mean's terms.
+__global__ void __launch_bounds__(256) k_nll(int M, int Mpad, const float* __restrict__ out,
+                                             const float* __restrict__ y, __nv_bfloat16* __restrict__ dout,
+                                             __nv_bfloat16* __restrict__ doutt, float* __restrict__ lossp) {
+  __shared__ float sh[256];
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= Mpad) return;
   float g0 = 0.0f, g1 = 0.0f, l = 0.0f;
   if (r < M) {
     const float mu = out[(size_t)r * MLP_OUT], ls = fminf(fmaxf(out[(size_t)r * MLP_OUT + 1], -12.0f), 4.0f);
@@ -472,45 +601,89 @@ __global__ void k_nll(int M, int Mpad, const float* __restrict__ out, const floa
     g0 = -e * inv / (float)M;
     g1 = (1.0f - e * e) / (float)M;
   }
-  for (int j = 0; j < MLP_OUT; ++j)
-    dout[(size_t)r * MLP_OUT + j] = __float2bfloat16_rn(j == 0 ? g0 : j == 1 ? g1 : 0.0f);
-  if (r < M) atomicAdd(loss, l / (float)M);
+  if (r < Mpad) {
+    const __nv_bfloat16 b0 = __float2bfloat16_rn(g0), b1 = __float2bfloat16_rn(g1);
+    uint4* d = reinterpret_cast<uint4*>(dout + (size_t)r * MLP_OUT);
+    d[0] = make_uint4(pack_bf16(b0, b1), 0u, 0u, 0u);
+#pragma unroll
+    for (int j = 1; j < MLP_OUT / 8; ++j) d[j] = make_uint4(0u, 0u, 0u, 0u);
+    doutt[r] = b0;
+    doutt[(size_t)Mpad + r] = b1;
+  }
+  sh[threadIdx.x] = r < M ? l / (float)M : 0.0f;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) lossp[blockIdx.x] = sh[0];
 }
 
-// dZ = dH * GELU'(Z)   (bf16 dH in, bf16 dZ out)
-__global__ void k_gelu_back(int n, const float* __restrict__ z, const __nv_bfloat16* __restrict__ dh,
-                            __nv_bfloat16* __restrict__ dz) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float x = z[i];
-  const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
-  const float pdf = 0.39894228040143268f * expf(-0.5f * x * x);
-  dz[i] = __float2bfloat16_rn(__bfloat162float(dh[i]) * (cdf + x * pdf));
-}
-
-// db[c] = sum_r dz[r, c]
-__global__ void k_colsum(int rows, int cols, const __nv_bfloat16* __restrict__ dz, float* __restrict__ db) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.0f;
-  for (int r = 0; r < rows; ++r) s += __bfloat162float(dz[(size_t)r * cols + c]);
-  db[c] = s;
-}
-
-// Adam with bias correction on FP32 masters; refreshes the bf16 copies
-__global__ void k_adam(int n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2,
-                       const unsigned char* __restrict__ mask, __nv_bfloat16* __restrict__ wb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (mask && !mask[i]) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi, vi = b2 * v[i] + (1.0f - b2) * gi * gi;
+// Gradients of all parameters and, with lr > 0, Adam with bias correction on
+// the FP32 masters (which refreshes the bf16 copies).  Blocks below nbw: one
+// weight per thread; the others: one bias per warp, the sum over the batch of
+// its row of dZ^T (a thread per bias that walked the batch took a third of a
+// step of 4096 rows); the last block: the loss.
+struct GradJob {
+  const __nv_bfloat16* dzt;
+  int woff, boff, nw, nb, poff, wblk0, bwarp0;
+};
+struct GradJobs {
+  GradJob j[MLP_LAYERS];
+};
+struct AdamArgs {
+  float lr, b1, b2, eps, c1, c2;
+};
+__device__ __forceinline__ void adam_one(int i, float gi, float* __restrict__ w, float* __restrict__ g,
+                                         float* __restrict__ m, float* __restrict__ v, const AdamArgs& A,
+                                         const unsigned char* __restrict__ mask, __nv_bfloat16* __restrict__ wb) {
+  g[i] = gi;
+  if (!(A.lr > 0.0f) || !mask[i]) return;
+  const float mi = A.b1 * m[i] + (1.0f - A.b1) * gi, vi = A.b2 * v[i] + (1.0f - A.b2) * gi * gi;
   m[i] = mi;
   v[i] = vi;
-  const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  const float wi = w[i] - A.lr * (mi / A.c1) / (sqrtf(vi / A.c2) + A.eps);
   w[i] = wi;
-  if (wb) wb[i] = __float2bfloat16_rn(wi);
+  wb[i] = __float2bfloat16_rn(wi);
+}
+__global__ void __launch_bounds__(256) k_grad(GradJobs jobs, int nbw, int nbb, int Mpad,
+                                              const float* __restrict__ dw, const float* __restrict__ lossp,
+                                              int nloss, float* __restrict__ loss, float* __restrict__ w,
+                                              float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
+                                              AdamArgs A, const unsigned char* __restrict__ mask,
+                                              __nv_bfloat16* __restrict__ wb) {
+  if ((int)blockIdx.x < nbw) {
+    int l = MLP_LAYERS - 1;
+    while (l > 0 && (int)blockIdx.x < jobs.j[l].wblk0) --l;
+    const GradJob& J = jobs.j[l];
+    const int i = ((int)blockIdx.x - J.wblk0) * 256 + threadIdx.x;
+    if (i >= J.nw) return;
+    adam_one(J.woff + i, dw[J.poff + i], w, g, m, v, A, mask, wb);
+  } else if ((int)blockIdx.x < nbw + nbb) {
+    const int gw = ((int)blockIdx.x - nbw) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    int l = MLP_LAYERS - 1;
+    while (l > 0 && gw < jobs.j[l].bwarp0) --l;
+    const GradJob& J = jobs.j[l];
+    const int c = gw - J.bwarp0;
+    if (c >= J.nb) return;
+    const uint4* row = reinterpret_cast<const uint4*>(J.dzt + (size_t)c * Mpad);
+    float s = 0.0f;
+    for (int q = lane; q < Mpad / 8; q += 32) {
+      const uint4 u = row[q];
+      const uint32_t a[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        s += __uint_as_float(a[e] << 16);
+        s += __uint_as_float(a[e] & 0xffff0000u);
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) adam_one(J.boff + c, s, w, g, m, v, A, mask, wb);
+  } else if (threadIdx.x == 0) {
+    float s = 0.0f;
+    for (int i = 0; i < nloss; ++i) s += lossp[i];
+    *loss = s;
+  }
 }
 
 }  // namespace
@@ -530,9 +703,13 @@ struct swdk_mlp {
   int step = 0;
   // activations for a batch of up to cap rows
   int cap = 0;
-  __nv_bfloat16 *xin = nullptr, *h[MLP_LAYERS] = {}, *dz[MLP_LAYERS] = {}, *xt = nullptr, *dzt = nullptr,
-                *dh = nullptr;
-  float *z[MLP_LAYERS] = {}, *out = nullptr, *y = nullptr, *loss = nullptr, *gscr = nullptr;
+  __nv_bfloat16 *xin = nullptr, *h[MLP_LAYERS] = {}, *dz[MLP_LAYERS] = {};
+  float *z[MLP_LAYERS] = {}, *loss = nullptr;
+  // a training step's: transposed layer inputs xt[l] (kin x rows) and output
+  // gradients dzt[l] (nout, padded to 128, x rows), padded dW blocks, loss terms
+  int tcap = 0;
+  __nv_bfloat16 *xt[MLP_LAYERS] = {}, *dzt[MLP_LAYERS] = {};
+  float *dw = nullptr, *lossp = nullptr;
   // fused inference: swizzled weight image, layer offsets on the device
   uint8_t* wsw = nullptr;
   size_t* d_offs = nullptr;  // woff[5], boff[5]
@@ -555,10 +732,18 @@ int mlp_fail(swdk_mlp* p, const char* what, cudaError_t e) {
     if (e_ != cudaSuccess) return mlp_fail(p, #call, e_);      \
   } while (0)
 
+// opts the GEMM kernels in to their dynamic shared memory on the current device
+cudaError_t gemm_ready() {
+  cudaError_t e = cudaFuncSetAttribute(k_gemm_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_dx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_gemm_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
+  return e;
+}
+
 int gemm(swdk_mlp* p, int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb,
-         const float* bias, int act, float* outf, __nv_bfloat16* outb, int ldc, cudaStream_t st) {
+         const float* bias, int act, float* outf, __nv_bfloat16* outb, int ldc, __nv_bfloat16* outt, cudaStream_t st) {
   dim3 grid(M / TM, N / TN);
-  k_gemm_tn<<<grid, 128, 0, st>>>(M, N, K, A, lda, B, ldb, bias, act, outf, outb, ldc, p->err);
+  k_gemm_tn<<<grid, 128, GEMM_SMEM, st>>>(M, N, K, A, lda, B, ldb, bias, act, outf, outb, ldc, outt, M, p->err);
   MCK(cudaGetLastError());
   return SWDK_OK;
 }
@@ -566,15 +751,10 @@ int gemm(swdk_mlp* p, int M, int N, int K, const __nv_bfloat16* A, int lda, cons
 int ensure_batch(swdk_mlp* p, int rows) {
   if (rows <= p->cap) return SWDK_OK;
   auto fr = [](void* q) { if (q) cudaFree(q); };
-  fr(p->xin); fr(p->xt); fr(p->dzt); fr(p->dh); fr(p->out); fr(p->y);
+  fr(p->xin);
   for (int l = 0; l < MLP_LAYERS; ++l) { fr(p->h[l]); fr(p->dz[l]); fr(p->z[l]); }
   const size_t R = (size_t)rows;
   MCK(cudaMalloc(&p->xin, R * MLP_IN * sizeof(__nv_bfloat16)));
-  MCK(cudaMalloc(&p->xt, R * MLP_IN * sizeof(__nv_bfloat16)));
-  MCK(cudaMalloc(&p->dzt, R * MLP_H * sizeof(__nv_bfloat16)));
-  MCK(cudaMalloc(&p->dh, R * MLP_IN * sizeof(__nv_bfloat16)));
-  MCK(cudaMalloc(&p->out, R * MLP_OUT * sizeof(float)));
-  MCK(cudaMalloc(&p->y, R * sizeof(float)));
   for (int l = 0; l < MLP_LAYERS; ++l) {
     MCK(cudaMalloc(&p->h[l], R * p->nout[l] * sizeof(__nv_bfloat16)));
     MCK(cudaMalloc(&p->dz[l], R * p->nout[l] * sizeof(__nv_bfloat16)));
@@ -584,14 +764,45 @@ int ensure_batch(swdk_mlp* p, int rows) {
   return SWDK_OK;
 }
 
+int pad128(int n) { return (n + TM - 1) / TM * TM; }
+int dw_total(const swdk_mlp* p) {
+  int t = 0;
+  for (int l = 0; l < MLP_LAYERS; ++l) t += pad128(p->nout[l]) * p->kin[l];
+  return t;
+}
+
+// the buffers of a training step on a batch of `rows` (the transposes have
+// rows as their row stride, so they are laid out again when it changes)
+int ensure_train(swdk_mlp* p, int rows, cudaStream_t st) {
+  if (rows > p->tcap) {
+    auto fr = [](void* q) { if (q) cudaFree(q); };
+    for (int l = 0; l < MLP_LAYERS; ++l) { fr(p->xt[l]); fr(p->dzt[l]); p->xt[l] = p->dzt[l] = nullptr; }
+    fr(p->lossp);
+    p->lossp = nullptr;
+    p->tcap = 0;
+    for (int l = 0; l < MLP_LAYERS; ++l) {
+      MCK(cudaMalloc(&p->xt[l], (size_t)rows * p->kin[l] * sizeof(__nv_bfloat16)));
+      MCK(cudaMalloc(&p->dzt[l], (size_t)rows * pad128(p->nout[l]) * sizeof(__nv_bfloat16)));
+    }
+    MCK(cudaMalloc(&p->lossp, (size_t)(rows / 128) * sizeof(float)));
+    p->tcap = rows;
+  }
+  if (!p->dw) MCK(cudaMalloc(&p->dw, (size_t)dw_total(p) * sizeof(float)));
+  // rows 2 and up of the output layer's transposed gradient are zero
+  __nv_bfloat16* t = p->dzt[MLP_LAYERS - 1];
+  MCK(cudaMemsetAsync(t + (size_t)2 * rows, 0, (size_t)(pad128(MLP_OUT) - 2) * rows * sizeof(__nv_bfloat16), st));
+  return SWDK_OK;
+}
+
 // forward pass on p->xin (rows Mpad); the last pre-activation z[4]
 // (Mpad x 64) holds (mu, log sigma) in columns 0, 1
-int forward(swdk_mlp* p, int Mpad, cudaStream_t st) {
+int forward(swdk_mlp* p, int Mpad, cudaStream_t st, bool train = false) {
   const __nv_bfloat16* x = p->xin;
   for (int l = 0; l < MLP_LAYERS; ++l) {
     const bool last = (l == MLP_LAYERS - 1);
     const int r = gemm(p, Mpad, p->nout[l], p->kin[l], x, p->kin[l], p->wb + p->woff[l], p->kin[l],
-                       p->w + p->boff[l], last ? 0 : 1, p->z[l], last ? nullptr : p->h[l], p->nout[l], st);
+                       p->w + p->boff[l], last ? 0 : 1, p->z[l], last ? nullptr : p->h[l], p->nout[l],
+                       train && !last ? p->xt[l + 1] : nullptr, st);
     if (r) return r;
     x = p->h[l];
   }
@@ -608,6 +819,7 @@ int swdk_mlp_create(swdk_mlp** out, int device, uint64_t seed) {
   swdk_mlp* p = new swdk_mlp();
   p->device = device;
   MCK(cudaSetDevice(device));
+  MCK(gemm_ready());
   MCK(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking));
   const int kin[MLP_LAYERS] = {MLP_IN, MLP_H, MLP_H, MLP_H, MLP_H};
   const int nout[MLP_LAYERS] = {MLP_H, MLP_H, MLP_H, MLP_H, MLP_OUT};
@@ -644,7 +856,6 @@ int swdk_mlp_create(swdk_mlp** out, int device, uint64_t seed) {
   MCK(cudaMalloc(&p->wb, off * sizeof(__nv_bfloat16)));
   MCK(cudaMalloc(&p->wt, off * sizeof(__nv_bfloat16)));
   MCK(cudaMalloc(&p->loss, sizeof(float)));
-  MCK(cudaMalloc(&p->gscr, (size_t)TM * MLP_IN * sizeof(float)));
   MCK(cudaMalloc(&p->err, sizeof(int)));
   MCK(cudaMemcpy(p->w, hw.data(), off * sizeof(float), cudaMemcpyHostToDevice));
   MCK(cudaMemcpy(p->mask, hm.data(), off, cudaMemcpyHostToDevice));
@@ -664,14 +875,16 @@ void swdk_mlp_destroy(swdk_mlp* p) {
   if (!p) return;
   cudaSetDevice(p->device);
   if (p->stream) cudaStreamSynchronize(p->stream);
-  void* bufs[] = {p->w, p->m, p->v, p->g, p->mask, p->wb, p->wt, p->loss, p->gscr, p->err, p->xin, p->xt, p->dzt,
-                  p->dh, p->out, p->y, p->wsw, p->d_offs};
+  void* bufs[] = {p->w, p->m, p->v, p->g, p->mask, p->wb, p->wt, p->loss, p->err, p->xin, p->dw, p->lossp,
+                  p->wsw, p->d_offs};
   for (void* b : bufs)
     if (b) cudaFree(b);
   for (int l = 0; l < MLP_LAYERS; ++l) {
     if (p->h[l]) cudaFree(p->h[l]);
     if (p->dz[l]) cudaFree(p->dz[l]);
     if (p->z[l]) cudaFree(p->z[l]);
+    if (p->xt[l]) cudaFree(p->xt[l]);
+    if (p->dzt[l]) cudaFree(p->dzt[l]);
   }
   if (p->stream) cudaStreamDestroy(p->stream);
   delete p;
@@ -700,9 +913,10 @@ int swdk_mlp_set_params(swdk_mlp* p, const float* host, int64_t n) {
 // y = A * B^T on device bf16 operands (exposed for the GEMM unit test)
 int swdk_gemm_bf16_tn(int M, int N, int K, const void* d_a, const void* d_b, float* d_c, int* d_err, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0 || M % TM || N % TN || K % TK || !d_a || !d_b || !d_c || !d_err) return SWDK_E_ARG;
+  if (gemm_ready() != cudaSuccess) return SWDK_E_CUDA;
   dim3 grid(M / TM, N / TN);
-  k_gemm_tn<<<grid, 128, 0, (cudaStream_t)stream>>>(M, N, K, (const __nv_bfloat16*)d_a, K, (const __nv_bfloat16*)d_b,
-                                                     K, nullptr, 0, d_c, nullptr, N, d_err);
+  k_gemm_tn<<<grid, 128, GEMM_SMEM, (cudaStream_t)stream>>>(M, N, K, (const __nv_bfloat16*)d_a, K, (const __nv_bfloat16*)d_b,
+                                                     K, nullptr, 0, d_c, nullptr, N, nullptr, 0, d_err);
   return cudaGetLastError() == cudaSuccess ? SWDK_OK : SWDK_E_CUDA;
 }
 
@@ -777,61 +991,58 @@ int swdk_mlp_train_step(swdk_mlp* p, const void* d_x, const float* d_y, int M, f
   if (r) return r;
   MCK(cudaMemsetAsync(p->xin + (size_t)M * MLP_IN, 0, (size_t)(Mpad - M) * MLP_IN * sizeof(__nv_bfloat16), st));
   MCK(cudaMemcpyAsync(p->xin, d_x, (size_t)M * MLP_IN * sizeof(__nv_bfloat16), cudaMemcpyDeviceToDevice, st));
-  MCK(cudaMemcpyAsync(p->y, d_y, (size_t)M * sizeof(float), cudaMemcpyDeviceToDevice, st));
-  MCK(cudaMemsetAsync(p->loss, 0, sizeof(float), st));
-  r = forward(p, Mpad, st);
+  r = ensure_train(p, Mpad, st);
   if (r) return r;
-  // output gradient (layer 4 pre-activation = output, no activation)
-  k_nll<<<(Mpad + 255) / 256, 256, 0, st>>>(M, Mpad, p->z[MLP_LAYERS - 1], p->y, p->dz[MLP_LAYERS - 1], p->loss);
-  MCK(cudaGetLastError());
-  // weight transposes for dX (bf16): wt block of layer l is (kin x nout)
-  for (int l = 1; l < MLP_LAYERS; ++l) {
-    dim3 g((p->kin[l] + 31) / 32, (p->nout[l] + 31) / 32);
-    k_transpose_bf16<<<g, dim3(32, 8), 0, st>>>(p->nout[l], p->kin[l], p->wb + p->woff[l], p->kin[l],
-                                                 p->wt + p->woff[l], p->nout[l]);
-  }
-  MCK(cudaGetLastError());
-  for (int l = MLP_LAYERS - 1; l >= 0; --l) {
-    const int nl = p->nout[l], kl = p->kin[l];
-    const __nv_bfloat16* xl = (l == 0) ? p->xin : p->h[l - 1];
-    if (l < MLP_LAYERS - 1) {  // dZ = dH * GELU'(Z)
-      const int n = Mpad * nl;
-      k_gelu_back<<<(n + 255) / 256, 256, 0, st>>>(n, p->z[l], p->dh, p->dz[l]);
-    }
-    // dW[nl x kl] = dZ^T[nl x M] X[M x kl]: A = dZ^T (nl rows, padded to 128), B = X^T (kl x M)
-    const int Mw = (nl + TM - 1) / TM * TM;
-    if (Mw > nl) MCK(cudaMemsetAsync(p->dzt + (size_t)nl * Mpad, 0, (size_t)(Mw - nl) * Mpad * 2, st));
-    {
-      dim3 g1((nl + 31) / 32, (Mpad + 31) / 32);
-      k_transpose_bf16<<<g1, dim3(32, 8), 0, st>>>(Mpad, nl, p->dz[l], nl, p->dzt, Mpad);
-      dim3 g2((kl + 31) / 32, (Mpad + 31) / 32);
-      k_transpose_bf16<<<g2, dim3(32, 8), 0, st>>>(Mpad, kl, xl, kl, p->xt, Mpad);
-    }
-    float* gw = p->g + p->woff[l];
-    r = gemm(p, Mw, kl, Mpad, p->dzt, Mpad, p->xt, Mpad, nullptr, 0, Mw == nl ? gw : p->gscr, nullptr, kl, st);
-    if (r) return r;
-    if (Mw != nl) MCK(cudaMemcpyAsync(gw, p->gscr, (size_t)nl * kl * sizeof(float), cudaMemcpyDeviceToDevice, st));
-    k_colsum<<<(nl + 127) / 128, 128, 0, st>>>(Mpad, nl, p->dz[l], p->g + p->boff[l]);
-    if (l > 0) {  // dX[M x kl] = dZ[M x nl] W[nl x kl]: A = dZ, B = W^T (kl x nl)
-      r = gemm(p, Mpad, kl, nl, p->dz[l], nl, p->wt + p->woff[l], nl, nullptr, 0, nullptr, p->dh, kl, st);
-      if (r) return r;
-    }
-  }
-  MCK(cudaGetLastError());
-  if (lr > 0.0f) {
-    p->step += 1;
-    const float b1 = 0.9f, b2 = 0.999f;
-    const float c1 = 1.0f - powf(b1, (float)p->step), c2 = 1.0f - powf(b2, (float)p->step);
-    k_adam<<<(int)((p->nparam + 255) / 256), 256, 0, st>>>((int)p->nparam, p->w, p->g, p->m, p->v, lr, b1, b2, 1e-8f,
-                                                           c1, c2, p->mask, p->wb);
-  p->wsw_dirty = true;
+  {  // X^T for the first layer's dW; W^T of layers 1 .. 4 for dX
+    k_transpose_bf16<<<dim3((MLP_IN + 31) / 32, Mpad / 32), dim3(32, 8), 0, st>>>(Mpad, MLP_IN, p->xin, MLP_IN, p->xt[0],
+                                                                                 Mpad);
+    WtJobs J;
+    for (int l = 0; l < MLP_LAYERS; ++l) { J.off[l] = p->woff[l]; J.kin[l] = p->kin[l]; J.nout[l] = p->nout[l]; }
+    k_transpose_weights<<<dim3(MLP_H / 32, MLP_H / 32, MLP_LAYERS - 1), dim3(32, 8), 0, st>>>(J, p->wb, p->wt);
     MCK(cudaGetLastError());
   }
-  if (loss_out) {
-    MCK(cudaMemcpyAsync(loss_out, p->loss, sizeof(float), cudaMemcpyDeviceToHost, st));
-    MCK(cudaStreamSynchronize(st));
+  r = forward(p, Mpad, st, true);
+  if (r) return r;
+  // output gradient (layer 4 pre-activation = output, no activation)
+  const int nloss = (Mpad + 255) / 256;
+  k_nll<<<nloss, 256, 0, st>>>(M, Mpad, p->z[MLP_LAYERS - 1], d_y, p->dz[MLP_LAYERS - 1], p->dzt[MLP_LAYERS - 1],
+                               p->lossp);
+  MCK(cudaGetLastError());
+  // down the layers: dZ[l-1] = (dZ[l] W[l]) GELU'(Z[l-1])
+  for (int l = MLP_LAYERS - 1; l > 0; --l) {
+    k_gemm_dx<<<dim3(Mpad / TM, p->kin[l] / TN), 128, GEMM_SMEM, st>>>(p->nout[l], p->kin[l], p->dz[l], p->wt + p->woff[l],
+                                                              p->z[l - 1], p->dz[l - 1], p->dzt[l - 1], Mpad, p->err);
+    MCK(cudaGetLastError());
   }
+  // every dW, then all gradients (and the Adam step)
+  DwJobs D;
+  GradJobs Gj;
+  int tiles = 0, off = 0, nbw = 0, bwarps = 0;
+  for (int l = 0; l < MLP_LAYERS; ++l) {
+    const int nl = p->nout[l], kl = p->kin[l], Mw = pad128(nl);
+    D.j[l] = DwJob{p->dzt[l], p->xt[l], tiles, kl / TN, kl, off};
+    Gj.j[l] = GradJob{p->dzt[l], (int)p->woff[l], (int)p->boff[l], nl * kl, nl, off, nbw, bwarps};
+    tiles += (Mw / TM) * (kl / TN);
+    off += Mw * kl;
+    nbw += (nl * kl + 255) / 256;
+    bwarps += nl;
+  }
+  k_gemm_dw<<<tiles, 128, GEMM_SMEM, st>>>(D, Mpad, p->dw, p->err);
+  MCK(cudaGetLastError());
+  AdamArgs A{0.0f, 0.9f, 0.999f, 1e-8f, 1.0f, 1.0f};
+  if (lr > 0.0f) {
+    p->step += 1;
+    A.lr = lr;
+    A.c1 = 1.0f - powf(A.b1, (float)p->step);
+    A.c2 = 1.0f - powf(A.b2, (float)p->step);
+    p->wsw_dirty = true;
+  }
+  const int nbb = (bwarps + 7) / 8;
+  k_grad<<<nbw + nbb + 1, 256, 0, st>>>(Gj, nbw, nbb, Mpad, p->dw, p->lossp, nloss, p->loss, p->w, p->g, p->m,
+                                        p->v, A, p->mask, p->wb);
+  MCK(cudaGetLastError());
   int herr = 0;
+  if (loss_out) MCK(cudaMemcpyAsync(loss_out, p->loss, sizeof(float), cudaMemcpyDeviceToHost, st));
   MCK(cudaMemcpyAsync(&herr, p->err, sizeof(int), cudaMemcpyDeviceToHost, st));
   MCK(cudaStreamSynchronize(st));
   if (herr) { p->msg = "tensor-core wait timed out"; return SWDK_E_CUDA; }
