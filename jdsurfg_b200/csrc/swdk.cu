@@ -202,91 +202,161 @@ __device__ void write_layers(int L, int ncol, int col, int lstride, const float*
 }
 
 // ---------------------------------------------------------------------------
-// k_prep: node model -> layer models (one thread per column)
+// k_prep: node model -> layer models, one warp per column, lanes over its
+// nodes and sublayers.  What bounds it is the dependent chain of a column
+// (Brocher's polynomials, the flattening's divisions and logarithms), not its
+// bytes: with a thread per column a call of any size took 0.25 to 0.5 ms (20
+// to 41 nodes) and 1.7 ms for 65 536 columns of 64.  The flattening of columns
+// without fluid nodes is the depth grid's own and comes from its table.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_prep(int ncol, int ldi, int nz, const float* __restrict__ vs_in,
+constexpr int PREP_COLS = 4;  // columns (warps) per block
+
+// sphere() (surfdisp96.f:499-571, ar = 6370) for one layer of thickness th
+// whose top lies dr0 (a running sum in layer order) below the surface; last:
+// the half-space, counted as 1 km
+__device__ __forceinline__ DepthLayer flatten_layer(double dr0, float th, bool first, bool last) {
+  const double ar = 6370.0;
+  const double r0 = first ? ar : dsub(ar, dr0);
+  const double r1 = dsub(ar, dadd(dr0, (double)(last ? 1.0f : th)));
+  const double z0 = dmul(ar, log(ddiv(ar, r0)));
+  const double z1 = dmul(ar, log(ddiv(ar, r1)));
+  DepthLayer q;
+  q.pad_ = 0.0f;
+  q.d = last ? 0.0f : (float)dsub(z1, z0);
+  q.tmp = ddiv(dadd(ar, ar), dadd(r0, r1));
+  const float btp = (float)q.tmp;
+  q.fR = (float)pow((double)btp, (double)(-2.275f));
+  const float b2 = fmul(btp, btp), b4 = fmul(b2, b2), b5 = fmul(b4, btp);
+  q.fL = fdiv(1.0f, b5);
+  return q;
+}
+
+__global__ void __launch_bounds__(32 * PREP_COLS) k_prep(int ncol, int ldi, int nz, const float* __restrict__ vs_in,
                                               const float* __restrict__ vp_in, const float* __restrict__ rho_in,
                                               const float* __restrict__ depth, int sphere, int Lmax,
                                               float4* __restrict__ layR, float4* __restrict__ layL,
                                               float4* __restrict__ lay0,
                                               ColInfo* __restrict__ info, float2* __restrict__ chainrule,
-                                              float4* __restrict__ nodefeat, float4* __restrict__ nodes) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
+                                              float4* __restrict__ nodefeat, float4* __restrict__ nodes,
+                                              const DepthLayer* __restrict__ dl) {
+  const unsigned FULL = 0xffffffffu;
+  __shared__ float sv[PREP_COLS][NZMAX], sp[PREP_COLS][NZMAX], sr[PREP_COLS][NZMAX], dep[NZMAX];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int k = threadIdx.x; k < nz; k += blockDim.x) dep[k] = depth[k];
+  __syncthreads();
+  const int col = blockIdx.x * PREP_COLS + w;
   if (col >= ncol) return;
-  float v[NZMAX], vp[NZMAX], rho[NZMAX], dep[NZMAX];
-  bool valid = true;
-  for (int k = 0; k < nz; ++k) {
-    v[k] = vs_in[col + (size_t)ldi * k];
-    dep[k] = depth[k];
+  float *v = sv[w], *vp = sp[w], *rho = sr[w];
+  bool bad = false;
+  int first = nz;  // first solid node
+  for (int k = lane; k < nz; k += 32) {
+    const float vk = vs_in[col + (size_t)ldi * k];
+    float pk, rk;
     if (vp_in) {
-      vp[k] = vp_in[col + (size_t)ldi * k];
-      rho[k] = rho_in[col + (size_t)ldi * k];
+      pk = vp_in[col + (size_t)ldi * k];
+      rk = rho_in[col + (size_t)ldi * k];
     } else {
-      brocher(v[k], vp[k], rho[k]);
+      brocher(vk, pk, rk);
     }
-    if (!finitef(v[k]) || !finitef(vp[k]) || !finitef(rho[k]) || v[k] < 0.0f || !(vp[k] > 0.0f) || !(rho[k] > 0.0f))
-      valid = false;
+    if (!finitef(vk) || !finitef(pk) || !finitef(rk) || vk < 0.0f || !(pk > 0.0f) || !(rk > 0.0f)) bad = true;
+    if (!(vk == 0.0f)) first = min(first, k);
+    v[k] = vk; vp[k] = pk; rho[k] = rk;
+    float drda = 0.0f, dadb = 0.0f;
+    brocher_deriv(pk, vk, drda, dadb);
+    chainrule[(size_t)k * ncol + col] = make_float2(dadb, drda);
+    // the grid nodes, from which the root search rebuilds the flattened
+    // sublayers of columns without fluid nodes (LayerView::layer)
+    if (nodes) nodes[(size_t)col * nz + k] = make_float4(pk, vk, rk, 0.0f);
   }
-  int nw = 0;
-  while (nw < nz - 1 && v[nw] == 0.0f) ++nw;
-  for (int k = nw; k < nz; ++k)
-    if (!(v[k] > 0.0f)) valid = false;
+  const int nw = min((int)__reduce_min_sync(FULL, (unsigned)first), nz - 1);  // leading fluid nodes
+  __syncwarp();
+  for (int k = nw + lane; k < nz; k += 32)
+    if (!(v[k] > 0.0f)) bad = true;
+  const bool valid = !__any_sync(FULL, bad);
   if (nodefeat) {  // proposal-network input: 64 nodes x (vs, vp, rho, thickness), normalised
-    for (int i = 0; i < FEAT_NODES; ++i) {
+    for (int i = lane; i < FEAT_NODES; i += 32) {
       const int k = i < nz ? i : nz - 1;
       const float thk = (i < nz - 1) ? dep[i + 1] - dep[i] : 0.0f;
       nodefeat[(size_t)col * FEAT_NODES + i] = make_float4(v[k] / 4.5f, vp[k] / 8.0f, rho[k] / 3.3f, thk / 5.0f);
     }
   }
-  for (int k = 0; k < nz; ++k) {
-    float drda = 0.0f, dadb = 0.0f;
-    brocher_deriv(vp[k], v[k], drda, dadb);
-    chainrule[(size_t)k * ncol + col] = make_float2(dadb, drda);
-  }
-  // grid2LayerModel (SurfaceWave.cpp:113-155), fluid nodes merged into one layer
-  float th[LMAX], a[LMAX], b[LMAX], r[LMAX], rR[LMAX], rL[LMAX];
-  const int n = 4;
-  int L, istart, k = 0;
-  if (nw > 0) {
-    L = (nz - nw) + (nz - nw - 1) * 3 + 1;
-    istart = nw;
-    th[0] = fsub(dep[nw], dep[0]);
-    r[0] = rho[0];
-    b[0] = 0.0f;
-    a[0] = vp[0];
-    k = 1;
-  } else {
-    L = nz + (nz - 1) * 3;
-    istart = 0;
-  }
-  for (int i = istart; i < nz - 1; ++i) {
-    const float thk = fdiv(fsub(dep[i + 1], dep[i]), (float)n);
-    const float dvp = fsub(vp[i + 1], vp[i]), dvs = fsub(v[i + 1], v[i]), drh = fsub(rho[i + 1], rho[i]);
-    for (int j = 0; j < n; ++j) {
-      const float w = (float)(2 * j + 1);
-      th[k] = thk;
-      a[k] = (float)dadd((double)vp[i], ddiv((double)fmul(w, dvp), 2.0 * n));
-      b[k] = (float)dadd((double)v[i], ddiv((double)fmul(w, dvs), 2.0 * n));
-      r[k] = (float)dadd((double)rho[i], ddiv((double)fmul(w, drh), 2.0 * n));
-      ++k;
+  // grid2LayerModel (SurfaceWave.cpp:113-155), fluid nodes merged into one
+  // layer; sublayer j of node interval i, its flattening, surfdisp96's
+  // extremal velocities
+  const int top = nw > 0 ? 1 : 0, L = 4 * (nz - nw) - 3 + top;
+  auto thickness = [&](int m) {  // of layer m < L - 1
+    if (m < top) return fsub(dep[nw], dep[0]);
+    const int i = nw + ((m - top) >> 2);
+    return fdiv(fsub(dep[i + 1], dep[i]), 4.0f);
+  };
+  const bool table = dl && nw == 0;          // the depth grid's flattening
+  const bool keep = nw > 0 || !nodes;        // the root search reads this column's layer tables
+  float key = 1.e20f, ka = 0.0f, kb = 0.0f;  // slowest layer so far: key velocity, its a and b
+  int kidx = 0x7fffffff;
+  float betmx = -1.e20f, b_top = 0.0f;
+  for (int m = lane; m < L; m += 32) {
+    float th, a, b, r;
+    if (m == L - 1) {
+      th = 0.0f; a = vp[nz - 1]; b = v[nz - 1]; r = rho[nz - 1];
+    } else if (m < top) {
+      th = thickness(m); a = vp[0]; b = 0.0f; r = rho[0];
+    } else {
+      const int i = nw + ((m - top) >> 2), j = (m - top) & 3;
+      const float wgt = (float)(2 * j + 1);
+      th = thickness(m);
+      a = (float)dadd((double)vp[i], ddiv((double)fmul(wgt, fsub(vp[i + 1], vp[i])), 8.0));
+      b = (float)dadd((double)v[i], ddiv((double)fmul(wgt, fsub(v[i + 1], v[i])), 8.0));
+      r = (float)dadd((double)rho[i], ddiv((double)fmul(wgt, fsub(rho[i + 1], rho[i])), 8.0));
     }
+    lay0[(size_t)col * Lmax + m] = make_float4(th, a, b, r);
+    float rR = r, rL = r;
+    if (sphere) {
+      DepthLayer q;
+      if (table) {
+        q = dl[m];
+      } else {
+        double dr = 0.0;  // in layer order, as one running sum
+        for (int k = 0; k < m; ++k) dr = dadd(dr, (double)thickness(k));
+        q = flatten_layer(dr, th, m == 0, m == L - 1);
+      }
+      th = q.d;
+      a = (float)dmul((double)a, q.tmp);
+      b = (float)dmul((double)b, q.tmp);
+      rR = fmul(r, q.fR);
+      rL = fmul(r, q.fL);
+    }
+    if (keep) {
+      const size_t o = layer_index(L - 1 - m, ncol, col, Lmax);
+      layR[o] = make_float4(th, a, b, rR);
+      layL[o] = make_float4(th, a, b, rL);
+    }
+    const float kv = b > 0.01f ? b : a;  // a fluid layer's P velocity
+    if (kv < key) { key = kv; ka = a; kb = b; kidx = m; }
+    if (b > betmx) betmx = b;
+    if (m == 0) b_top = b;
   }
-  th[L - 1] = 0.0f;
-  a[L - 1] = vp[nz - 1];
-  b[L - 1] = v[nz - 1];
-  r[L - 1] = rho[nz - 1];
-  for (int m = 0; m < L; ++m) lay0[(size_t)col * Lmax + m] = make_float4(th[m], a[m], b[m], r[m]);
-  // the grid nodes, from which the root search rebuilds the flattened
-  // sublayers of columns without fluid nodes (LayerView::layer)
-  if (nodes)
-    for (int k2 = 0; k2 < nz; ++k2) nodes[(size_t)col * nz + k2] = make_float4(vp[k2], v[k2], rho[k2], 0.0f);
-  ColInfo ci;
-  ci.L = L;
-  ci.nw = nw;
-  ci.valid = valid ? 1 : 0;
-  sd96_setup(L, sphere, th, a, b, r, rR, rL, ci);
-  write_layers(L, ncol, col, Lmax, th, a, b, rR, rL, layR, layL);
-  info[col] = ci;
+  // the first layer with the smallest key velocity
+  for (int o = 16; o > 0; o >>= 1) {
+    const float k2 = __shfl_xor_sync(FULL, key, o), a2 = __shfl_xor_sync(FULL, ka, o), b2 = __shfl_xor_sync(FULL, kb, o);
+    const int i2 = __shfl_xor_sync(FULL, kidx, o);
+    if (k2 < key || (k2 == key && i2 < kidx)) { key = k2; ka = a2; kb = b2; kidx = i2; }
+    const float m2 = __shfl_xor_sync(FULL, betmx, o);
+    if (m2 > betmx) betmx = m2;
+  }
+  if (lane == 0) {
+    ColInfo ci;
+    ci.L = L;
+    ci.nw = nw;
+    ci.valid = valid ? 1 : 0;
+    ci.llw = (b_top <= 0.0f) ? 2 : 1;
+    float cc1 = !(kb > 0.01f) ? key : gtsolh(ka, kb);
+    cc1 = fmul(0.95f, cc1);
+    cc1 = fmul(0.90f, cc1);
+    ci.cc = (double)cc1;
+    ci.betmx = betmx;
+    ci.pad_ = 0.0f;
+    info[col] = ci;
+  }
 }
 
 // k_prep_layers: layered models (surfdisp96_ input) -> layer models
@@ -313,36 +383,32 @@ __global__ void k_prep_layers(int nmodel, int nlayer, const float* __restrict__ 
 
 // The flattening of the standard sublayer grid (no fluid nodes) of a depth
 // vector: thicknesses as grid2LayerModel makes them (4 per node interval,
-// SurfaceWave.cpp:113-155), then sphere()'s loop (surfdisp96.f:499-571,
-// ar = 6370) in the same arithmetic as sd96_setup; one thread.
+// SurfaceWave.cpp:113-155), their running sum, then sphere() layer by layer
+// in the same arithmetic as sd96_setup; one block.
 __global__ void k_depth_table(int nz, const float* __restrict__ depth, int sphere, DepthLayer* __restrict__ dl) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
   const int L = 4 * nz - 3;
-  const double ar = 6370.0;
-  double dr = 0.0, r0 = ar;
-  for (int m = 0; m < L; ++m) {
-    float th;
-    if (m == L - 1) th = sphere ? 1.0f : 0.0f;  // sphere(): the half-space counts 1 km in the depth sum
-    else {
-      const int i = m >> 2;
-      th = fdiv(fsub(depth[i + 1], depth[i]), 4.0f);
+  __shared__ float th[LMAX];
+  __shared__ double dr[LMAX];
+  for (int m = threadIdx.x; m < L; m += blockDim.x) {
+    const int i = m >> 2;
+    th[m] = m == L - 1 ? 0.0f : fdiv(fsub(depth[i + 1], depth[i]), 4.0f);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double d = 0.0;
+    for (int m = 0; m < L; ++m) {
+      dr[m] = d;
+      d = dadd(d, (double)th[m]);
     }
+  }
+  __syncthreads();
+  for (int m = threadIdx.x; m < L; m += blockDim.x) {
     DepthLayer q;
-    q.pad_ = 0.0f;
     if (sphere) {
-      dr = dadd(dr, (double)th);
-      const double r1 = dsub(ar, dr);
-      const double z0 = dmul(ar, log(ddiv(ar, r0)));
-      const double z1 = dmul(ar, log(ddiv(ar, r1)));
-      q.d = (m == L - 1) ? 0.0f : (float)dsub(z1, z0);
-      q.tmp = ddiv(dadd(ar, ar), dadd(r0, r1));
-      const float btp = (float)q.tmp;
-      q.fR = (float)pow((double)btp, (double)(-2.275f));
-      const float b2 = fmul(btp, btp), b4 = fmul(b2, b2), b5 = fmul(b4, btp);
-      q.fL = fdiv(1.0f, b5);
-      r0 = r1;
+      q = flatten_layer(dr[m], th[m], m == 0, m == L - 1);
     } else {
-      q.d = th;
+      q.pad_ = 0.0f;
+      q.d = th[m];
       q.tmp = 1.0;
       q.fR = 1.0f;
       q.fL = 1.0f;
@@ -1701,15 +1767,16 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
   ctx->launches = 0;
   if (use_nodes) {
     ctx->launches += 1;
-    k_depth_table<<<1, 32, 0, st>>>(nz, ctx->depth_d.as<float>(), ctx->cfg.sphere, ctx->dltab.as<DepthLayer>());
+    k_depth_table<<<1, LMAX, 0, st>>>(nz, ctx->depth_d.as<float>(), ctx->cfg.sphere, ctx->dltab.as<DepthLayer>());
     CK(cudaGetLastError());
   }
   ctx->launches += 1;
-  k_prep<<<(ncol + 127) / 128, 128, 0, st>>>(ncol, ldi, nz, d_vs, d_vp, d_rho, ctx->depth_d.as<float>(), ctx->cfg.sphere,
+  k_prep<<<(ncol + PREP_COLS - 1) / PREP_COLS, 32 * PREP_COLS, 0, st>>>(ncol, ldi, nz, d_vs, d_vp, d_rho, ctx->depth_d.as<float>(), ctx->cfg.sphere,
                                              Lmax, ctx->layR.as<float4>(), ctx->layL.as<float4>(),
                                              ctx->lay0.as<float4>(), ctx->info.as<ColInfo>(),
                                              ctx->chainrule.as<float2>(), wantfeat ? ctx->nodefeat.as<float4>() : nullptr,
-                                             use_nodes ? ctx->nodes.as<float4>() : nullptr);
+                                             use_nodes ? ctx->nodes.as<float4>() : nullptr,
+                                             use_nodes ? ctx->dltab.as<DepthLayer>() : nullptr);
   CK(cudaGetLastError());
   if (timing) CK(cudaEventRecord(ctx->ev[1], st));
   if (useprop) {
@@ -2579,17 +2646,18 @@ int ragged_enqueue(swdk_ragged* R, cudaStream_t st, bool timing) {
     const swdk_call& c = R->calls[i];
     if (use_nodes) {
       R->launches += 1;
-      k_depth_table<<<1, 32, 0, st>>>(M.nz, R->ctx[i]->depth_d.as<float>(), cfg.sphere,
+      k_depth_table<<<1, LMAX, 0, st>>>(M.nz, R->ctx[i]->depth_d.as<float>(), cfg.sphere,
                                       R->dltab.as<DepthLayer>() + M.dl0);
       CK(cudaGetLastError());
     }
     R->launches += 1;
-    k_prep<<<(M.ncol + 127) / 128, 128, 0, st>>>(
+    k_prep<<<(M.ncol + PREP_COLS - 1) / PREP_COLS, 32 * PREP_COLS, 0, st>>>(
         M.ncol, M.ncol, M.nz, c.d_vs, c.d_vp, c.d_rho, R->ctx[i]->depth_d.as<float>(), cfg.sphere, M.Lmax,
         R->layR.as<float4>() + M.lay0, R->layL.as<float4>() + M.lay0, R->lay0.as<float4>() + M.lay0,
         R->info.as<ColInfo>() + M.col0, R->chainrule.as<float2>() + M.crs0,
         R->useprop ? R->nodefeat.as<float4>() + M.col0 * FEAT_NODES : nullptr,
-        use_nodes ? R->nodes.as<float4>() + M.node0 : nullptr);
+        use_nodes ? R->nodes.as<float4>() + M.node0 : nullptr,
+        use_nodes ? R->dltab.as<DepthLayer>() + M.dl0 : nullptr);
     CK(cudaGetLastError());
   }
   if (timing) CK(cudaEventRecord(R->ev[1], st));
