@@ -972,7 +972,8 @@ __global__ void __launch_bounds__(128, SWDK_RETRY_MINB) k_retry(int ncol, const 
 cudaError_t roots_occupancy(int* per) {
   cudaError_t e = cudaFuncSetAttribute(k_roots_queue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROOTS_SMEM);
   const int cs = (int)coop_smem(COOP_MIN_G);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_roots_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_roots_coop<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_roots_coop<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_retry, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RETRY_SMEM);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, k_roots_queue, 128, ROOTS_SMEM);
   return e;
@@ -1025,10 +1026,10 @@ cudaError_t launch_roots(const RootsCall& c, int rblocks, int nsm, bool tuned, c
   const int G = tuned ? 1 : coop_lanes(c.nitems, nsm);
   if (G > 1) {
     const long long need = (c.nitems * G + 127) / 128;
-    k_roots_coop<<<(unsigned)std::max(1LL, std::min<long long>(need, 3LL * nsm)), 128, coop_smem(G), st>>>(
+    k_roots_coop<false><<<(unsigned)std::max(1LL, std::min<long long>(need, 3LL * nsm)), 128, coop_smem(G), st>>>(
         c.ncol, (int)c.nitems, G, c.order, c.chains, c.periods, c.layR, c.layL, c.info, c.refine, c.rtol, c.sngl,
         RETRY_DEFERRED, c.croot, c.cstat, c.queue, c.prop, c.retry_list, c.rctr, c.rcap, c.nevals, c.rg, c.nodes,
-        c.dl);
+        c.dl, nullptr);
   } else {
     k_roots_queue<<<(unsigned)std::max(1LL, std::min<long long>(rblocks, (c.nitems + 127) / 128)), 128, ROOTS_SMEM,
                     st>>>(c.ncol, (int)c.nitems, c.order, c.chains, c.periods, c.layR, c.layL, c.info, c.refine,
@@ -1479,6 +1480,7 @@ struct swdk_ctx {
   DevBuf layR, layL, lay0, info, chainrule, croot, cstat, nevals, depth_d, ierr, queue;
   DevBuf nodes, dltab;  // grid nodes and the depth grid's flattening (node-source root search)
   int roots_blocks = 0, nsm = 148;
+  bool coop_ready = false;  // the layered-model call's kernels are opted in to their shared memory
   DevBuf in_vs, in_vp, in_rho, out_vc, out_vout, out_kernel, out_status, in_misc;
   // learned bracket proposals
   swdk_mlp* net[2] = {nullptr, nullptr};  // 0: Rayleigh, 1: Love
@@ -2328,6 +2330,23 @@ int swdk_surfdisp96_batch(swdk_ctx* ctx, int nmodel, int nlayer, const float* th
   CK(cudaEventRecord(ctx->ev[1], st));
   CK(cudaEventRecord(ctx->ev[5], st));
   ctx->stats.kernel_launches = 2;
+  if (!ctx->coop_ready) {
+    int dev = 0, per = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, dev));
+    CK(roots_occupancy(&per));
+    ctx->coop_ready = true;
+  }
+  if (const int G = coop_lanes(nmodel, ctx->nsm); G > 1) {
+    CK(ctx->queue.ensure(sizeof(unsigned int)));
+    CK(cudaMemsetAsync(ctx->queue.p, 0, sizeof(unsigned int), st));
+    const long long need = ((long long)nmodel * G + 127) / 128;
+    k_roots_coop<true><<<(unsigned)std::min<long long>(need, 3LL * ctx->nsm), 128, coop_smem(G), st>>>(
+        nmodel, nmodel, G, nullptr, d_ch, d_t, ctx->layR.as<float4>(), ctx->layL.as<float4>(), ctx->info.as<ColInfo>(),
+        ctx->cfg.refine, ctx->cfg.rtol, ctx->cfg.sngl, RETRY_NONE, ctx->croot.as<double>(), ctx->cstat.as<int32_t>(),
+        ctx->queue.as<unsigned int>(), nullptr, nullptr, nullptr, 0u, ctx->nevals.as<unsigned long long>(),
+        RaggedMap{nullptr, nullptr, 0, nlayer}, nullptr, nullptr, ctx->ierr.as<int32_t>());
+  } else
   k_roots<<<dim3((nmodel + 127) / 128, 1), 128, 0, st>>>(nmodel, d_ch, d_t, ctx->layR.as<float4>(),
                                                          ctx->layL.as<float4>(), ctx->info.as<ColInfo>(),
                                                          ctx->cfg.refine, ctx->cfg.rtol, ctx->cfg.sngl, 0,

@@ -61,6 +61,72 @@ __device__ __forceinline__ Dunkin load_dunkin(const double* row) {
   return d;
 }
 
+// dltar4's and dltar1's own forms of a layer (surfdisp96.f:712-1095), for
+// layered models: the divisions, square roots and exponentials as dltar4 /
+// dltar1 write them
+__device__ __forceinline__ void vertical_ref(double wvno, double xk, double dpth, double& over, double& times,
+                                             double& cosv, double& ex) {
+  const double r = sqrt((wvno + xk) * fabs(wvno - xk)), p = r * dpth;
+  ex = 0.0;
+  if (wvno < xk) {
+    double s, c;
+    sincos(p, &s, &c);
+    over = s / r; times = -r * s; cosv = c;
+  } else if (wvno == xk) {
+    cosv = 1.0; over = dpth; times = 0.0;
+  } else {
+    ex = p;
+    const double fac = (p < 16.0) ? exp(-2.0 * p) : 0.0;
+    cosv = (1.0 + fac) * 0.5;
+    const double s = (1.0 - fac) * 0.5;
+    over = s / r; times = r * s;
+  }
+}
+
+__device__ __forceinline__ LayerCoef layer_coef_ref(const float4 ly, double wvno, double wvno2, double omega,
+                                                    double iom) {
+  LayerCoef k;
+  k.rho = ly.w;
+  k.irho = 1.0 / k.rho;
+  const double t = (double)ly.z * iom;
+  k.gammk = 2.0 * t * t;
+  k.gam = k.gammk * wvno2;
+  double w, x, cosp, pex, y, z, cosq, sex;
+  vertical_ref(wvno, omega / (double)ly.y, ly.x, w, x, cosp, pex);
+  vertical_ref(wvno, omega / (double)ly.z, ly.x, y, z, cosq, sex);
+  const double exa = pex + sex;
+  k.a0 = (exa < 60.0) ? exp(-exa) : 0.0;
+  k.cpcq = cosp * cosq; k.cpy = cosp * y; k.cpz = cosp * z; k.cqw = cosq * w; k.cqx = cosq * x;
+  k.xy = x * y; k.xz = x * z; k.wy = w * y; k.wz = w * z;
+  return k;
+}
+
+__device__ __forceinline__ RayVec rayleigh_start_ref(const float4 h, double wvno, double wvno2, double omega,
+                                                     double iom) {
+  const double a = h.y, b = h.z, rho1 = h.w;
+  const double xka = omega / a, xkb = omega / b;
+  const double ra = sqrt((wvno + xka) * fabs(wvno - xka)), rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
+  const double t = b * iom, gammk = 2.0 * t * t, gam = gammk * wvno2, gamm1 = gam - 1.0;
+  RayVec e;
+  e.e0 = rho1 * rho1 * (gamm1 * gamm1 - gam * gammk * ra * rb);
+  e.e1 = -rho1 * ra;
+  e.e2 = rho1 * (gamm1 - gammk * ra * rb);
+  e.e3 = rho1 * rb;
+  e.e4 = wvno2 - ra * rb;
+  return e;
+}
+
+__device__ __forceinline__ LoveCoef love_coef_ref(const float4 ly, double wvno, double omega) {
+  const double beta1 = ly.z, rho1 = ly.w;
+  LoveCoef k;
+  double ex;
+  k.xmu = rho1 * beta1 * beta1;
+  k.ixmu = 1.0 / k.xmu;
+  vertical_ref(wvno, omega / beta1, ly.x, k.y, k.z, k.cosq, ex);
+  return k;
+}
+
+// NORM 0: dltar4 as written (normalised at every layer by the reciprocal)
 template <int NORM>
 __device__ double coop_rayleigh(bool on, const LayerView& V, double wvno, double omga, int W, int l, double* rows) {
   double omega = omga;
@@ -70,7 +136,8 @@ __device__ double coop_rayleigh(bool on, const LayerView& V, double wvno, double
   const int hs = on ? V.L - 1 : 0, mlo = on ? V.llw - 1 : 0;
   double e0 = 0.0, e1 = 0.0, e2 = 0.0, e3 = 0.0, e4 = 0.0;
   if (on) {
-    const RayVec st = rayleigh_start(V.layer(hs), wvno, wvno2, omega, iom);
+    const RayVec st = NORM == 0 ? rayleigh_start_ref(V.get(hs), wvno, wvno2, omega, iom)
+                                : rayleigh_start(V.layer(hs), wvno, wvno2, omega, iom);
     e0 = st.e0; e1 = st.e1; e2 = st.e2; e3 = st.e3; e4 = st.e4;
   }
   const int n = hs - mlo;  // layers to propagate
@@ -79,7 +146,8 @@ __device__ double coop_rayleigh(bool on, const LayerView& V, double wvno, double
   for (int a = 0; a < nmax; a += W) {
     const int m = hs - 1 - a - l;
     if (m >= mlo && on) {
-      const LayerCoef k = layer_coef(V.layer(m), wvno, wvno2, omega, iom);
+      const LayerCoef k = NORM == 0 ? layer_coef_ref(V.get(m), wvno, wvno2, omega, iom)
+                                    : layer_coef(V.layer(m), wvno, wvno2, omega, iom);
       const Dunkin d = dunkin_entries(k, wvno2);
       double2* q = reinterpret_cast<double2*>(rows + (size_t)l * COOP_ROW);
       q[0] = make_double2(d.c11, d.c12);
@@ -112,12 +180,21 @@ __device__ double coop_rayleigh(bool on, const LayerView& V, double wvno, double
       dunkin_product(load_dunkin(rows + (size_t)i * COOP_ROW), e0, e1, e2, e3, e4);
       if (++since >= NORM || a + i == n - 1) {
         since = 0;
-        rayleigh_norm<NORM>(e0, e1, e2, e3, e4);
+        rayleigh_norm<NORM == 0 ? 4 : NORM>(e0, e1, e2, e3, e4);
       }
     }
     __syncwarp();
   }
-  if (on && V.llw != 1) return rayleigh_fluid_top(V.layer(0), wvno, omega, e0, e1);
+  if (on && V.llw != 1) {
+    if (NORM == 0) {
+      const float4 ly = V.get(0);
+      double w, x, cosp, ex;
+      vertical_ref(wvno, omega / (double)ly.y, ly.x, w, x, cosp, ex);
+      const double w0 = -(double)ly.w * w;
+      return cosp * e0 + w0 * e1;
+    }
+    return rayleigh_fluid_top(V.layer(0), wvno, omega, e0, e1);
+  }
   return e0;
 }
 
@@ -125,14 +202,21 @@ template <int NORM>
 __device__ double coop_love(bool on, const LayerView& V, double wvno, double omega, int W, int l, double* rows) {
   const int hs = on ? V.L - 1 : 0, mlo = on ? V.llw - 1 : 0;
   double e1 = 0.0, e2 = 0.0;
-  if (on) love_start(V.layer(hs), wvno, omega, e1, e2);
+  if (on && NORM == 0) {
+    const float4 h = V.get(hs);
+    const double beta1 = h.z, xkb = omega / beta1;
+    e1 = (double)h.w * sqrt((wvno + xkb) * fabs(wvno - xkb));
+    e2 = 1.0 / (beta1 * beta1);
+  } else if (on) {
+    love_start(V.layer(hs), wvno, omega, e1, e2);
+  }
   const int n = hs - mlo;
   const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);
   int since = 0;
   for (int a = 0; a < nmax; a += W) {
     const int m = hs - 1 - a - l;
     if (m >= mlo && on) {
-      const LoveCoef k = love_coef(V.layer(m), wvno, omega);
+      const LoveCoef k = NORM == 0 ? love_coef_ref(V.get(m), wvno, omega) : love_coef(V.layer(m), wvno, omega);
       double2* q = reinterpret_cast<double2*>(rows + (size_t)l * COOP_ROW);
       q[0] = make_double2(k.cosq, k.y);
       q[1] = make_double2(k.z, k.xmu);
@@ -150,7 +234,7 @@ __device__ double coop_love(bool on, const LayerView& V, double wvno, double ome
       t = q[2]; k.ixmu = t.x;
       const bool norm = ++since >= NORM || a + i == n - 1;
       if (norm) since = 0;
-      love_product<NORM>(k, norm, e1, e2);
+      love_product<NORM == 0 ? 4 : NORM>(k, norm, e1, e2);
     }
     __syncwarp();
   }
@@ -216,9 +300,12 @@ __device__ int coop_plan(ChainState& s, const ChainParams& P, const ChainIO& io,
   return n;
 }
 
-// k_roots_coop: G lanes (4, 8, 16 or 32) per work item of k_roots_queue.  The group's first lane runs the chain's state
+// k_roots_coop: G lanes (4, 8, 16 or 32) per work item of k_roots_queue; with
+// REF, per layered model, one chain each, the secular functions as dltar1 /
+// dltar4 write them, and the chains' ierr.  The group's first lane runs the chain's state
 // machine; an evaluation takes all of the group's lanes, for one trial
 // velocity or for several planned together (W = G / number lanes each).
+template <bool REF>
 __global__ void __launch_bounds__(128, 3) k_roots_coop(int ncol, int nitems, int G, const int* __restrict__ order,
                                                        const ChainDesc* __restrict__ chains,
                                                        const double* __restrict__ periods,
@@ -232,7 +319,8 @@ __global__ void __launch_bounds__(128, 3) k_roots_coop(int ncol, int nitems, int
                                                        unsigned int* __restrict__ retry_count, unsigned int retry_cap,
                                                        unsigned long long* __restrict__ nevals, RaggedMap rg,
                                                        const float4* __restrict__ nodes,
-                                                       const DepthLayer* __restrict__ dl) {
+                                                       const DepthLayer* __restrict__ dl,
+                                                       int32_t* __restrict__ ierr_out) {
   extern __shared__ __align__(16) unsigned char coop_sm[];
   __shared__ unsigned long long phase_ev[NPHASE_EV];
   __shared__ unsigned long long blk_ev[5];
@@ -282,7 +370,7 @@ __global__ void __launch_bounds__(128, 3) k_roots_coop(int ncol, int nitems, int
             lstride = M.Lmax;
             o_col = M.col0; o_lay = M.lay0; o_root = M.root0; o_node = M.node0; o_dl = M.dl0;
           } else {
-            cd = chains[order[item_of / ncol]];
+            cd = chains[REF ? 0 : order[item_of / ncol]];
             col = item_of % ncol;
           }
           const ColInfo ci = info[o_col + col];
@@ -293,11 +381,12 @@ __global__ void __launch_bounds__(128, 3) k_roots_coop(int ncol, int nitems, int
               outp[(size_t)i * mcol] = 0.0;
               stp[(size_t)i * mcol] = ST_NAN_INPUT;
             }
+            if (REF) ierr_out[col] = 1;
             continue;
           }
           LayerView& V = g.V;
           V.lay = ((cd.iwave == 2) ? layR : layL) + o_lay;
-          V.fast = 1;
+          V.fast = REF ? 0 : 1;
           V.ncol = mcol;
           V.col = col;
           V.lstride = lstride;
@@ -328,6 +417,7 @@ __global__ void __launch_bounds__(128, 3) k_roots_coop(int ncol, int nitems, int
           have = true;
         }
         if (!chain_advance(s, P, io)) {  // chain finished
+          if (REF) ierr_out[g.V.col] = s.ierr;
           if (s.iterlim)
             for (int i = 0; i < P.nmode * P.kmax; ++i)
               if (io.st[(size_t)i * io.ostride] == ST_OK) io.st[(size_t)i * io.ostride] = ST_ITER_LIMIT;
@@ -386,17 +476,19 @@ __global__ void __launch_bounds__(128, 3) k_roots_coop(int ncol, int nitems, int
       double f = 0.0;
       if (W == 1) {
         const LayerView V = g.V;  // in registers: read at every layer
-        if (mine) f = secular_fast(V, g.P.iwave, refine, wv, om);
+        if (mine) f = REF ? secular(V, g.P.iwave, wv, om) : secular_fast(V, g.P.iwave, refine, wv, om);
       } else {
         double* rows = wbuf + (size_t)(lane - l) * COOP_ROW;
         if (__ballot_sync(FULL, ray)) {
-          const double v = refine == 0 ? coop_rayleigh<1>(ray, g.V, wv, om, W, l, rows)
-                                       : coop_rayleigh<4>(ray, g.V, wv, om, W, l, rows);
+          const double v = REF           ? coop_rayleigh<0>(ray, g.V, wv, om, W, l, rows)
+                           : refine == 0 ? coop_rayleigh<1>(ray, g.V, wv, om, W, l, rows)
+                                         : coop_rayleigh<4>(ray, g.V, wv, om, W, l, rows);
           if (ray) f = v;
         }
         if (__ballot_sync(FULL, lov)) {
-          const double v = refine == 0 ? coop_love<1>(lov, g.V, wv, om, W, l, rows)
-                                       : coop_love<4>(lov, g.V, wv, om, W, l, rows);
+          const double v = REF           ? coop_love<0>(lov, g.V, wv, om, W, l, rows)
+                           : refine == 0 ? coop_love<1>(lov, g.V, wv, om, W, l, rows)
+                                         : coop_love<4>(lov, g.V, wv, om, W, l, rows);
           if (lov) f = v;
         }
       }
