@@ -83,35 +83,54 @@ __global__ void k_fmst_refvel(Grid G, int npair, const int32_t* __restrict__ cp,
     }
 }
 
-// fmst.f90:108-310: each warp marches `lanes / per` pairs at a time, `per`
-// lanes per pair (1: one lane solves all four neighbours of an accepted
-// node; 4: four lanes solve one each, lane 0 of the four owns the heap; 8:
-// lane 0 owns the heap and lanes 1-4 solve), and
-// loops over the pairs; the grid holds the number of warps per SM that keeps
-// the marching fronts in L1.
-__global__ void __launch_bounds__(128) k_fmst_travel(Grid G, int npair, int lanes, int per,
-                                                     const int32_t* __restrict__ cp, const float* __restrict__ srcx,
-                                                     const float* __restrict__ srcz, const int32_t* __restrict__ pslot,
+// fmst.f90:108-310, one lane per pair: `lanes` lanes of each warp march one
+// pair each and loop over the pairs.
+__global__ void __launch_bounds__(128) k_fmst_travel(Grid G, int npair, int lanes, const int32_t* __restrict__ cp,
+                                                     const float* __restrict__ srcx, const float* __restrict__ srcz,
+                                                     const int32_t* __restrict__ pslot,
                                                      const float* __restrict__ slwn, const float* __restrict__ risti_c,
                                                      const float* __restrict__ risti_r, Scratch S,
                                                      unsigned int* __restrict__ n_overflow, int smem_cap) {
     extern __shared__ __align__(16) FHeap sheap[];
     const int lane = threadIdx.x & 31;
     if (lane >= lanes) return;
-    const int ppw = lanes / per, slot = lane / per;
-    const int g4 = lane % per;        // lane within the pair's group
-    if (per == 8 && g4 > 4) return;   // groups of eight use five lanes
-    const unsigned gmask = per == 1 ? (1u << lane) : per == 4 ? (0xFu << (lane & ~3)) : (0x1Fu << (lane & ~7));
     // with smem_cap > 0 each pair's heap (1..smem_cap) lives in shared memory;
     // a band that outgrows it flags the pair for a second pass with the full
     // heap in global memory
-    FHeap* hp = smem_cap > 0 ? sheap + (size_t)(((threadIdx.x >> 5) * ppw + slot) * ((smem_cap + 2) & ~1)) : nullptr;
+    FHeap* hp = smem_cap > 0 ? sheap + (size_t)(((threadIdx.x >> 5) * lanes + lane) * ((smem_cap + 2) & ~1)) : nullptr;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;; warp += nwarps) {
-        const int p = warp * ppw + slot;
-        if (p >= npair) return;  // the same for the lanes of one pair
-        march_pair(G, p, cp[p], srcx, srcz, pslot, slwn, risti_c, risti_r, S, n_overflow, hp, smem_cap,
-                   per == 1 ? 0 : per == 4 ? 2 : 3, g4, gmask);
+        const int p = warp * lanes + lane;
+        if (p >= npair) return;
+        march_pair(G, p, cp[p], srcx, srcz, pslot, slwn, risti_c, risti_r, S, n_overflow, hp, smem_cap, 0, 0,
+                   1u << lane);
+    }
+}
+
+// The same with two pairs per warp (March::march_half), one warp per block;
+// the pairs go round the resident warps.
+template <bool SMEM>
+__global__ void __launch_bounds__(32) k_fmst_travel_half(Grid G, int npair, const int32_t* __restrict__ cp,
+                                                         const float* __restrict__ srcx,
+                                                         const float* __restrict__ srcz,
+                                                         const int32_t* __restrict__ pslot,
+                                                         const float* __restrict__ slwn,
+                                                         const float* __restrict__ risti_c,
+                                                         const float* __restrict__ risti_r, Scratch S,
+                                                         unsigned int* __restrict__ n_overflow, int smem_cap) {
+    extern __shared__ __align__(16) FHeap sheap[];
+    const int half = threadIdx.x >> 4;
+    for (int p0 = 2 * blockIdx.x; p0 < npair; p0 += 2 * gridDim.x) {
+        const bool mine = p0 + half < npair;
+        const int p = mine ? p0 + half : p0;
+        const unsigned mask = mine ? 0xffffu << (16 * half) : 0u;
+        if (SMEM)
+            march_pair<1>(G, p, cp[p], srcx, srcz, pslot, slwn, risti_c, risti_r, S, n_overflow,
+                          sheap + (size_t)half * ((smem_cap + 2) & ~1), smem_cap, 2, threadIdx.x & 15, mask);
+        else
+            march_pair<0>(G, p, cp[p], srcx, srcz, pslot, slwn, risti_c, risti_r, S, n_overflow, nullptr, 0, 2,
+                          threadIdx.x & 15, mask);
+        __syncwarp();
     }
 }
 
@@ -192,12 +211,12 @@ struct swdk_fmst {
     unsigned int* d_overflow = nullptr;
     size_t budget = (size_t)16 << 30;
     // marching layout (measured on B200 with the 3040-pair, 33 x 36 survey):
-    // 8 lanes per warp as two pairs of four lanes, 12 warps per SM, heaps of
-    // 1.5 (nnx + nnz) entries in shared memory
+    // two pairs per warp, 12 warps per SM, heaps of 1.5 (nnx + nnz) entries in
+    // shared memory
     int lanes = 8;
     int warps_per_sm = 12; // resident marching warps per SM (0: one warp per pair group)
     int smem_heap = -1;    // heap entries per pair in shared memory (0: global heap, -1: automatic)
-    int per = 4;           // lanes per pair (1 or 4)
+    int per = 4;           // lanes per pair asked for: 1, or more (half a warp marches the pair)
     int nsm = 148;
     double ms_last = 0.0;
     int max_band = 0, overflow_pairs = 0;  // of the last call
@@ -223,6 +242,7 @@ extern "C" int swdk_fmst_create(swdk_fmst** out, int device, const swdk_fmst_gri
     if (e != cudaSuccess) { delete f; return SWDK_E_CUDA; }
     cudaDeviceGetAttribute(&f->nsm, cudaDevAttrMultiProcessorCount, device);
     cudaFuncSetAttribute(k_fmst_travel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(k_fmst_travel_half<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     // fmst_init (fmst.f90:27-64) and the r*sin(colatitude) tables
     f->G = make_grid(grid->nx, grid->ny, grid->goxd, grid->gozd, grid->dvxd, grid->dvzd);
     make_risti(f->G, f->risti_c, f->risti_r);
@@ -413,7 +433,7 @@ extern "C" int swdk_fmst_pairs(swdk_fmst* f, int npairs, const int32_t* slot, co
     // is a front across the grid), within 160 KB of shared memory per SM
     int smem_heap = f->smem_heap;
     if (smem_heap < 0) {
-        const int pairs_per_sm = std::max(1, (f->warps_per_sm > 0 ? f->warps_per_sm : 16) * (f->lanes / f->per));
+        const int pairs_per_sm = std::max(1, (f->warps_per_sm > 0 ? f->warps_per_sm : 16) * (f->per == 1 ? f->lanes : 2));
         smem_heap = (int)std::min<size_t>((size_t)(1.5 * (G.nnx + G.nnz)), (160u << 10) / (8u * pairs_per_sm) - 2);
         if (smem_heap < 256) smem_heap = 0;
     }
@@ -489,7 +509,7 @@ extern "C" int swdk_fmst_pairs(swdk_fmst* f, int npairs, const int32_t* slot, co
             k_fmst_refvel<<<dim3(8, np), 256, 0, st>>>(G, np, dcp, d_srcx, d_srcz, d_pslot, d_used, d_vc, S.rvel,
                                                       S.rslw, S.geo);
             {
-                const int lanes = f->lanes, ppw = lanes / f->per;
+                const int ppw = f->per == 1 ? f->lanes : 2;  // pairs marched by a warp at a time
                 int warps = (np + ppw - 1) / ppw;
                 if (f->warps_per_sm > 0) warps = std::min(warps, f->warps_per_sm * f->nsm);
                 const size_t shm = smem ? (size_t)ppw * hstride * sizeof(FHeap) : 0;
@@ -499,10 +519,17 @@ extern "C" int swdk_fmst_pairs(swdk_fmst* f, int npairs, const int32_t* slot, co
                     const int wps = f->warps_per_sm > 0 ? f->warps_per_sm : 32;
                     carve = (int)std::min<size_t>(100, (shm * wps * 100 + 228 * 1024 - 1) / (228 * 1024));
                 }
-                cudaFuncSetAttribute(k_fmst_travel, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
-                k_fmst_travel<<<warps, 32, shm, st>>>(G, np, lanes, f->per, dcp, d_srcx, d_srcz, d_pslot, slwn,
-                                                      f->d_risti_c,
-                                                      f->d_risti_r, S, f->d_overflow, smem ? (int)cap : 0);
+                if (f->per == 1) {
+                    cudaFuncSetAttribute(k_fmst_travel, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
+                    k_fmst_travel<<<warps, 32, shm, st>>>(G, np, f->lanes, dcp, d_srcx, d_srcz, d_pslot, slwn,
+                                                          f->d_risti_c, f->d_risti_r, S, f->d_overflow,
+                                                          smem ? (int)cap : 0);
+                } else {
+                    const auto k = smem ? k_fmst_travel_half<true> : k_fmst_travel_half<false>;
+                    cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
+                    k<<<warps, 32, shm, st>>>(G, np, dcp, d_srcx, d_srcz, d_pslot, slwn, f->d_risti_c, f->d_risti_r, S,
+                                              f->d_overflow, smem ? (int)cap : 0);
+                }
             }
             if (nrc > 0)
                 k_fmst_rays<<<(int)((nrc + 127) / 128), 128, 0, st>>>(G, (int)nrc, dcr, dcq, dcp, d_srcx, d_srcz,

@@ -434,52 +434,256 @@ struct March {
     }
 
 #if defined(__CUDA_ARCH__)
-    // march() by the lanes of a group (lane g4 of the group, mask gmask): the
-    // lanes base .. base+3 solve the trial times of the neighbours x-1, x+1,
-    // z-1, z+1; lane 0 of the group owns the heap, sifts it down meanwhile
-    // and applies the four updates in the reference's order.  base = 0: lane
-    // 0 also solves x-1 (groups of four lanes); base = 1: lane 0 only keeps
-    // the heap, so its sift-down overlaps the solves (groups of eight lanes,
-    // five of them active).  Every lane runs this with the same March state;
-    // only lane 0's heap fields are live.
-    __device__ void march_coop(bool refined, const PairGeo& g, int g4, unsigned gmask, int base) {
-        const int lead = __ffs(gmask) - 1;
-        const int q = g4 - base;  // neighbour this lane solves (0..3), or none
-        const int dz = q == 2 ? -1 : (q == 3 ? 1 : 0), dx = q == 0 ? -1 : (q == 1 ? 1 : 0);
-        for (;;) {
-            int go = 0, pk = 0;
-            float tacc = 0.0f;
-            if (g4 == 0 && ntr > 0 && !overflow) {
-                const FHeap root = heap[1];
-                const int iz = (root.node & 0xFFFF) + 1, ix = (root.node >> 16) + 1;
-                nd[idx(iz, ix)].s = 0;
-                go = (refined && at_refined_side(g, iz, ix)) ? 0 : 1;
-                pk = root.node;
-                tacc = root.key;
-            }
-            go = __shfl_sync(gmask, go, lead);
-            if (!go) break;
-            pk = __shfl_sync(gmask, pk, lead);
-            tacc = __shfl_sync(gmask, tacc, lead);
-            __syncwarp(gmask);
-            const int iz = (pk & 0xFFFF) + 1, ix = (pk >> 16) + 1;
-            float t = 0.0f;
-            int s = -2;
-            if (q >= 0 && q < 4) s = solve_neighbour(iz, ix, tacc, dz, dx, &t);
-            if (g4 == 0) downtree();
-            const int s0 = __shfl_sync(gmask, s, lead + base), s1 = __shfl_sync(gmask, s, lead + base + 1),
-                      s2 = __shfl_sync(gmask, s, lead + base + 2), s3 = __shfl_sync(gmask, s, lead + base + 3);
-            const float t0 = __shfl_sync(gmask, t, lead + base), t1 = __shfl_sync(gmask, t, lead + base + 1),
-                        t2 = __shfl_sync(gmask, t, lead + base + 2), t3 = __shfl_sync(gmask, t, lead + base + 3);
-            if (g4 == 0) {
-                apply(iz, ix - 1, s0, t0);
-                apply(iz, ix + 1, s1, t1);
-                apply(iz - 1, ix, s2, t2);
-                apply(iz + 1, ix, s3, t3);
-            }
-            __syncwarp(gmask);
+    // -- the march by half a warp -------------------------------------------
+    // Two pairs per warp, 16 lanes each; the lanes of a half hold the same
+    // March, and the halves go through the same instructions (`on`: this half
+    // takes part), so one instruction stream serves both.
+    //
+    // An accepted node is a dependent chain of some hundred instructions at
+    // four cycles or more each, which is what bounds the march (a pair alone
+    // and 3040 pairs together take nearly the same time): the root, the
+    // stencils' loads, the sift-down, the trial times, up to four heap
+    // updates.  So the chain is kept short:
+    //   * lane 4q + (a + 2b) of a half solves quadrant (a, b) of neighbour q
+    //     with straight-line code;
+    //   * the loads of the next root's stencils start one node ahead: the next
+    //     root is nearly always the smaller child of this one, and all that a
+    //     node's acceptance changes in another's stencils is that node itself
+    //     (patched when used; a wrong guess, 1 in 15 000, loads again);
+    //   * a sift-down loads four tree levels at once, and each lane tells from
+    //     two votes whether it lies on the path and what it writes; an update
+    //     loads its whole path to the root;
+    //   * the neighbours' heap positions are loaded together, before the trial
+    //     times, and again only after an update that moved other entries.
+    static __device__ __forceinline__ unsigned half_ballot(bool p, int sh) {
+        return (__ballot_sync(0xffffffffu, p) >> sh) & 0xffffu;
+    }
+
+    // the entry (key, pk) of node n from free slot tpc up to its place
+    // (addtree's and updtree's loop): lane j holds the ancestor tpc >> (j + 1)
+    // and writes slot tpc >> j.  Returns whether other entries moved.
+    __device__ __forceinline__ bool sift_up_half(bool on, int tpc, int pk, int n, float key, int l, int sh) {
+        const int slot = tpc >> l, anc = slot >> 1;
+        FHeap h{0.0f, 0};
+        bool below = false;
+        if (on && anc >= 1) {
+            h = heap[anc];
+            below = key < h.key;
         }
-        __syncwarp(gmask);
+        const unsigned up = half_ballot(below, sh);
+        const int moves = __ffs(~up) - 1;  // ancestors from the bottom with key < theirs
+        if (on && l <= moves) {
+            const bool self = l == moves;
+            heap[slot] = self ? FHeap{key, pk} : h;
+            FNode* d = &nd[self ? n : lin(h.node)];
+            d->s = slot;
+            if (self) d->t = key;
+        }
+        __syncwarp();
+        return on && moves > 0;
+    }
+
+    // a node that joins the heap (addtree); false when the heap is full
+    __device__ __forceinline__ bool grow_half(bool on, int n, float key, int l) {
+        if (on && ntr >= cap) {
+            overflow = true;
+            if (l == 0) nd[n].t = key;
+            return false;
+        }
+        if (on) {
+            ++ntr;
+            ntr_max = max(ntr_max, ntr);
+        }
+        return on;
+    }
+
+    // downtree.  Lane p holds the children of local node p of the four-level
+    // subtree under the hole (local node 1): which child the reference would
+    // take (the left one unless its key is the greater) and whether that
+    // child moves up (its key below the last entry's).  A lane is on the path
+    // if all its ancestors move and lead to it (amask: their bits; rmask: the
+    // ones that lead right); it writes the child that moves into its node, or
+    // the last entry where the path ends.
+    __device__ __forceinline__ void down_half(bool on, int l, int sh, int lv, unsigned amask, unsigned rmask) {
+        bool go = on && ntr > 1;
+        const FHeap last = go ? heap[ntr] : FHeap{0.0f, 0};
+        if (on) ntr = ntr - 1;
+        int hole = 1;
+        while (__any_sync(0xffffffffu, go)) {
+            const int g = (hole << lv) + l - (1 << lv);  // heap slot of this lane's local node
+            const int c0 = 2 * g;
+            float4 cc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const bool mine = go && l >= 1, has = mine && c0 <= ntr;
+            if (has) cc = *reinterpret_cast<const float4*>(&heap[c0]);
+            const bool right = c0 < ntr && cc.x > cc.z;
+            const float ck = right ? cc.z : cc.x;
+            const bool moves = has && ck < last.key;
+            const unsigned rm = half_ballot(right, sh), mm = half_ballot(moves, sh);
+            const bool path = mine && (mm & amask) == amask && (rm & amask) == rmask;
+            if (path) {
+                const FHeap w{moves ? ck : last.key, moves ? __float_as_int(right ? cc.w : cc.y) : last.node};
+                heap[g] = w;
+                nd[lin(w.node)].s = g;
+            }
+            // the path goes on below the subtree when it moves at its fourth level
+            const unsigned leaf = half_ballot(path && moves && l >= 8, sh);
+            go = leaf != 0u;
+            const int u = __ffs(leaf) - 1;
+            hole = (hole << 4) + 2 * (u - 8) + (int)((rm >> (u & 15)) & 1u);
+        }
+        __syncwarp();
+    }
+
+    // The candidate of fouds2 (fmm.f90:437-610) for one quadrant from its
+    // two sides: xo / zo order of the x / z side (0 none), (tj, tj2), (tk,
+    // tk2) their times.  The reference's five formulas differ in factors
+    // that are selected here; factors of 1, 2 and the division by 1 are
+    // exact, so every case keeps the reference's bits (root2, root1 above).
+    // NaN when the quadrant gives none (fminf then takes the other operand).
+    __device__ __forceinline__ float quadrant(int xo, int zo, float tj, float tj2, float tk, float tk2, float slown,
+                                              float risti) const {
+        const float ri = EARTH;
+        const float U = ri * dnx, Z = risti * dnz;
+        const float x2 = 4.0f * tj - tj2, z2 = 4.0f * tk - tk2;
+        const float s2 = sq(slown);
+        const bool xx = xo == 2, zz = zo == 2, both = xo > 0 && zo > 0;
+        // two-sided
+        const float Ux = xx ? 2.0f * U : U, Vz = zz ? 2.0f * Z : Z;
+        const bool swap = xx && !zz;
+        const float u = swap ? Z : Ux, v = swap ? Ux : Vz;
+        float em = zz ? (xx ? x2 - 4.0f * tk : 3.0f * tj - 4.0f * tk) : (xx ? 3.0f * tk - 4.0f * tj : tk - tj);
+        em = (xx || zz) ? em + (zz ? tk2 : tj2) : em;
+        const bool one = xx != zz;  // second order on one side only
+        const float u2 = sq(u), v2 = sq(v);
+        // one-sided
+        const bool ox = xo > 0, two = ox ? xx : zz;
+        const float r = ox ? ri : risti, dn = ox ? dnx : dnz, w = ox ? U : Z;
+        const float c1 = two ? -sq(2.0f * w) * s2 : -s2 * sq(r) * sq(dn);
+        const float a = both ? v2 + (one ? 9.0f * u2 : u2) : 1.0f;
+        const float b = both ? ((one ? 6.0f : xx ? 2.0f : -2.0f) * em) * u2 : 0.0f;
+        const float c = both ? u2 * (sq(em) - s2 * v2) : c1;
+        const float tref = both ? ((xx && zz) ? x2 : swap ? tk : tj) : ox ? (two ? x2 : tj) : (two ? z2 : tk);
+        const bool third = both ? xx && zz : two;
+        float rd1 = sq(b) - 4.0f * a * c;
+        if (rd1 < 0.0f) rd1 = 0.0f;
+        const float tdsh = (-b + sqrtf(rd1)) / (2.0f * a);
+        return (xo > 0 || zo > 0) ? (tref + tdsh) / (third ? 3.0f : 1.0f) : __int_as_float(0x7fc00000);
+    }
+
+    // run: this half has a pair to march
+    __device__ void march_half(bool run, bool refined, const PairGeo& g, int l, int sh) {
+        const unsigned FULL = 0xffffffffu;
+        const int q = l >> 2, qa = l & 1, qb = (l >> 1) & 1;
+        const int dz = q == 2 ? -1 : (q == 3 ? 1 : 0), dx = q == 0 ? -1 : (q == 1 ? 1 : 0);
+        const int sj = 2 * qa - 1, sk = 2 * qb - 1;
+        const bool accx = dx != 0 && sj == -dx, accz = dz != 0 && sk == -dz;  // that side is the accepted node
+        const int lv = l ? 31 - __clz(l) : 0;  // level of local node l in a sift-down's subtree
+        unsigned amask = 0, rmask = 0;         // its ancestors, and the ones that lead right to it
+        for (int c = l; c > 1; c >>= 1) {
+            amask |= 1u << (c >> 1);
+            if (c & 1) rmask |= 1u << (c >> 1);
+        }
+        // the two sides of this lane's quadrant at its neighbour of node pk
+        // (times and statuses), the neighbour's slowness, r*sin(colatitude)
+        struct Sides {
+            FNode j, j2, k, k2;
+            float sl, rs;
+        };
+        const int onb = dz + dx * ld, oj = sj * ld;  // linear offsets
+        auto load_sides = [&](Sides& S, bool has, int pk) {
+            const int z0 = pk & 0xFFFF, x0 = pk >> 16;
+            const bool inner = z0 >= 3 && z0 + 3 < nnz && x0 >= 3 && x0 + 3 < nnx;  // no side leaves the grid
+            const int n = z0 + x0 * ld + onb;
+            if (has && inner) {
+                const FNode* p = nd + n;
+                S.j = p[oj];
+                S.j2 = p[2 * oj];
+                S.k = p[sk];
+                S.k2 = p[2 * sk];
+                S.sl = slw[n];
+                S.rs = risti[x0 + dx];
+            } else if (has) {
+                const int z = z0 + 1 + dz, x = x0 + 1 + dx;
+                if (z >= 1 && z <= nnz && x >= 1 && x <= nnx) {
+                    S.j = wload(z, x, 0, sj);
+                    S.j2 = wload(z, x, 0, 2 * sj);
+                    S.k = wload(z, x, sk, 0);
+                    S.k2 = wload(z, x, 2 * sk, 0);
+                    S.sl = slw[n];
+                    S.rs = risti_at(x);
+                }
+            }
+        };
+        const int dpk = dz + dx * 65536;
+        Sides S{}, N{};          // of this root, and loaded ahead for the next
+        int pre = -1;            // the node N is for
+        int prev = -0x40000000;  // the node accepted before (none: no node's side), and its time
+        float prev_t = 0.0f;
+        for (;;) {
+            __syncwarp();
+            bool on = run && ntr > 0 && !overflow;
+            if (!__any_sync(FULL, on)) break;
+            const float4 top = on ? *reinterpret_cast<const float4*>(&heap[0]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const int pk = __float_as_int(top.w);
+            const float tacc = top.z;
+            const int z0 = (pk & 0xFFFF) + dz, x0 = (pk >> 16) + dx;  // this lane's neighbour, from 0
+            const bool in = on && (unsigned)z0 < (unsigned)nnz && (unsigned)x0 < (unsigned)nnx;
+            const int n0 = lin(pk), nn = n0 + onb;
+            S = N;
+            const bool miss = on && pk != pre;
+            if (__any_sync(FULL, miss)) load_sides(S, miss, pk);
+            // the next root's stencils: the child that the sift-down would take
+            pre = -1;
+            if (on && ntr >= 2) {
+                const float4 cc = *reinterpret_cast<const float4*>(&heap[2]);
+                pre = __float_as_int(ntr >= 3 && cc.x > cc.z ? cc.w : cc.y);
+            }
+            load_sides(N, pre >= 0, pre);
+            if (on && l == 0) nd[n0].s = 0;
+            if (refined && on && at_refined_side(g, (pk & 0xFFFF) + 1, (pk >> 16) + 1)) {
+                run = false;
+                on = false;
+            }
+            down_half(on, l, sh, lv, amask, rmask);
+            // the neighbour's status and heap position, needed by the updates only
+            int s0 = on && in ? nd[nn].s : -2;
+            // loaded ahead, a side that was accepted since is patched
+            const int nb = pk + dpk;
+            const bool pj = nb + sj * 65536 == prev, pj2 = nb + sj * 131072 == prev;
+            const bool pq = nb + sk == prev, pq2 = nb + 2 * sk == prev;
+            const float tj = accx ? tacc : pj ? prev_t : S.j.t, tj2 = pj2 ? prev_t : S.j2.t;
+            const float tk = accz ? tacc : pq ? prev_t : S.k.t, tk2 = pq2 ? prev_t : S.k2.t;
+            const bool aj = accx || pj || S.j.s == 0, ak = accz || pq || S.k.s == 0;
+            const bool aj2 = pj2 || S.j2.s == 0, ak2 = pq2 || S.k2.s == 0;
+            const bool live = in && (unsigned)(x0 + sj) < (unsigned)nnx && (unsigned)(z0 + sk) < (unsigned)nnz;
+            const int xo = !live || !aj ? 0 : (aj2 && tj > tj2) ? 2 : 1;
+            const int zo = !live || !ak ? 0 : (ak2 && tk > tk2) ? 2 : 1;
+            // (the accepted node is one side of a quadrant of every neighbour,
+            // so each has a candidate)
+            float t = quadrant(xo, zo, tj, tj2, tk, tk2, S.sl, S.rs);
+            t = fminf(t, __shfl_xor_sync(FULL, t, 1));
+            t = fminf(t, __shfl_xor_sync(FULL, t, 2));
+            // the four heap updates in the reference's order
+            const unsigned far = half_ballot(s0 == -1, sh), close = half_ballot(s0 > 0, sh);
+            const bool any = __any_sync(FULL, on);
+            bool stale = false;  // entries moved since s0 was loaded
+#pragma unroll 1
+            for (int i = 0; any && i < 4; ++i) {
+                const bool fi = (far >> (4 * i)) & 1u, ci = (close >> (4 * i)) & 1u;
+                if (!__any_sync(FULL, fi || ci)) continue;
+                const int d = i & 1 ? 1 : -1;
+                const int n = n0 + (i < 2 ? d * ld : d), pn = pk + (i < 2 ? d * 65536 : d);
+                const float ti = __shfl_sync(FULL, t, sh + 4 * i);
+                int tpc = __shfl_sync(FULL, s0, sh + 4 * i);
+                if (ci && stale) tpc = nd[n].s;
+                const bool added = grow_half(fi, n, ti, l);
+                if (added) tpc = ntr;
+                stale |= sift_up_half(ci || added, tpc, pn, n, ti, l, sh);
+            }
+            prev = pk;
+            prev_t = tacc;
+        }
+        __syncwarp();
     }
 #endif
 
@@ -567,31 +771,52 @@ struct Scratch {  // device arrays of one chunk of pairs
     int cap, hstride;
 };
 
+// HEAP: where the pair's heap lies: 0 at hp if given, else in S (either
+// address space); 1 at hp, in shared memory (a device caller that says so gets
+// shared-memory accesses; generic ones return in order behind outstanding
+// global loads, which cost the march 2000 cycles per accepted node).
+template <int HEAP = 0>
 FM_HD void march_pair(const Grid& G, int p, int gp, const float* __restrict__ srcx,
                            const float* __restrict__ srcz, const int32_t* __restrict__ pslot,
                            const float* __restrict__ slwn, const float* __restrict__ risti_c,
                            const float* __restrict__ risti_r, const Scratch& S, unsigned int* __restrict__ n_overflow,
-                           FHeap* hp, int smem_cap, int mode, int g4, unsigned gmask) {
+                           FHeap* hp, int smem_cap, int mode, int lane, unsigned mask) {
     // mode 0: one lane, window march; 1: one lane, neighbours one by one;
-    // 2: the four lanes g4 = 0..3 of mask gmask march the pair together
-    // (lane 0 writes the grids and owns the heap); 3: five lanes, lane 0 only
-    // owns the heap and lanes 1..4 solve.
-    PairGeo g = S.geo[p];
-    if (g.status) return;
-    const bool lead = g4 == 0;
+    // 2 (device): half a warp (lane 0 .. 15, mask its lanes) marches the pair,
+    // every lane holding the same state; the other half marches another pair
+    // or none (mask 0: this half has none) and takes part in every step.
+    const bool mine = mode != 2 || mask != 0u;
+    PairGeo g{};
+    if (mine) g = S.geo[p];
+    const bool go = mine && !g.status;
+    if (mode != 2 && !go) return;
+    const bool lead = go && (mode != 2 || lane == 0);
+    const int l0 = mode == 2 ? lane : 0, lstep = mode == 2 ? 16 : 1;  // this lane's share of a loop over nodes
     auto group_sync = [&]() {
 #if defined(__CUDA_ARCH__)
-        if (mode >= 2) __syncwarp(gmask);
+        if (mode == 2) __syncwarp();
 #endif
+    };
+    // (iz, ix) joins the heap with time t (on: this half adds one)
+    auto add = [&](March& M, bool on, int iz, int ix, float t) {
+#if defined(__CUDA_ARCH__)
+        if (mode == 2) {
+            const int n = M.idx(iz, ix);
+            const bool added = M.grow_half(on, n, t, lane);
+            M.sift_up_half(added, M.ntr, March::pack(iz, ix), n, t, lane, threadIdx.x & 16);
+            return;
+        }
+#endif
+        if (on) M.addtree(March::pack(iz, ix), t);
     };
     auto run = [&](March& M, bool refined) {
         if (mode == 1) M.march_nb(refined, g);
 #if defined(__CUDA_ARCH__)
-        else if (mode == 2 || mode == 3) M.march_coop(refined, g, g4, gmask, mode == 3 ? 1 : 0);
+        else if (mode == 2) M.march_half(go, refined, g, lane, threadIdx.x & 16);
 #endif
         else M.march(refined, g);
     };
-    const float x = srcx[gp], z = srcz[gp];
+    const float x = mine ? srcx[gp] : 0.0f, z = mine ? srcz[gp] : 0.0f;
     FNode* fine = S.fine + (size_t)p * RMAX * RMAX;
 
     // refined source grid pass (urg = 1): fmm.f90:170-205 start, then march
@@ -600,19 +825,20 @@ FM_HD void march_pair(const Grid& G, int p, int gp, const float* __restrict__ sr
     R.slw = S.rslw + (size_t)p * RMAX * RMAX;
     const float* rvel = S.rvel + (size_t)p * RMAX * RMAX;
     R.risti = risti_r + (size_t)(g.vnl - 1) * RMAX;
-    R.heap = hp ? hp : S.fheap + (size_t)p * (RCAP + 1);
+    R.heap = HEAP == 1 || hp ? hp : S.fheap + (size_t)p * (RCAP + 1);
     R.ld = RMAX;
     R.nnx = g.nrnx;
     R.nnz = g.nrnz;
-    R.cap = hp ? min(smem_cap, RCAP) : RCAP;
+    R.cap = HEAP == 1 || hp ? min(smem_cap, RCAP) : RCAP;
     R.ntr = 0;
     R.ntr_max = 0;
     R.dnx = G.drnx;
     R.dnz = G.drnz;
     R.overflow = false;
-    if (lead) {
-        for (int ix = 1; ix <= g.nrnx; ++ix)
-            for (int iz = 1; iz <= g.nrnz; ++iz) R.nd[R.idx(iz, ix)] = FNode{0.0f, -1};
+    for (int ix = 1; go && ix <= g.nrnx; ++ix)
+        for (int iz = 1 + l0; iz <= g.nrnz; iz += lstep) R.nd[R.idx(iz, ix)] = FNode{0.0f, -1};
+    group_sync();
+    {
         int isx = (int)((x - g.gorx) / G.drnx) + 1;
         int isz = (int)((z - g.gorz) / G.drnz) + 1;
         if (isx == g.nrnx) isx -= 1;
@@ -621,7 +847,7 @@ FM_HD void march_pair(const Grid& G, int p, int gp, const float* __restrict__ sr
         isz = min(max(isz, 1), g.nrnz - 1);
         float vss[2][2];
         for (int i = 1; i <= 2; ++i)
-            for (int j = 1; j <= 2; ++j) vss[i - 1][j - 1] = rvel[R.idx(isz - 1 + j, isx - 1 + i)];
+            for (int j = 1; j <= 2; ++j) vss[i - 1][j - 1] = go ? rvel[R.idx(isz - 1 + j, isx - 1 + i)] : 1.0f;
         float dsx = (x - g.gorx) - (float)(isx - 1) * G.drnx;
         float dsz = (z - g.gorz) - (float)(isz - 1) * G.drnz;
         float vsrc = bilinear(vss, dsx, dsz, G.drnx, G.drnz);
@@ -629,8 +855,8 @@ FM_HD void march_pair(const Grid& G, int p, int gp, const float* __restrict__ sr
             for (int j = 1; j <= 2; ++j) {
                 float ds = sqrtf(sq(dsx - (float)(i - 1) * G.drnx) + sq(dsz - (float)(j - 1) * G.drnz));
                 float t = 2.0f * ds / (vss[i - 1][j - 1] + vsrc);
-                R.nd[R.idx(isz - 1 + j, isx - 1 + i)].t = t;
-                R.addtree(March::pack(isz - 1 + j, isx - 1 + i), t);
+                if (lead) R.nd[R.idx(isz - 1 + j, isx - 1 + i)].t = t;
+                add(R, go, isz - 1 + j, isx - 1 + i, t);
             }
     }
     group_sync();
@@ -642,45 +868,55 @@ FM_HD void march_pair(const Grid& G, int p, int gp, const float* __restrict__ sr
     C.nd = S.coarse + (size_t)p * S.N;
     C.slw = slwn + (size_t)pslot[gp] * S.N;
     C.risti = risti_c;
-    C.heap = hp ? hp : S.heap + (size_t)p * S.hstride;
+    C.heap = HEAP == 1 || hp ? hp : S.heap + (size_t)p * S.hstride;
     C.ld = G.nnz;
     C.nnx = G.nnx;
     C.nnz = G.nnz;
-    C.cap = hp ? smem_cap : S.cap;
+    C.cap = HEAP == 1 || hp ? smem_cap : S.cap;
     C.ntr = 0;
     C.ntr_max = 0;
     C.dnx = G.dnx;
     C.dnz = G.dnz;
     C.overflow = false;
-    if (lead) {
-        for (int k = 1; k <= g.nrnz; k += SGDL) {
-            const int idm1 = g.vnt + (k - 1) / SGDL;
-            for (int l = 1; l <= g.nrnx; l += SGDL) {
-                const int idm2 = g.vnl + (l - 1) / SGDL;
-                const FNode f = fine[R.idx(k, l)];
-                FNode& c = C.nd[C.idx(idm1, idm2)];
-                c.s = f.s;
-                if (f.s >= 0) c.t = f.t;
-            }
+    group_sync();
+    for (int k = 1 + l0 * SGDL; go && k <= g.nrnz; k += lstep * SGDL) {
+        const int idm1 = g.vnt + (k - 1) / SGDL;
+        for (int l = 1; l <= g.nrnx; l += SGDL) {
+            const int idm2 = g.vnl + (l - 1) / SGDL;
+            const FNode f = fine[R.idx(k, l)];
+            FNode& c = C.nd[C.idx(idm1, idm2)];
+            c.s = f.s;
+            if (f.s >= 0) c.t = f.t;
         }
-        // narrow-band completion (fmst.f90:275-296), only the box can hold alive nodes
-        for (int k = g.vnl; k <= g.vnr; ++k)
-            for (int l = g.vnt; l <= g.vnb; ++l) {
-                FNode& c = C.nd[C.idx(l, k)];
-                if (c.s != 0) continue;
-                if (l - 1 >= 1 && C.nd[C.idx(l - 1, k)].s == -1) c.s = 1;
-                if (l + 1 <= G.nnz && C.nd[C.idx(l + 1, k)].s == -1) c.s = 1;
-                if (k - 1 >= 1 && C.nd[C.idx(l, k - 1)].s == -1) c.s = 1;
-                if (k + 1 <= G.nnx && C.nd[C.idx(l, k + 1)].s == -1) c.s = 1;
-            }
-        // second pass (urg = 2): the narrow band from the resampled grid, in the
-        // reference's scan order (fmm.f90:188-195)
-        for (int i = g.vnl; i <= g.vnr; ++i)
-            for (int j = g.vnt; j <= g.vnb; ++j) {
-                const int n = C.idx(j, i);
-                if (C.nd[n].s > 0) C.addtree(March::pack(j, i), C.nd[n].t);
-            }
     }
+    group_sync();
+    // narrow-band completion (fmst.f90:275-296), only the box can hold alive
+    // nodes; a node reads its neighbours only for "far", which this never sets
+    for (int k = g.vnl; go && k <= g.vnr; ++k)
+        for (int l = g.vnt + l0; l <= g.vnb; l += lstep) {
+            FNode& c = C.nd[C.idx(l, k)];
+            if (c.s != 0) continue;
+            if (l - 1 >= 1 && C.nd[C.idx(l - 1, k)].s == -1) c.s = 1;
+            if (l + 1 <= G.nnz && C.nd[C.idx(l + 1, k)].s == -1) c.s = 1;
+            if (k - 1 >= 1 && C.nd[C.idx(l, k - 1)].s == -1) c.s = 1;
+            if (k + 1 <= G.nnx && C.nd[C.idx(l, k + 1)].s == -1) c.s = 1;
+        }
+    group_sync();
+    // second pass (urg = 2): the narrow band from the resampled grid, in the
+    // reference's scan order (fmm.f90:188-195)
+    // (a box has at most 2 SGS + 1 nodes a side; halves of different boxes
+    // run the same loops)
+    const int bi = mode == 2 ? 2 * SGS + 1 : g.vnr - g.vnl + 1, bj = mode == 2 ? 2 * SGS + 1 : g.vnb - g.vnt + 1;
+    for (int di = 0; di < bi; ++di)
+        for (int dj = 0; dj < bj; ++dj) {
+            const int i = g.vnl + di, j = g.vnt + dj;
+            FNode c{0.0f, 0};
+            if (go && i <= g.vnr && j <= g.vnb) c = C.nd[C.idx(j, i)];
+#if defined(__CUDA_ARCH__)
+            if (mode == 2 && !__any_sync(0xffffffffu, c.s > 0)) continue;
+#endif
+            add(C, c.s > 0, j, i, c.t);
+        }
     group_sync();
     run(C, false);
     if (!lead) return;
