@@ -75,8 +75,10 @@ typedef struct swdk_config {
   double rtol;     /* bracket width for SWDK_REFINE_TIGHT (default 1e-10)     */
   int sngl;        /* 1: roots rounded to REAL*4 as surfdisp96 does (default) */
   int sphere;      /* 1: spherical earth as SurfTime (default); 0: flat       */
-  int block_roots; /* blocks of the persistent root kernel, 0 = occupancy
-                      default (swdk_autotune sets it)                       */
+  int block_roots; /* blocks of the persistent root kernel with one lane per
+                      chain; 0: as many as are resident, and groups of lanes
+                      per chain for calls with few chains.  The roots are the
+                      same bits either way.                                 */
   int split_cols;  /* calls with at least this many columns run as two
                       concurrent column halves on child contexts; <= 0
                       (default) = never.  Host-memory calls stream their

@@ -972,8 +972,9 @@ __global__ void __launch_bounds__(128, SWDK_RETRY_MINB) k_retry(int ncol, const 
 cudaError_t roots_occupancy(int* per) {
   cudaError_t e = cudaFuncSetAttribute(k_roots_queue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ROOTS_SMEM);
   const int cs = (int)coop_smem(COOP_MIN_G);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_roots_coop<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_roots_coop<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_roots_coop<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_roots_coop<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_roots_coop<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, cs);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_retry, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RETRY_SMEM);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, k_roots_queue, 128, ROOTS_SMEM);
   return e;
@@ -983,21 +984,29 @@ cudaError_t roots_occupancy(int* per) {
 // lane each needs about 75 000 chains to fill the GPU; a call's time is then
 // the longest chain's, about 30 ms whatever the size.  More lanes shorten the
 // chain and cost throughput (the products run in every lane of a group; groups
-// of one warp that evaluate different numbers of velocities take turns).  ms of
-// the search with 1 / 4 / 8 / 32 lanes, 20 periods of 41 nodes, Rayleigh:
-//   1188 chains 24.6 / 10.0 / 9.2 / 4.4     3840  29.5 / 18.7 / 12.6 / 23.2
-//   1500        28.7 / 17.7 / 10.3 / 10.2   10000 36.3 / 23.9 / 33.6 / 42.2
-//   2400        28.7 / 18.7 / 11.7 / 16.0   16384 27.3 / 27.8 / 38.2 / 92.7
-// (16 lanes lie between 8 and 32 and lead nowhere).  The lines are a device's
-// of 148 SMs and move with its size.
-int coop_lanes(long long nitems, int nsm) {
+// of one warp that evaluate different numbers of velocities take turns).
+// Chains that walk the scan grid (no proposals, or higher modes, whose scans
+// the proposals leave) gain most from many lanes, which take eight points of
+// it at a time.  ms of the search with 1 / 4 / 32 lanes, 20 periods of 41
+// nodes, one mode:
+//   Rayleigh, proposals                    Rayleigh and Love, plain scan
+//   1500   28.7 / 17.7 /  5.1              11834  86.5 / 48.5 / 42.4 (30 periods)
+//   5200   28.9 / 12.7 / 15.8              16384  65.2 / 51.5 / 51.8
+//   12800  28.2 / 16.2 / 38.9              23040  69.8 / 56.7 / 71.6
+//   16384  28.4 / 26.9 / 48.3              32768  71.4 / 85.8 / 101.9
+// and two modes with coast columns 10240: 186.9 / 106.3 / 66.1, 20000: 257 /
+// 157 / 125 (8 and 16 lanes lie between and lead nowhere).  The lines are a
+// device's of 148 SMs and move with its size.
+int coop_lanes(long long nitems, int nsm, bool scans) {
   const long long n = nitems * 148 / std::max(1, nsm);
-  return n <= 1500 ? 32 : n <= 6000 ? 8 : n <= 14000 ? 4 : 1;
+  if (scans) return n <= 18000 ? 32 : n <= 26000 ? 4 : 1;
+  return n <= 4500 ? 32 : n <= 16000 ? 4 : 1;
 }
 
 struct RootsCall {
   int ncol;
   long long nitems;
+  bool scans;  // chains without proposals or of several modes
   const int* order;
   const ChainDesc* chains;
   const double* periods;
@@ -1023,13 +1032,14 @@ struct RootsCall {
 // k_roots_queue; tuned: that count was asked for (swdk_autotune, or the
 // caller's configuration), so the one-lane kernel runs
 cudaError_t launch_roots(const RootsCall& c, int rblocks, int nsm, bool tuned, cudaStream_t st) {
-  const int G = tuned ? 1 : coop_lanes(c.nitems, nsm);
+  const int G = tuned ? 1 : coop_lanes(c.nitems, nsm, c.scans);
   if (G > 1) {
     const long long need = (c.nitems * G + 127) / 128;
-    k_roots_coop<false><<<(unsigned)std::max(1LL, std::min<long long>(need, 3LL * nsm)), 128, coop_smem(G), st>>>(
-        c.ncol, (int)c.nitems, G, c.order, c.chains, c.periods, c.layR, c.layL, c.info, c.refine, c.rtol, c.sngl,
-        RETRY_DEFERRED, c.croot, c.cstat, c.queue, c.prop, c.retry_list, c.rctr, c.rcap, c.nevals, c.rg, c.nodes,
-        c.dl, nullptr);
+    const auto k = c.refine == 0 ? k_roots_coop<1> : k_roots_coop<4>;
+    const CoopArgs A{c.ncol,  (int)c.nitems,  G,       c.order,      c.chains, c.periods, c.layR,  c.layL, c.info,
+                     c.refine, c.rtol,        c.sngl,  RETRY_DEFERRED, c.croot, c.cstat,  c.queue, c.prop, c.retry_list,
+                     c.rctr,  c.rcap,         c.nevals, c.rg,          c.nodes, c.dl,     nullptr};
+    k<<<(unsigned)std::max(1LL, std::min<long long>(need, 3LL * nsm)), 128, coop_smem(G), st>>>(A);
   } else {
     k_roots_queue<<<(unsigned)std::max(1LL, std::min<long long>(rblocks, (c.nitems + 127) / 128)), 128, ROOTS_SMEM,
                     st>>>(c.ncol, (int)c.nitems, c.order, c.chains, c.periods, c.layR, c.layL, c.info, c.refine,
@@ -1806,6 +1816,8 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
   RootsCall rc;
   rc.ncol = ncol;
   rc.nitems = nitems;
+  rc.scans = !useprop;
+  for (const ChainDesc& d : P.chains) rc.scans |= d.nmode > 1;
   rc.order = P.d_order.as<int>();
   rc.chains = P.d_chains.as<ChainDesc>();
   rc.periods = P.d_periods.as<double>();
@@ -2337,15 +2349,16 @@ int swdk_surfdisp96_batch(swdk_ctx* ctx, int nmodel, int nlayer, const float* th
     CK(roots_occupancy(&per));
     ctx->coop_ready = true;
   }
-  if (const int G = coop_lanes(nmodel, ctx->nsm); G > 1) {
+  if (const int G = coop_lanes(nmodel, ctx->nsm, true); G > 1) {
     CK(ctx->queue.ensure(sizeof(unsigned int)));
     CK(cudaMemsetAsync(ctx->queue.p, 0, sizeof(unsigned int), st));
     const long long need = ((long long)nmodel * G + 127) / 128;
-    k_roots_coop<true><<<(unsigned)std::min<long long>(need, 3LL * ctx->nsm), 128, coop_smem(G), st>>>(
-        nmodel, nmodel, G, nullptr, d_ch, d_t, ctx->layR.as<float4>(), ctx->layL.as<float4>(), ctx->info.as<ColInfo>(),
-        ctx->cfg.refine, ctx->cfg.rtol, ctx->cfg.sngl, RETRY_NONE, ctx->croot.as<double>(), ctx->cstat.as<int32_t>(),
-        ctx->queue.as<unsigned int>(), nullptr, nullptr, nullptr, 0u, ctx->nevals.as<unsigned long long>(),
-        RaggedMap{nullptr, nullptr, 0, nlayer}, nullptr, nullptr, ctx->ierr.as<int32_t>());
+    const CoopArgs A{nmodel, nmodel, G, nullptr, d_ch, d_t, ctx->layR.as<float4>(), ctx->layL.as<float4>(),
+                     ctx->info.as<ColInfo>(), ctx->cfg.refine, ctx->cfg.rtol, ctx->cfg.sngl, RETRY_NONE,
+                     ctx->croot.as<double>(), ctx->cstat.as<int32_t>(), ctx->queue.as<unsigned int>(), nullptr, nullptr,
+                     nullptr, 0u, ctx->nevals.as<unsigned long long>(), RaggedMap{nullptr, nullptr, 0, nlayer}, nullptr,
+                     nullptr, ctx->ierr.as<int32_t>()};
+    k_roots_coop<0><<<(unsigned)std::min<long long>(need, 3LL * ctx->nsm), 128, coop_smem(G), st>>>(A);
   } else
   k_roots<<<dim3((nmodel + 127) / 128, 1), 128, 0, st>>>(nmodel, d_ch, d_t, ctx->layR.as<float4>(),
                                                          ctx->layL.as<float4>(), ctx->info.as<ColInfo>(),
@@ -2704,6 +2717,8 @@ int ragged_enqueue(swdk_ragged* R, cudaStream_t st, bool timing) {
   RootsCall rc;
   rc.ncol = 0;
   rc.nitems = R->nitems;
+  rc.scans = !R->useprop;
+  for (const ChainDesc& d : R->chains) rc.scans |= d.nmode > 1;
   rc.order = nullptr;
   rc.chains = R->d_chains.as<ChainDesc>();
   rc.periods = R->d_periods.as<double>();
@@ -2724,7 +2739,7 @@ int ragged_enqueue(swdk_ragged* R, cudaStream_t st, bool timing) {
   rc.rg = rg;
   rc.nodes = use_nodes ? R->nodes.as<float4>() : nullptr;
   rc.dl = R->dltab.as<DepthLayer>();
-  CK(launch_roots(rc, R->roots_blocks, R->nsm, false, st));
+  CK(launch_roots(rc, R->roots_blocks, R->nsm, cfg.block_roots > 0, st));
   if (timing) CK(cudaEventRecord(R->ev[2], st));
   if (R->path != 2) {
     using EigR = void (*)(const REBlock*, int, const RModel*, const float4*, const ColInfo*, const float2*,
@@ -2941,6 +2956,7 @@ int swdk_ragged_create(int n, swdk_ctx* const* ctxs, const swdk_call* calls, swd
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) e = roots_occupancy(&per);
   if (e != cudaSuccess) return bail(SWDK_E_CUDA, std::string("ragged batch set-up: ") + cudaGetErrorString(e));
+  R->nsm = std::max(1, nsm);
   R->roots_blocks = ctx->cfg.block_roots > 0 ? ctx->cfg.block_roots : std::max(1, nsm * std::max(1, per));
   *out = R;
   return SWDK_OK;
@@ -3013,8 +3029,9 @@ int swdk_autotune(swdk_ctx* ctx, int nx, int ny, int nz, const float* d_vs, cons
   CK(roots_occupancy(&per));
   per = std::max(1, per);
   // candidates: resident blocks of the persistent root kernel, 1..per per SM
-  // plus one oversubscribed grid (queue items then also spread over waves)
-  std::vector<int> cand;
+  // plus one oversubscribed grid (queue items then also spread over waves);
+  // 0, the default, is the groups of lanes where the call has few chains
+  std::vector<int> cand = {0};
   for (int k = 1; k <= per; ++k) cand.push_back(k * nsm);
   cand.push_back(2 * per * nsm);
   const int saved = ctx->cfg.block_roots;
@@ -3037,7 +3054,7 @@ int swdk_autotune(swdk_ctx* ctx, int nx, int ny, int nz, const float* d_vs, cons
   }
   ctx->cfg.block_roots = best;
   drop_kids(ctx);  // the column halves are recreated with the tuned grid
-  if (blocks_out) *blocks_out = best;
+  if (blocks_out) *blocks_out = best > 0 ? best : ctx->roots_blocks;
   return SWDK_OK;
 }
 

@@ -13,9 +13,10 @@
 // love_product), in the same order, so the values are the same bits.
 //
 //
-// What bounds it: the dependent FP64 chain.  With W = 32 one evaluation of 161
-// layers takes 57 000 cycles (entries 19 000, products 27 000 at 170 a layer)
-// against 210 000 by one lane.
+// What bounds it: the dependent FP64 chain.  With W = 32 and a warp or two per
+// scheduler an evaluation of 161 layers takes 57 000 cycles (entries 19 000,
+// products 27 000, 170 a layer) against 210 000 by one lane; a round of the
+// state machine between evaluations 4000 to 8000.
 #pragma once
 
 namespace {
@@ -30,7 +31,9 @@ struct CoopGroup {
   LayerView V;
   double cc[32], cf[32];
   double cw;
+  int npts;    // velocities to evaluate now
   int cn, ch;  // valid entries, the one expected next
+  int have, exhausted, asked, item;  // a chain is running; the queue is empty; cc[0] is the chain's request; its item
   unsigned ev[NPHASE_EV];  // evaluations by phase of the current chain
 };
 
@@ -244,14 +247,14 @@ __device__ double coop_love(bool on, const LayerView& V, double wvno, double ome
 // Trial velocities worth evaluating together with the chain's request
 // (s.creq, s.next), in cc[0..n): the request itself, then the ones that the
 // search asks for next unless a sign change ends its walk before.  G: lanes
-// of the group.  Only the values' reuse depends on this guess, never a root.
+// of the group; n is a power of two and at most G.  Only the values' reuse depends on this guess, never a root.
 __device__ int coop_plan(ChainState& s, const ChainParams& P, const ChainIO& io, int G, double* cc) {
   cc[0] = s.creq;
   int n = 1;
   switch (s.next) {
     case PH_SCAN_GOT: {  // the scan's next points; the first period's scan is the long one
       const double step = s.idir > 0 ? DC : -DC;
-      n = s.k == 1 ? G : max(1, G / 4);
+      n = s.k == 1 ? G : G / 4;
       for (int i = 1; i < n; ++i) cc[i] = cc[i - 1] + step;
       break;
     }
@@ -262,7 +265,7 @@ __device__ int coop_plan(ChainState& s, const ChainParams& P, const ChainIO& io,
       const bool jump = s.pj == -1 && first_cell(s, P, io, m);
       s.del1st = d1;
       if (jump) {
-        n = max(1, min(G, 1 + m / FIRST_STRIDE));
+        n = min(G, 1 + m / FIRST_STRIDE);
         int g = 1;
         while (g < n) g <<= 1;
         n = g;
@@ -273,7 +276,7 @@ __device__ int coop_plan(ChainState& s, const ChainParams& P, const ChainIO& io,
         }
         break;
       }
-      n = s.k == 1 ? G : max(1, G / 4);
+      n = s.k == 1 ? G : G / 4;
       for (int i = 1; i < n; ++i) cc[i] = cc[i - 1] + DC;
       break;
     }
@@ -300,167 +303,194 @@ __device__ int coop_plan(ChainState& s, const ChainParams& P, const ChainIO& io,
   return n;
 }
 
-// k_roots_coop: G lanes (4, 8, 16 or 32) per work item of k_roots_queue; with
-// REF, per layered model, one chain each, the secular functions as dltar1 /
-// dltar4 write them, and the chains' ierr.  The group's first lane runs the chain's state
-// machine; an evaluation takes all of the group's lanes, for one trial
-// velocity or for several planned together (W = G / number lanes each).
+// What every group of a launch shares.
+struct CoopArgs {
+  int ncol, nitems, G;
+  const int* order;
+  const ChainDesc* chains;
+  const double* periods;
+  const float4 *layR, *layL;
+  const ColInfo* info;
+  int refine;
+  double rtol;
+  int sngl, retry;
+  double* croot;
+  int32_t* cstat;
+  unsigned int* queue;
+  const float2* prop;
+  int2* retry_list;
+  unsigned int* retry_count;
+  unsigned int retry_cap;
+  unsigned long long* nevals;
+  RaggedMap rg;
+  const float4* nodes;
+  const DepthLayer* dl;
+  int32_t* ierr_out;  // REF: the chains' ierr
+};
+
+// The group's first lane: gives the chain its value, runs its state machine
+// through all that needs no new evaluation (taking the next item when the
+// chain ends) and plans the next evaluations.  Returns their number, 0 when
+// there is no work left.  Not inlined.
 template <bool REF>
-__global__ void __launch_bounds__(128, 3) k_roots_coop(int ncol, int nitems, int G, const int* __restrict__ order,
-                                                       const ChainDesc* __restrict__ chains,
-                                                       const double* __restrict__ periods,
-                                                       const float4* __restrict__ layR,
-                                                       const float4* __restrict__ layL,
-                                                       const ColInfo* __restrict__ info, int refine, double rtol,
-                                                       int sngl, int retry, double* __restrict__ croot,
-                                                       int32_t* __restrict__ cstat, unsigned int* __restrict__ queue,
-                                                       const float2* __restrict__ prop,
-                                                       int2* __restrict__ retry_list,
-                                                       unsigned int* __restrict__ retry_count, unsigned int retry_cap,
-                                                       unsigned long long* __restrict__ nevals, RaggedMap rg,
-                                                       const float4* __restrict__ nodes,
-                                                       const DepthLayer* __restrict__ dl,
-                                                       int32_t* __restrict__ ierr_out) {
+__device__ __noinline__ int coop_step(CoopGroup& g, const CoopArgs& A, unsigned long long* phase_ev,
+                                      unsigned long long* blk_ev) {
+  ChainState& s = g.s;
+  ChainParams& P = g.P;
+  ChainIO& io = g.io;
+  // the chain takes its value
+  auto answer = [&](int i) {
+    g.ev[eval_phase(s)] += 1u;
+    s.last = g.cf[i];
+    s.nevals++;
+    s.phase = s.next;
+    g.ch = i + 1 < g.cn ? i + 1 : 0;
+  };
+  if (g.asked) answer(0);
+  g.asked = 0;
+  for (;;) {
+    if (!g.have) {
+      if (g.exhausted) return 0;
+      const unsigned int r = atomicAdd(A.queue, 1u);
+      if (r >= (unsigned int)A.nitems) { g.exhausted = 1; return 0; }
+      const int item_of = (int)r;
+      g.item = item_of;
+      int mcol = A.ncol, lstride = A.rg.lstride, col;
+      ChainDesc cd;
+      long long o_col = 0, o_lay = 0, o_root = 0, o_node = 0, o_dl = 0;
+      if (A.rg.blocks) {
+        const RBlock B = A.rg.blocks[ragged_find(A.rg.blocks, A.rg.nblocks, (long long)item_of, &RBlock::item0)];
+        const RModel& M = A.rg.models[B.model];
+        cd = A.chains[B.chain];
+        col = (int)((long long)item_of - B.item0);
+        mcol = M.ncol;
+        lstride = M.Lmax;
+        o_col = M.col0; o_lay = M.lay0; o_root = M.root0; o_node = M.node0; o_dl = M.dl0;
+      } else {
+        cd = A.chains[REF ? 0 : A.order[item_of / A.ncol]];
+        col = item_of % A.ncol;
+      }
+      const ColInfo ci = A.info[o_col + col];
+      double* outp = A.croot + o_root + (size_t)cd.out_off * mcol + col;
+      int32_t* stp = A.cstat + o_root + (size_t)cd.out_off * mcol + col;
+      if (!ci.valid) {
+        for (int i = 0; i < cd.nmode * cd.np; ++i) {
+          outp[(size_t)i * mcol] = 0.0;
+          stp[(size_t)i * mcol] = ST_NAN_INPUT;
+        }
+        if (REF) A.ierr_out[col] = 1;
+        continue;
+      }
+      LayerView& V = g.V;
+      V.lay = ((cd.iwave == 2) ? A.layR : A.layL) + o_lay;
+      V.fast = REF ? 0 : 1;
+      V.ncol = mcol;
+      V.col = col;
+      V.lstride = lstride;
+      V.L = ci.L;
+      V.llw = ci.llw;
+      V.nodes = (A.nodes && ci.nw == 0) ? A.nodes + o_node + (size_t)col * ((lstride + 3) / 4) : nullptr;
+      V.dl = A.dl + o_dl;
+      V.wave = cd.iwave;
+      P.t = A.periods + cd.t_off;
+      P.kmax = cd.np;
+      P.nmode = cd.nmode;
+      P.igr = cd.igr;
+      P.iwave = cd.iwave;
+      P.refine = A.refine;
+      P.rtol = A.rtol;
+      P.sngl = A.sngl;
+      P.cc = ci.cc;
+      P.betmx = ci.betmx;
+      P.retry = A.retry;
+      io.out = outp;
+      io.st = stp;
+      io.stride = cd.np * mcol;
+      io.ostride = mcol;
+      io.prop = A.prop ? A.prop + o_root + (size_t)cd.out_off * mcol + col : nullptr;
+      chain_init(s);
+      g.cn = 0;
+      for (int i = 0; i < NPHASE_EV; ++i) g.ev[i] = 0u;
+      g.have = 1;
+    }
+    if (!chain_advance(s, P, io)) {  // chain finished
+      if (REF) A.ierr_out[g.V.col] = s.ierr;
+      if (s.iterlim)
+        for (int i = 0; i < P.nmode * P.kmax; ++i)
+          if (io.st[(size_t)i * io.ostride] == ST_OK) io.st[(size_t)i * io.ostride] = ST_ITER_LIMIT;
+      if (A.retry == RETRY_DEFERRED && s.ierr != 0) {  // failed slots: single-period work items for k_retry
+        for (int m = 1; m <= P.nmode; ++m)
+          for (int k = 1; k <= P.kmax; ++k) {
+            const double v = out_at(io, m, k);
+            if (v == 0.0 || !(v == v)) {
+              const unsigned int q = atomicAdd(A.retry_count, 1u);
+              if (q < A.retry_cap) A.retry_list[q] = make_int2(g.item, (m << 16) | k);
+            }
+          }
+      }
+      for (int i = 0; i < NPHASE_EV; ++i)
+        if (g.ev[i]) atomicAdd(&phase_ev[i], (unsigned long long)g.ev[i]);
+      atomicAdd(&blk_ev[0], (unsigned long long)s.nevals);
+      atomicAdd(&blk_ev[P.iwave == 2 ? 1 : 2], (unsigned long long)s.nevals * g.V.L);
+      if (s.nprop_ok) atomicAdd(&blk_ev[3], (unsigned long long)s.nprop_ok);
+      if (s.nprop_fail) atomicAdd(&blk_ev[4], (unsigned long long)s.nprop_fail);
+      g.have = 0;
+      continue;
+    }
+    // a value evaluated ahead?
+    int hit = -1;
+    if (g.cw == s.omega) {
+      const int cn = g.cn, ch = g.ch;
+      for (int t = 0; t < cn && hit < 0; ++t) {
+        const int i = ch + t < cn ? ch + t : ch + t - cn;
+        if (g.cc[i] == s.creq) hit = i;
+      }
+    }
+    if (hit < 0) {
+      g.cn = coop_plan(s, P, io, A.G, g.cc);
+      g.cw = s.omega;
+      g.asked = 1;
+      return g.cn;
+    }
+    answer(hit);
+  }
+}
+
+// k_roots_coop: G lanes (4, 8, 16 or 32) per work item of k_roots_queue; an
+// evaluation takes all of the group's lanes, for one trial velocity or for
+// several planned together (W = G / number lanes each).  NORM 4 and 1: the
+// tight and the reference refinement's secular functions; 0: layered models,
+// one chain each, the functions as dltar1 / dltar4 write them.
+template <int NORM>
+__global__ void __launch_bounds__(128, 3) k_roots_coop(const __grid_constant__ CoopArgs A) {
+  const unsigned FULL = 0xffffffffu;
   extern __shared__ __align__(16) unsigned char coop_sm[];
   __shared__ unsigned long long phase_ev[NPHASE_EV];
   __shared__ unsigned long long blk_ev[5];
   if (threadIdx.x < NPHASE_EV) phase_ev[threadIdx.x] = 0ull;
   if (threadIdx.x < 5) blk_ev[threadIdx.x] = 0ull;
   __syncthreads();
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+  const int G = A.G, lane = threadIdx.x & 31, gl = lane & (G - 1);
   double* wbuf = reinterpret_cast<double*>(coop_sm + (threadIdx.x >> 5) * COOP_BUF);
   CoopGroup& g = reinterpret_cast<CoopGroup*>(coop_sm + 4 * COOP_BUF)[threadIdx.x / G];
   double cbuf[KMAX_CHAIN];
   double cbbuf[KMAX_CHAIN + 24];
-  bool have = false, exhausted = false, asked = false;  // the leader's; asked: cc[0] is the chain's request
-  int item_of = 0;
-  if (gl == 0) { g.cn = 0; g.io.c = cbuf; g.io.cb = cbbuf; }
+  if (gl == 0) {
+    g.cn = 0;
+    g.have = g.exhausted = g.asked = 0;
+    g.io.c = cbuf;
+    g.io.cb = cbbuf;
+  }
   for (;;) {
-    int npts = 0;  // the leader's: velocities to evaluate
+    // the number goes through shared memory: with it in a register the
+    // compiler left the first lane apart from the others, and the evaluation
+    // ran twice (16 active lanes an instruction instead of 30)
     if (gl == 0) {
-      ChainState& s = g.s;
-      ChainParams& P = g.P;
-      ChainIO& io = g.io;
-      // the chain takes its value
-      auto answer = [&](int i) {
-        g.ev[eval_phase(s)] += 1u;
-        s.last = g.cf[i];
-        s.nevals++;
-        s.phase = s.next;
-        g.ch = i + 1 < g.cn ? i + 1 : 0;
-      };
-      if (asked) answer(0);
-      asked = false;
-      for (;;) {
-        if (!have) {
-          if (exhausted) break;
-          const unsigned int r = atomicAdd(queue, 1u);
-          if (r >= (unsigned int)nitems) { exhausted = true; break; }
-          item_of = (int)r;
-          int mcol = ncol, lstride = rg.lstride, col;
-          ChainDesc cd;
-          long long o_col = 0, o_lay = 0, o_root = 0, o_node = 0, o_dl = 0;
-          if (rg.blocks) {
-            const RBlock B = rg.blocks[ragged_find(rg.blocks, rg.nblocks, (long long)item_of, &RBlock::item0)];
-            const RModel& M = rg.models[B.model];
-            cd = chains[B.chain];
-            col = (int)((long long)item_of - B.item0);
-            mcol = M.ncol;
-            lstride = M.Lmax;
-            o_col = M.col0; o_lay = M.lay0; o_root = M.root0; o_node = M.node0; o_dl = M.dl0;
-          } else {
-            cd = chains[REF ? 0 : order[item_of / ncol]];
-            col = item_of % ncol;
-          }
-          const ColInfo ci = info[o_col + col];
-          double* outp = croot + o_root + (size_t)cd.out_off * mcol + col;
-          int32_t* stp = cstat + o_root + (size_t)cd.out_off * mcol + col;
-          if (!ci.valid) {
-            for (int i = 0; i < cd.nmode * cd.np; ++i) {
-              outp[(size_t)i * mcol] = 0.0;
-              stp[(size_t)i * mcol] = ST_NAN_INPUT;
-            }
-            if (REF) ierr_out[col] = 1;
-            continue;
-          }
-          LayerView& V = g.V;
-          V.lay = ((cd.iwave == 2) ? layR : layL) + o_lay;
-          V.fast = REF ? 0 : 1;
-          V.ncol = mcol;
-          V.col = col;
-          V.lstride = lstride;
-          V.L = ci.L;
-          V.llw = ci.llw;
-          V.nodes = (nodes && ci.nw == 0) ? nodes + o_node + (size_t)col * ((lstride + 3) / 4) : nullptr;
-          V.dl = dl + o_dl;
-          V.wave = cd.iwave;
-          P.t = periods + cd.t_off;
-          P.kmax = cd.np;
-          P.nmode = cd.nmode;
-          P.igr = cd.igr;
-          P.iwave = cd.iwave;
-          P.refine = refine;
-          P.rtol = rtol;
-          P.sngl = sngl;
-          P.cc = ci.cc;
-          P.betmx = ci.betmx;
-          P.retry = retry;
-          io.out = outp;
-          io.st = stp;
-          io.stride = cd.np * mcol;
-          io.ostride = mcol;
-          io.prop = prop ? prop + o_root + (size_t)cd.out_off * mcol + col : nullptr;
-          chain_init(s);
-          g.cn = 0;
-          for (int i = 0; i < NPHASE_EV; ++i) g.ev[i] = 0u;
-          have = true;
-        }
-        if (!chain_advance(s, P, io)) {  // chain finished
-          if (REF) ierr_out[g.V.col] = s.ierr;
-          if (s.iterlim)
-            for (int i = 0; i < P.nmode * P.kmax; ++i)
-              if (io.st[(size_t)i * io.ostride] == ST_OK) io.st[(size_t)i * io.ostride] = ST_ITER_LIMIT;
-          if (retry == RETRY_DEFERRED && s.ierr != 0) {  // failed slots: single-period work items for k_retry
-            for (int m = 1; m <= P.nmode; ++m)
-              for (int k = 1; k <= P.kmax; ++k) {
-                const double v = out_at(io, m, k);
-                if (v == 0.0 || !(v == v)) {
-                  const unsigned int q = atomicAdd(retry_count, 1u);
-                  if (q < retry_cap) retry_list[q] = make_int2(item_of, (m << 16) | k);
-                }
-              }
-          }
-          for (int i = 0; i < NPHASE_EV; ++i)
-            if (g.ev[i]) atomicAdd(&phase_ev[i], (unsigned long long)g.ev[i]);
-          atomicAdd(&blk_ev[0], (unsigned long long)s.nevals);
-          atomicAdd(&blk_ev[P.iwave == 2 ? 1 : 2], (unsigned long long)s.nevals * g.V.L);
-          if (s.nprop_ok) atomicAdd(&blk_ev[3], (unsigned long long)s.nprop_ok);
-          if (s.nprop_fail) atomicAdd(&blk_ev[4], (unsigned long long)s.nprop_fail);
-          have = false;
-          continue;
-        }
-        // a value evaluated ahead?
-        int hit = -1;
-        if (g.cw == s.omega) {
-          const int cn = g.cn, ch = g.ch;
-          for (int t = 0; t < cn && hit < 0; ++t) {
-            const int i = ch + t < cn ? ch + t : ch + t - cn;
-            if (g.cc[i] == s.creq) hit = i;
-          }
-        }
-        if (hit < 0) {
-          npts = coop_plan(s, P, io, G, g.cc);
-          g.cn = npts;
-          g.cw = s.omega;
-          asked = true;
-          break;
-        }
-        answer(hit);
-      }
+      const int np = coop_step<NORM == 0>(g, A, phase_ev, blk_ev);
+      g.npts = np;
     }
     __syncwarp();
-    npts = __shfl_sync(FULL, npts, lane & ~(G - 1));
+    const int npts = g.npts;
     unsigned todo = __ballot_sync(FULL, npts > 0);
     if (todo == 0u) break;
     // the groups that evaluate the same number of velocities together
@@ -474,21 +504,18 @@ __global__ void __launch_bounds__(128, 3) k_roots_coop(int ncol, int nitems, int
       const double wv = mine ? om / g.cc[j] : 1.0;
       const bool ray = mine && g.P.iwave == 2, lov = mine && g.P.iwave != 2;
       double f = 0.0;
-      if (W == 1) {
-        const LayerView V = g.V;  // in registers: read at every layer
-        if (mine) f = REF ? secular(V, g.P.iwave, wv, om) : secular_fast(V, g.P.iwave, refine, wv, om);
+      if (W == 1) {  // a velocity per lane: nothing to share
+        const LayerView V = g.V;
+        if (mine)
+          f = NORM == 0 ? secular(V, g.P.iwave, wv, om) : secular_fast(V, g.P.iwave, NORM == 1 ? 0 : 1, wv, om);
       } else {
         double* rows = wbuf + (size_t)(lane - l) * COOP_ROW;
         if (__ballot_sync(FULL, ray)) {
-          const double v = REF           ? coop_rayleigh<0>(ray, g.V, wv, om, W, l, rows)
-                           : refine == 0 ? coop_rayleigh<1>(ray, g.V, wv, om, W, l, rows)
-                                         : coop_rayleigh<4>(ray, g.V, wv, om, W, l, rows);
+          const double v = coop_rayleigh<NORM>(ray, g.V, wv, om, W, l, rows);
           if (ray) f = v;
         }
         if (__ballot_sync(FULL, lov)) {
-          const double v = REF           ? coop_love<0>(lov, g.V, wv, om, W, l, rows)
-                           : refine == 0 ? coop_love<1>(lov, g.V, wv, om, W, l, rows)
-                                         : coop_love<4>(lov, g.V, wv, om, W, l, rows);
+          const double v = coop_love<NORM>(lov, g.V, wv, om, W, l, rows);
           if (lov) f = v;
         }
       }
@@ -497,9 +524,9 @@ __global__ void __launch_bounds__(128, 3) k_roots_coop(int ncol, int nitems, int
     }
   }
   __syncthreads();
-  if (threadIdx.x < NPHASE_EV && nevals && phase_ev[threadIdx.x])
-    atomicAdd(nevals + EV_BASE + threadIdx.x, phase_ev[threadIdx.x]);
-  if (threadIdx.x < 5 && nevals && blk_ev[threadIdx.x]) atomicAdd(nevals + threadIdx.x, blk_ev[threadIdx.x]);
+  if (threadIdx.x < NPHASE_EV && A.nevals && phase_ev[threadIdx.x])
+    atomicAdd(A.nevals + EV_BASE + threadIdx.x, phase_ev[threadIdx.x]);
+  if (threadIdx.x < 5 && A.nevals && blk_ev[threadIdx.x]) atomicAdd(A.nevals + threadIdx.x, blk_ev[threadIdx.x]);
 }
 
 }  // namespace

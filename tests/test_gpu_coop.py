@@ -32,13 +32,13 @@ def _roots(case, learned, **kw):
     return out
 
 
-# chains on both sides of every line of the launch rule (1500, 6000, 14000) and
+# chains on both sides of every line of the launch rule (4500, 16000; scans 18000, 26000) and
 # the smallest ones; layer counts that leave every remainder of a group's lanes
 @pytest.mark.parametrize("ncol,nz,waves,nmode,water,learned", [
     (1, 2, ("Rc",), 1, False, False), (1, 80, ("Rc", "Lc"), 2, True, False), (3, 5, ("Lg",), 1, True, True),
-    (1500, 9, ("Rc",), 1, False, True), (1501, 9, ("Rc",), 1, True, False), (751, 12, ("Rc", "Lc"), 2, True, True),
-    (3000, 7, ("Rc", "Lc"), 1, False, True), (6001, 6, ("Rc",), 1, True, False), (14000, 4, ("Lc",), 1, False, True),
-    (14001, 4, ("Rc",), 1, False, False)])
+    (4500, 9, ("Rc",), 1, False, True), (4501, 9, ("Rc",), 1, True, True), (751, 12, ("Rc", "Lc"), 2, True, True),
+    (3000, 7, ("Rc", "Lc"), 1, False, True), (18000, 6, ("Rc",), 1, True, False), (16000, 4, ("Lc",), 1, False, True),
+    (18001, 4, ("Rc",), 1, False, False), (13001, 5, ("Lc", "Rc"), 1, False, False)])
 def test_group_search_equals_one_lane(ncol, nz, waves, nmode, water, learned):
     case = _case(ncol, nz, waves, nmode, water, seed=ncol + nz)
     c1, s1 = _roots(case, learned, block_roots=592)
