@@ -1477,6 +1477,9 @@ int nt_of(const double* col, int ntmax) {
 // 14.9, 8 chunks 15.25, 16 chunks 15.33 M slots/s with device time 15.4;
 // with the faster eigen stage 16 chunks 17.29, 32 chunks 16.72 M slots/s)
 constexpr int HOST_CHUNKS = SWDK_HOST_CHUNKS;
+// and as many as leave a chunk this many output bytes: 16 chunks of 16 columns
+// each took 2.4 ms of launches and copies where one takes 0.3 ms
+constexpr size_t HOST_CHUNK_BYTES = 4u << 20;
 
 struct swdk_ctx {
   swdk_config cfg;
@@ -1857,9 +1860,11 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
       }
       if (!ctx->evefork) CK(cudaEventCreateWithFlags(&ctx->evefork, cudaEventDisableTiming));
       const int kmax = P.kmax;
+      const size_t bytes = (size_t)ncol * kmax * (20 + (path == 0 ? 8 * (size_t)nz : 0));
+      const int nch = (int)std::min<size_t>(HOST_CHUNKS, std::max<size_t>(1, bytes / HOST_CHUNK_BYTES));
       auto chunk = [&](int h, int& a, int& b) {
-        a = (int)((long long)ncol * h / HOST_CHUNKS);
-        b = (int)((long long)ncol * (h + 1) / HOST_CHUNKS);
+        a = (int)((long long)ncol * h / nch);
+        b = (int)((long long)ncol * (h + 1) / nch);
       };
       // every chunk is queued before the first copy is issued: a copy to
       // pageable host memory returns only when done, and the chunks behind
@@ -1868,7 +1873,7 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
       // other's last wave leaves idle (the outputs are disjoint columns).
       CK(cudaEventRecord(ctx->evefork, st));
       for (int i = 0; i < 2; ++i) CK(cudaStreamWaitEvent(ctx->estream[i], ctx->evefork, 0));
-      for (int h = 0; h < HOST_CHUNKS; ++h) {
+      for (int h = 0; h < nch; ++h) {
         int a, b;
         chunk(h, a, b);
         if (b <= a) continue;
@@ -1881,7 +1886,7 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
         CK(cudaEventRecord(ctx->evejoin[i], ctx->estream[i]));
         CK(cudaStreamWaitEvent(st, ctx->evejoin[i], 0));
       }
-      for (int h = 0; h < HOST_CHUNKS; ++h) {
+      for (int h = 0; h < nch; ++h) {
         int a, b;
         chunk(h, a, b);
         if (b <= a) continue;
