@@ -1099,7 +1099,8 @@ __device__ __noinline__ void eigen_column(int col, int ncol, int nz, int Lmax, c
                                              const SlotDesc* __restrict__ slots, int g0, int gn,
                                              const double* __restrict__ croot, const int32_t* __restrict__ cstat,
                                              int sphere, double* __restrict__ vc, double* __restrict__ vout,
-                                             double* __restrict__ kernel, int32_t* __restrict__ status, int ldo) {
+                                             double* __restrict__ kernel, int32_t* __restrict__ status, int ldo,
+                                             double* __restrict__ store) {
   constexpr int path = PATH;
   constexpr bool love = WT >= 2;
   using Layer = typename std::conditional<love, LoveLayer, RayLayer>::type;
@@ -1147,8 +1148,7 @@ __device__ __noinline__ void eigen_column(int col, int ncol, int nz, int Lmax, c
   }
   __syncthreads();
 
-  using Scratch = typename std::conditional<love, LoveScratch, RayScratch>::type;
-  Scratch scr;  // up-pass checkpoints and the segment being consumed (per slot thread)
+  const PassStore<love ? LOVE_STORE : RAY_STORE> scr{store + threadIdx.x, (int)blockDim.x};
   double kp[NZMAX];  // one pass's node sums; the scaled sums accumulate in the output
   NodeSink sink;
   sink.kp = (path == 0) ? kp : nullptr;
@@ -1275,32 +1275,58 @@ __device__ __noinline__ void eigen_column(int col, int ncol, int nz, int Lmax, c
   }
 }
 
+// Warps that an SM holds of a pass kernel (its launch bounds), and the blocks
+// of et threads for n columns: no more than fit the SMs, each taking every
+// gridDim.x-th column, so that the up-pass stores are those of the resident
+// threads only.  A map's phase slots run no pass: a block per column.
+constexpr int eigen_minb(int wt) { return wt >= 2 ? SWDK_EIGEN_MINB_LOVE : SWDK_EIGEN_MINB; }
+bool eigen_passes(int wt, int path) { return path == 0 || wt == 1 || wt == 3; }
+int eigen_blocks(int wt, int path, int et, long long n, int nsm) {
+  if (!eigen_passes(wt, path)) return (int)n;
+  return (int)std::min<long long>(n, (long long)nsm * (eigen_minb(wt) * 128 / et));
+}
+// doubles of up-pass store of one block
+size_t eigen_store(int wt, int path, int et, int Lmax) {
+  return eigen_passes(wt, path) ? (size_t)(wt >= 2 ? LOVE_STORE : RAY_STORE) * et * Lmax : 0;
+}
+int eigen_threads(int gn) { return std::min(128, ((gn + 31) / 32) * 32); }
+
 template <int WT, int PATH>
-__global__ void __launch_bounds__(128, (WT >= 2) ? SWDK_EIGEN_MINB_LOVE : SWDK_EIGEN_MINB) k_eigen(int ncol, int nz, int Lmax, const float4* __restrict__ lay0,
+__global__ void __launch_bounds__(128, eigen_minb(WT)) k_eigen(int ncol, int nz, int Lmax, const float4* __restrict__ lay0,
                                                const ColInfo* __restrict__ info, const float2* __restrict__ chainrule,
                                                const SlotDesc* __restrict__ slots, int g0, int gn,
                                                const double* __restrict__ croot, const int32_t* __restrict__ cstat,
                                                int sphere, double* __restrict__ vc, double* __restrict__ vout,
                                                double* __restrict__ kernel, int32_t* __restrict__ status, int ldo,
-                                               int col0) {
-  eigen_column<WT, PATH>(col0 + (int)blockIdx.x, ncol, nz, Lmax, lay0, info, chainrule, slots, g0, gn, croot, cstat, sphere, vc,
-                         vout, kernel, status, ldo);
+                                               int col0, int col1, double* __restrict__ store) {
+  if (PATH == 0 || (WT & 1)) store += (size_t)blockIdx.x * blockDim.x * Lmax * (WT >= 2 ? LOVE_STORE : RAY_STORE);
+#pragma unroll 1
+  for (int col = col0 + (int)blockIdx.x; col < col1; col += gridDim.x) {
+    __syncthreads();  // the layer records of the last column are read
+    eigen_column<WT, PATH>(col, ncol, nz, Lmax, lay0, info, chainrule, slots, g0, gn, croot, cstat, sphere, vc,
+                           vout, kernel, status, ldo, store);
+  }
 }
 
-// the same over a ragged batch: block b is column b - blk0 of the model of
+// the same over a ragged batch: item b is column b - blk0 of the model of
 // the REBlock entry holding b
 template <int WT, int PATH>
-__global__ void __launch_bounds__(128, (WT >= 2) ? SWDK_EIGEN_MINB_LOVE : SWDK_EIGEN_MINB)
+__global__ void __launch_bounds__(128, eigen_minb(WT))
     k_eigen_ragged(const REBlock* __restrict__ eb, int neb, const RModel* __restrict__ models,
                    const float4* __restrict__ lay0, const ColInfo* __restrict__ info,
                    const float2* __restrict__ chainrule, const SlotDesc* __restrict__ slots,
-                   const double* __restrict__ croot, const int32_t* __restrict__ cstat, int sphere) {
-  const long long b = blockIdx.x;
-  const REBlock E = eb[ragged_find(eb, neb, b, &REBlock::blk0)];
-  const RModel M = models[E.model];
-  eigen_column<WT, PATH>((int)(b - E.blk0), M.ncol, M.nz, M.Lmax, lay0 + M.lay0, info + M.col0, chainrule + M.crs0,
-                         slots, E.g0, E.gn, croot + M.root0, cstat + M.root0, sphere, M.vc, M.vout, M.kernel,
-                         M.status, M.ncol);
+                   const double* __restrict__ croot, const int32_t* __restrict__ cstat, int sphere,
+                   long long nblk, int maxL, double* __restrict__ store) {
+  if (PATH == 0 || (WT & 1)) store += (size_t)blockIdx.x * blockDim.x * maxL * (WT >= 2 ? LOVE_STORE : RAY_STORE);
+#pragma unroll 1
+  for (long long b = blockIdx.x; b < nblk; b += gridDim.x) {
+    const REBlock E = eb[ragged_find(eb, neb, b, &REBlock::blk0)];
+    const RModel M = models[E.model];
+    __syncthreads();  // the layer records of the last column are read
+    eigen_column<WT, PATH>((int)(b - E.blk0), M.ncol, M.nz, M.Lmax, lay0 + M.lay0, info + M.col0, chainrule + M.crs0,
+                           slots, E.g0, E.gn, croot + M.root0, cstat + M.root0, sphere, M.vc, M.vout, M.kernel,
+                           M.status, M.ncol, store);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1491,6 +1517,7 @@ struct swdk_ctx {
   bool dirty = true;
   Plan plan[2];  // 0: get_1d_kernel, 1: get_2d_map
   DevBuf layR, layL, lay0, info, chainrule, croot, cstat, nevals, depth_d, ierr, queue;
+  DevBuf store;         // up-pass values of the eigen stage's resident threads
   DevBuf nodes, dltab;  // grid nodes and the depth grid's flattening (node-source root search)
   int roots_blocks = 0, nsm = 148;
   bool coop_ready = false;  // the layered-model call's kernels are opted in to their shared memory
@@ -1733,7 +1760,7 @@ struct HostOut {
 };
 
 int launch_eigen(swdk_ctx* ctx, const Plan& P, int path, int ncol, int nz, int c0, int c1, double* d_vc,
-                 double* d_vout, double* d_kernel, int32_t* d_status, int ldo, cudaStream_t st);
+                 double* d_vout, double* d_kernel, int32_t* d_status, int ldo, double* store, cudaStream_t st);
 
 int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_vs, const float* d_vp,
                const float* d_rho, double* d_vc, double* d_vout, double* d_kernel, int32_t* d_status,
@@ -1807,6 +1834,15 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
     ctx->nsm = nsm;
     ctx->roots_blocks = std::max(1, nsm * std::max(1, per));
   }
+  size_t store = 0;  // doubles of the eigen stage's up-pass stores
+  if (!roots_only) {
+    for (int g = 0; g < P.groups.n; ++g) {
+      const int wt = P.slots[P.groups.start[g]].wtype, et = eigen_threads(P.groups.count[g]);
+      store = std::max(store, eigen_blocks(wt, path, et, ncol, ctx->nsm) * eigen_store(wt, path, et, Lmax));
+    }
+    if (ho) store *= 2;  // its chunks run on two streams
+    CK(ctx->store.ensure(store * sizeof(double)));
+  }
   const int nitems = (int)P.chains.size() * ncol;
   const int rblocks = ctx->cfg.block_roots > 0 ? ctx->cfg.block_roots : ctx->roots_blocks;
   const unsigned int rcap = (unsigned int)std::min<size_t>((size_t)P.nroot * ncol, 0x7fffffffu);
@@ -1845,7 +1881,8 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
   if (timing) CK(cudaEventRecord(ctx->ev[2], st));
   if (!roots_only) {
     if (!ho) {
-      r = launch_eigen(ctx, P, path, ncol, nz, 0, ncol, d_vc, d_vout, d_kernel, d_status, ldo, st);
+      r = launch_eigen(ctx, P, path, ncol, nz, 0, ncol, d_vc, d_vout, d_kernel, d_status, ldo,
+                       ctx->store.as<double>(), st);
       if (r) return r;
     } else {
       // host-memory call: the eigen stage in column chunks, each chunk's
@@ -1878,7 +1915,8 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
         chunk(h, a, b);
         if (b <= a) continue;
         cudaStream_t es = ctx->estream[h & 1];
-        r = launch_eigen(ctx, P, path, ncol, nz, a, b, d_vc, d_vout, d_kernel, d_status, ldo, es);
+        r = launch_eigen(ctx, P, path, ncol, nz, a, b, d_vc, d_vout, d_kernel, d_status, ldo,
+                         ctx->store.as<double>() + (h & 1) * (store / 2), es);
         if (r) return r;
         CK(cudaEventRecord(ctx->evchunk[h], es));
       }
@@ -1969,22 +2007,22 @@ void collect_stats(swdk_ctx* ctx) {
 
 // the eigen stage over columns [c0, c1): one launch per wave-type slot group
 int launch_eigen(swdk_ctx* ctx, const Plan& P, int path, int ncol, int nz, int c0, int c1, double* d_vc,
-                 double* d_vout, double* d_kernel, int32_t* d_status, int ldo, cudaStream_t st) {
+                 double* d_vout, double* d_kernel, int32_t* d_status, int ldo, double* store, cudaStream_t st) {
   using EigFn = void (*)(int, int, int, const float4*, const ColInfo*, const float2*, const SlotDesc*, int, int,
-                         const double*, const int32_t*, int, double*, double*, double*, int32_t*, int, int);
+                         const double*, const int32_t*, int, double*, double*, double*, int32_t*, int, int, int, double*);
   static const EigFn eig[4][2] = {{k_eigen<0, 0>, k_eigen<0, 1>}, {k_eigen<1, 0>, k_eigen<1, 1>},
                                   {k_eigen<2, 0>, k_eigen<2, 1>}, {k_eigen<3, 0>, k_eigen<3, 1>}};
   const int Lmax = 4 * nz - 3;
   for (int g = 0; g < P.groups.n; ++g) {
     const int g0 = P.groups.start[g], gn = P.groups.count[g];
     const int wt = P.slots[g0].wtype;
-    const int et = std::min(128, ((gn + 31) / 32) * 32);
+    const int et = eigen_threads(gn);
     const size_t smem = (size_t)Lmax * (wt >= 2 ? sizeof(LoveLayer) : sizeof(RayLayer)) + (size_t)nz * sizeof(float2);
     ctx->launches += 1;
-    eig[wt][path]<<<c1 - c0, et, smem, st>>>(ncol, nz, Lmax, ctx->lay0.as<float4>(), ctx->info.as<ColInfo>(),
+    eig[wt][path]<<<eigen_blocks(wt, path, et, c1 - c0, ctx->nsm), et, smem, st>>>(ncol, nz, Lmax, ctx->lay0.as<float4>(), ctx->info.as<ColInfo>(),
                                              ctx->chainrule.as<float2>(), P.d_slots.as<SlotDesc>(), g0, gn,
                                              ctx->croot.as<double>(), ctx->cstat.as<int32_t>(), ctx->cfg.sphere,
-                                             d_vc, d_vout, d_kernel, d_status, ldo, c0);
+                                             d_vc, d_vout, d_kernel, d_status, ldo, c0, c1, store);
     CK(cudaGetLastError());
   }
   return SWDK_OK;
@@ -2204,7 +2242,7 @@ void swdk_destroy(swdk_ctx* ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->cfg.device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  DevBuf* bufs[] = {&ctx->layR, &ctx->layL, &ctx->lay0, &ctx->info, &ctx->chainrule, &ctx->croot, &ctx->cstat,
+  DevBuf* bufs[] = {&ctx->layR, &ctx->layL, &ctx->lay0, &ctx->info, &ctx->chainrule, &ctx->store, &ctx->croot, &ctx->cstat,
                     &ctx->nodes, &ctx->dltab,
                     &ctx->nevals, &ctx->depth_d, &ctx->ierr, &ctx->in_vs, &ctx->in_vp, &ctx->in_rho,
                     &ctx->out_vc, &ctx->out_vout, &ctx->out_kernel, &ctx->out_status, &ctx->in_misc,
@@ -2652,7 +2690,7 @@ struct swdk_ragged {
   int maxL = 0, maxnz = 0, roots_blocks = 0, nsm = 148;
   bool useprop = false;
   DevBuf d_models, d_blocks, d_eb[4], d_chains, d_periods, d_slots;
-  DevBuf layR, layL, lay0, info, chainrule, croot, cstat, prop, nodefeat, retry_list, retry_ctr, queue, nevals;
+  DevBuf layR, layL, lay0, info, chainrule, store, croot, cstat, prop, nodefeat, retry_list, retry_ctr, queue, nevals;
   DevBuf nodes, dltab;
   long long node_tot = 0, dl_tot = 0;
   cudaStream_t stream = nullptr;
@@ -2748,7 +2786,7 @@ int ragged_enqueue(swdk_ragged* R, cudaStream_t st, bool timing) {
   if (timing) CK(cudaEventRecord(R->ev[2], st));
   if (R->path != 2) {
     using EigR = void (*)(const REBlock*, int, const RModel*, const float4*, const ColInfo*, const float2*,
-                          const SlotDesc*, const double*, const int32_t*, int);
+                          const SlotDesc*, const double*, const int32_t*, int, long long, int, double*);
     static const EigR eig[4][2] = {{k_eigen_ragged<0, 0>, k_eigen_ragged<0, 1>},
                                    {k_eigen_ragged<1, 0>, k_eigen_ragged<1, 1>},
                                    {k_eigen_ragged<2, 0>, k_eigen_ragged<2, 1>},
@@ -2758,10 +2796,10 @@ int ragged_enqueue(swdk_ragged* R, cudaStream_t st, bool timing) {
       const size_t smem = (size_t)R->maxL * (wt >= 2 ? sizeof(LoveLayer) : sizeof(RayLayer)) +
                           (size_t)R->maxnz * sizeof(float2);
       R->launches += 1;
-      eig[wt][R->path]<<<(unsigned)R->eblocks[wt], R->et[wt], smem, st>>>(
+      eig[wt][R->path]<<<eigen_blocks(wt, R->path, R->et[wt], R->eblocks[wt], R->nsm), R->et[wt], smem, st>>>(
           R->d_eb[wt].as<REBlock>(), (int)R->eb[wt].size(), R->d_models.as<RModel>(), R->lay0.as<float4>(),
           R->info.as<ColInfo>(), R->chainrule.as<float2>(), R->d_slots.as<SlotDesc>(), R->croot.as<double>(),
-          R->cstat.as<int32_t>(), cfg.sphere);
+          R->cstat.as<int32_t>(), cfg.sphere, R->eblocks[wt], R->maxL, R->store.as<double>());
       CK(cudaGetLastError());
     }
   }
@@ -2804,7 +2842,7 @@ void swdk_ragged_destroy(swdk_ragged* R) {
   if (R->exec) cudaGraphExecDestroy(R->exec);
   if (R->graph) cudaGraphDestroy(R->graph);
   DevBuf* bufs[] = {&R->d_models, &R->d_blocks, &R->d_eb[0], &R->d_eb[1], &R->d_eb[2], &R->d_eb[3], &R->d_chains,
-                    &R->d_periods, &R->d_slots, &R->layR, &R->layL, &R->lay0, &R->info, &R->chainrule, &R->croot,
+                    &R->d_periods, &R->d_slots, &R->layR, &R->layL, &R->lay0, &R->info, &R->chainrule, &R->store, &R->croot,
                     &R->cstat, &R->prop, &R->nodefeat, &R->retry_list, &R->retry_ctr, &R->queue, &R->nevals,
                     &R->nodes, &R->dltab};
   for (DevBuf* b : bufs) b->release();
@@ -2898,7 +2936,7 @@ int swdk_ragged_create(int n, swdk_ctx* const* ctxs, const swdk_call* calls, swd
       E.pad_ = 0;
       R->eb[wt].push_back(E);
       R->eblocks[wt] += M.ncol;
-      R->et[wt] = std::max(R->et[wt], std::min(128, ((E.gn + 31) / 32) * 32));
+      R->et[wt] = std::max(R->et[wt], eigen_threads(E.gn));
     }
     if (proposals_on(c)) R->useprop = true;
     // the model's depth vector on the device (k_prep reads it)
@@ -2959,9 +2997,15 @@ int swdk_ragged_create(int n, swdk_ctx* const* ctxs, const swdk_call* calls, swd
   int dev = 0, nsm = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  R->nsm = std::max(1, nsm);
+  size_t store = 0;
+  for (int wt = 0; wt < 4 && R->path != 2; ++wt)
+    if (R->eblocks[wt])
+      store = std::max(store, eigen_blocks(wt, R->path, R->et[wt], R->eblocks[wt], R->nsm) *
+                                  eigen_store(wt, R->path, R->et[wt], R->maxL));
+  if (store) e = R->store.ensure(store * sizeof(double));
   if (e == cudaSuccess) e = roots_occupancy(&per);
   if (e != cudaSuccess) return bail(SWDK_E_CUDA, std::string("ragged batch set-up: ") + cudaGetErrorString(e));
-  R->nsm = std::max(1, nsm);
   R->roots_blocks = ctx->cfg.block_roots > 0 ? ctx->cfg.block_roots : std::max(1, nsm * std::max(1, per));
   *out = R;
   return SWDK_OK;

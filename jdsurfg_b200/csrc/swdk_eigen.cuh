@@ -558,23 +558,42 @@ SWDK_HD int pass_layers(const Layer* lay, int L, double k2, double om2, double t
 // relative (CPU harness test).
 constexpr double EIG_TRUNC_Q = 0.0;
 
-// Up-pass storage of a Rayleigh pass with checkpoints: the compound vector
-// (and its exponent bookkeeping) is kept only at every RAY_SEG-th layer and
-// at the half-space; the down sweep recomputes each segment of RAY_SEG
-// layers from its checkpoint into seg[] just before it needs them.  The
-// recomputation repeats the up pass's arithmetic exactly, so the values are
-// the ones a full per-layer store would hold, with about 2 KB of scratch per
-// slot instead of 6 doubles per layer.
-#ifndef SWDK_RAY_SEG
-#define SWDK_RAY_SEG 16
-#endif
-constexpr int RAY_SEG = SWDK_RAY_SEG;
-constexpr int RAY_NCK = (LMAX + RAY_SEG - 1) / RAY_SEG;
-struct RayScratch {
-  double ck[RAY_NCK][8];  // layer j*RAY_SEG: cd[5], exponent sum, exr, exi
-  double hs[8];           // the half-space start of the (cut) pass
-  double seg[RAY_SEG][6];  // the segment being consumed: cd[5], exponent sum
+// Up-pass storage of a pass: N doubles per layer, kept for the down sweep.
+// Rayleigh: the compound vector cd[5] and its exponent sum; Love: uu, tt, exl.
+//
+// The device keeps them in global memory (PassStore), one thread's doubles a
+// block width apart, so a warp's loads and stores are whole lines: 48 (24)
+// bytes out and back per layer and slot, under a sixth of the memory's rate
+// at the pace of the sweeps, and fetched before the layer's square roots and
+// exponentials need the time anyway.  (Checkpoints at every 16th layer with the
+// segments computed a second time, 2 KB of local memory a slot, cost a second
+// evaluation of every layer: eigen stage 133 ms against 108 ms at 65 536
+// columns of 64 nodes, 60 Rayleigh and 60 Love periods.)
+template <int N>
+struct PassStore {
+  double* p;   // this thread's first double
+  int stride;  // threads of the block
+  SWDK_HD void put(int l, const double* v) const {
+    for (int i = 0; i < N; ++i) p[(size_t)(l * N + i) * stride] = v[i];
+  }
+  SWDK_HD void get(int l, double* v) const {
+    for (int i = 0; i < N; ++i) v[i] = p[(size_t)(l * N + i) * stride];
+  }
 };
+constexpr int RAY_STORE = 6, LOVE_STORE = 3;
+// the same within the caller's frame
+template <int N>
+struct LocalStore {
+  double v[LMAX][N];
+  SWDK_HD void put(int l, const double* x) {
+    for (int i = 0; i < N; ++i) v[l][i] = x[i];
+  }
+  SWDK_HD void get(int l, double* x) const {
+    for (int i = 0; i < N; ++i) x[i] = v[l][i];
+  }
+};
+using RayScratch = LocalStore<RAY_STORE>;
+using LoveScratch = LocalStore<LOVE_STORE>;
 
 // one step of the up pass (sregn96.f90:401-489) after vars_lean of its
 // layer: the compound vector cd of layer m from that of layer m+1 (in
@@ -594,28 +613,20 @@ SWDK_HD void ray_up_apply(const LVars& v, const RayLayer& y, int iw, const SlotK
   cd[5] = exr + (double)exi * LN2;
 }
 
-SWDK_HD void ray_keep(double* dst, const double* cd, double exr, int exi) {
-  for (int i = 0; i < 6; ++i) dst[i] = cd[i];
-  dst[6] = exr;
-  dst[7] = (double)exi;
-}
-
 // One Rayleigh pass (sregn96's svfunc + energy) at (omega, wvno) over the
 // column's layer records lay[0..L-1] (top-down, lay[L-1] the half-space),
 // depth-truncated by pass_layers.  Returns ugr (flat) and norm = ugr*sumi0;
 // the raw layer kernels go to the sink as the top-down sweep produces them.
 //
-// One loop runs the up pass (layers L-2 .. 0, keeping checkpoints), then
-// the top-down sweep (layers 0 .. L-1), which at the first layer of each
-// segment recomputes the segment's compound vectors from its checkpoint by
-// further up steps.  Every step evaluates its layer's variables (vars_lean:
-// square roots, exponentials or sines and cosines) at one place in the
-// code, so the kernel holds one copy of that code instead of three (the
-// Rayleigh eigen kernel waited on instruction fetch about as often as on
-// its FP64 results).  The steps and their arithmetic are those of separate
-// up, recompute and down loops.
-template <class Sink>
-SWDK_HDI void rayleigh_pass(const RayLayer* lay, int Lfull, double omega, double wvno, RayScratch& scr, double& ugr,
+// One loop runs the up pass (layers L-2 .. 0, into the store), then the
+// top-down sweep (layers 0 .. L-1).  Every step evaluates its layer's
+// variables (vars_lean: square roots, exponentials or sines and cosines) at
+// one place in the code, so the kernel holds one copy of that code instead of
+// two (the Rayleigh eigen kernel waited on instruction fetch about as often as
+// on its FP64 results).  The steps and their arithmetic are those of separate
+// up and down loops.
+template <class Store, class Sink>
+SWDK_HDI void rayleigh_pass(const RayLayer* lay, int Lfull, double omega, double wvno, Store& scr, double& ugr,
                             double& norm, const Sink& sink, double trunc_q = EIG_TRUNC_Q) {
   const SlotK s = slot_consts(omega, wvno);
   const int L = pass_layers(lay, Lfull, s.k2, s.om2, trunc_q);
@@ -628,8 +639,7 @@ SWDK_HDI void rayleigh_pass(const RayLayer* lay, int Lfull, double omega, double
   }
   double exr = 0.0;
   int exi = 0;
-  ray_keep(scr.hs, cd, exr, exi);
-  if ((L - 1) % RAY_SEG == 0) ray_keep(scr.ck[(L - 1) / RAY_SEG], cd, exr, exi);
+  scr.put(L - 1, cd);
   // ---- down + svfunc + energy state ----
   double if1213 = 0.0, exe0 = 0.0;
   Eig4 u0 = {0.0, 0.0, 0.0, 0.0};
@@ -638,60 +648,33 @@ SWDK_HDI void rayleigh_pass(const RayLayer* lay, int Lfull, double omega, double
   int dxi = 0;
   EnergyAcc acc = {0.0, 0.0, 0.0, 0.0};
   const double c = omega * s.ik;
-  int up = L - 2;        // layer of the next up-pass step (< 0: the up pass is done)
-  int dn = 0;            // layer of the next down step
-  int sl = -1, sj0 = -1;  // segment recomputation: its next layer sl while sl > sj0
+  int lm = L - 2;         // layer of the step
   bool down = false;
-  auto begin_down = [&]() {
+  auto begin_down = [&]() {  // cd is layer 0's
     sink.start();
-    const double* top = scr.ck[0];  // layer 0
-    if1213 = -1.0 / top[1];
-    exe0 = top[5];
-    u0.ur = top[2] / top[1];
+    if1213 = -1.0 / cd[1];
+    exe0 = cd[5];
+    u0.ur = cd[2] / cd[1];
     u0.uz = 1.0; u0.tz = 0.0; u0.tr = 0.0;
     if (lay[0].zb <= 0.0) { u0.ur = 0.0; u0.tr = 0.0; }  // fluid top (jwat)
     down = true;
+    lm = 0;
   };
-  if (up < 0) begin_down();
+  if (lm < 0) begin_down();
 #pragma unroll 1  // a layer recursion: unrolling only grows the code
   for (;;) {
-    int lm;
-    bool upstep;
-    if (!down) {
-      lm = up;
-      upstep = true;
-    } else {
-      const int j0 = dn - dn % RAY_SEG;  // first layer of dn's segment
-      if (sl <= sj0 && dn == j0 && dn < L - 1 && sj0 != j0) {
-        // cd of layers j0+1 .. t from the checkpoint at t
-        const int t = (j0 + RAY_SEG < L - 1) ? j0 + RAY_SEG : L - 1;
-        const double* src = (t == L - 1) ? scr.hs : scr.ck[t / RAY_SEG];
-        for (int i = 0; i < 6; ++i) cd[i] = src[i];
-        exr = src[6];
-        exi = (int)src[7];
-        for (int i = 0; i < 6; ++i) scr.seg[t - j0 - 1][i] = cd[i];
-        sj0 = j0;
-        sl = t - 1;
-      }
-      upstep = sl > sj0;
-      lm = upstep ? sl : dn;
-    }
     const RayLayer& y = lay[lm];
     const int iw = (y.zb > 0.0) ? 0 : 1;
+    if (down && lm < L - 1) scr.get(lm + 1, cd);
     LVars v;
     vars_lean(s.k2 - s.om2 * y.ia2, s.k2 - s.om2 * y.ib2, y.d, iw, v);
-    if (upstep) {
+    if (!down) {
       ray_up_apply(v, y, iw, s, cd, exr, exi);
-      if (!down) {
-        if (up % RAY_SEG == 0) ray_keep(scr.ck[up / RAY_SEG], cd, exr, exi);
-        if (--up < 0) begin_down();
-      } else {
-        for (int i = 0; i < 6; ++i) scr.seg[sl - sj0 - 1][i] = cd[i];
-        --sl;
-      }
+      if (lm > 0) scr.put(lm, cd);
+      if (--lm < 0) begin_down();
       continue;
     }
-    const bool half = (dn == L - 1);
+    const bool half = (lm == L - 1);
     Eig4 u1 = u0;
     if (!half) {
       double a0[4];
@@ -704,14 +687,13 @@ SWDK_HDI void rayleigh_pass(const RayLayer* lay, int Lfull, double omega, double
       dxr = dxr + v.pex;
       dxi += e;
       const double exa1 = dxr + (double)dxi * LN2;
-      const double* cd1 = scr.seg[dn - (dn - dn % RAY_SEG)];  // layer dn + 1
-      u1 = eigen_at(cd1, vv, exa1 + cd1[5] - exe0, if1213);
+      u1 = eigen_at(cd, vv, exa1 + cd[5] - exe0, if1213);
     }
     double da, db, dr;
     energy_lean(y, v, iw, half, u0, u1, s, c, acc, da, db, dr);
-    sink.add(dn, y.vtp, y.rtp, da, db, dr);
+    sink.add(lm, y.vtp, y.rtp, da, db, dr);
     u0 = u1;
-    if (++dn >= L) break;
+    if (++lm >= L) break;
   }
   sink.finish();
   ugr = (wvno * acc.sumi1 + acc.sumi2) / (omega * acc.sumi0);
@@ -720,17 +702,9 @@ SWDK_HDI void rayleigh_pass(const RayLayer* lay, int Lfull, double omega, double
 
 // ---------------------------------------------------------------------------
 // One Love pass (slegn96.f90): up, shfunc normalisation, energy.  The up
-// pass keeps (uu, tt, exl) only at every RAY_SEG-th layer and the
-// half-space; the energy sweep recomputes each segment from its checkpoint
-// and applies shfunc's normalisation exp(-ext) on the fly.  Returns ugr and
-// the normaliser sumi1.
+// pass keeps (uu, tt, exl) of every layer; the energy sweep applies shfunc's
+// normalisation exp(-ext) on the fly.  Returns ugr and the normaliser sumi1.
 // ---------------------------------------------------------------------------
-struct LoveScratch {
-  double ck[RAY_NCK][3];
-  double hs[3];
-  double seg[RAY_SEG + 1][3];  // layers j0 .. j0 + RAY_SEG of the current segment
-};
-
 // one step of slegn96's up pass (slegn96.f90:372-445): (uu, tt) of layer k
 // from layer k+1 (s1), power-of-two normalised, and the step's exponent exl
 SWDK_HD void love_up_step(const LoveLayer& y, double wvno2, double om2, const double* s1, double* sk) {
@@ -766,22 +740,12 @@ SWDK_HD void love_up_step(const LoveLayer& y, double wvno2, double om2, const do
   sk[2] = (double)e * LN2 + eexl;
 }
 
-// the raw up-pass values of layers j0 .. t (t the checkpoint at or below
-// j0 + RAY_SEG) into seg[0 .. t - j0]
-SWDK_HD void love_fill_segment(const LoveLayer* lay, int L, double wvno2, double om2, LoveScratch& scr, int j0) {
-  const int t = (j0 + RAY_SEG < L - 1) ? j0 + RAY_SEG : L - 1;
-  const double* src = (t == L - 1) ? scr.hs : scr.ck[t / RAY_SEG];
-  for (int i = 0; i < 3; ++i) scr.seg[t - j0][i] = src[i];
-#pragma unroll 1
-  for (int l = t - 1; l >= j0; --l) love_up_step(lay[l], wvno2, om2, scr.seg[l - j0 + 1], scr.seg[l - j0]);
-}
-
-template <class Sink>
-SWDK_HDI void love_pass(const LoveLayer* lay, int Lfull, double omega, double wvno, LoveScratch& scr, double& ugr,
+template <class Store, class Sink>
+SWDK_HDI void love_pass(const LoveLayer* lay, int Lfull, double omega, double wvno, Store& scr, double& ugr,
                         double& norm, const Sink& sink, double trunc_q = EIG_TRUNC_Q) {
   const double wvno2 = wvno * wvno, om2 = omega * omega, ik = 1.0 / wvno, ik2 = ik * ik;
   const int L = pass_layers(lay, Lfull, wvno2, om2, trunc_q);
-  // ---- up (slegn96.f90:372-445), checkpoints only ----
+  // ---- up (slegn96.f90:372-445) ----
   double sv[3];
   {
     const LoveLayer& y = lay[L - 1];
@@ -795,35 +759,32 @@ SWDK_HDI void love_pass(const LoveLayer* lay, int Lfull, double omega, double wv
     }
     sv[2] = 0.0;
   }
-  for (int i = 0; i < 3; ++i) scr.hs[i] = sv[i];
-  if ((L - 1) % RAY_SEG == 0)
-    for (int i = 0; i < 3; ++i) scr.ck[(L - 1) / RAY_SEG][i] = sv[i];
+  scr.put(L - 1, sv);
 #pragma unroll 1  // a layer recursion: unrolling only grows the code
   for (int k = L - 2; k >= 0; --k) {
     double nv[3];
     love_up_step(lay[k], wvno2, om2, sv, nv);
     for (int i = 0; i < 3; ++i) sv[i] = nv[i];
-    if (k % RAY_SEG == 0)
-      for (int i = 0; i < 3; ++i) scr.ck[k / RAY_SEG][i] = sv[i];
+    if (k > 0) scr.put(k, sv);
   }
   // ---- shfunc normalisation (slegn96.f90:212-240): layer k's (uu, tt)
   // are the raw values times exp(-ext), ext summing the exl of the solid
   // layers above; tt(1) = 0.  The amplitude scale umax is uu(1) unless
   // that is zero (a fluid top), then the largest normalised |uu|. ----
-  const double top0 = scr.ck[0][0];
+  const double top0 = sv[0], topx = sv[2];  // layer 0's
   double umax = top0;
   if (top0 == 0.0) {
-    double ext = 0.0;
+    double ext = 0.0, exl = topx;
 #pragma unroll 1
     for (int k = 1; k < L; ++k) {
-      const int j0 = (k - 1) - (k - 1) % RAY_SEG;
-      if (k - 1 == j0) love_fill_segment(lay, L, wvno2, om2, scr, j0);
-      double u = 0.0;
+      double w[3], u = 0.0;
+      scr.get(k, w);
       if (lay[k].zb > 0.0) {
-        ext = ext + scr.seg[k - 1 - j0][2];
+        ext = ext + exl;
         const double fact = (ext < 80.0) ? exp(-ext) : 0.0;
-        u = scr.seg[k - j0][0] * fact;
+        u = w[0] * fact;
       }
+      exl = w[2];
       if (fabs(u) > fabs(umax)) umax = u;
     }
   }
@@ -831,21 +792,23 @@ SWDK_HDI void love_pass(const LoveLayer* lay, int Lfull, double omega, double wv
   // ---- energy (slegn96.f90:447-576) with uu/tt scaled by 1/umax on the fly ----
   const double c = omega * ik;
   double sumi0 = 0.0, sumi1 = 0.0;
-  double ext = 0.0;
+  double ext = 0.0, exl = topx;  // exl: layer k's
   double uu = top0 * iumax, tt = 0.0;
+  double nxt[3] = {0.0, 0.0, 0.0};  // layer k + 1's, fetched a layer ahead
+  if (L > 1) scr.get(1, nxt);
   sink.start();
 #pragma unroll 1  // a layer recursion: unrolling only grows the code
   for (int k = 0; k < L; ++k) {
-    const int j0 = k - k % RAY_SEG;
     double nuu = 0.0, ntt = 0.0;
     if (k < L - 1) {
-      if (k == j0) love_fill_segment(lay, L, wvno2, om2, scr, j0);
       if (lay[k + 1].zb > 0.0) {
-        ext = ext + scr.seg[k - j0][2];
+        ext = ext + exl;
         const double fact = (ext < 80.0) ? exp(-ext) : 0.0;
-        nuu = scr.seg[k + 1 - j0][0] * fact * iumax;
-        ntt = scr.seg[k + 1 - j0][1] * fact * iumax;
+        nuu = nxt[0] * fact * iumax;
+        ntt = nxt[1] * fact * iumax;
       }
+      exl = nxt[2];
+      if (k + 2 < L) scr.get(k + 2, nxt);
     }
     const LoveLayer& y = lay[k];
     const double zb = y.zb;
