@@ -1157,21 +1157,97 @@ __device__ __noinline__ void eigen_column(int col, int ncol, int nz, int Lmax, c
   sink.nw = ci.nw;
   sink.nz = nz;
   const NodeSink nosink = {nullptr, crs, L, ci.nw, nz};
+  constexpr bool group = (WT == 1 || WT == 3);
+  if constexpr (PATH == 0 && group) {
+    // sregnpu / slegnpu (sregn96.f90:1737-1878, slegn96.f90:785-918): a slot's
+    // three passes, at its period and the two beside it, by three threads.  A
+    // thread leaves its node sums in its own store, which its pass is done
+    // with; the slot's three threads then share the nodes and add the scaled
+    // sums in the order of the passes.  (One thread for all three took
+    // 3.1 ms of eigen stage where this takes 2.0, 1188 columns of 41 nodes
+    // and 19 group periods: a third of the threads, three times the chain.)
+    __shared__ double norms[128], ugrs[128];
+    const int per = blockDim.x / 3;  // slots of a round
+    const int pass = threadIdx.x / per, j = threadIdx.x % per;
+#pragma unroll 1
+    for (int s0 = 0; s0 < gn; s0 += per) {
+      const bool on = pass < 3 && s0 + j < gn;
+      const SlotDesc sd = slots[g0 + (on ? s0 + j : 0)];
+      const double c0 = croot[(size_t)sd.r0 * ncol + col];
+      const double c1 = croot[(size_t)sd.r1 * ncol + col];
+      const double c2 = croot[(size_t)sd.r2 * ncol + col];
+      const size_t oo = (size_t)sd.oslot * ldo + col;  // outputs: row stride ldo (>= ncol)
+      double* kout = kernel + (size_t)sd.oslot * nz * ldo + col;  // node i at kout[i * ldo]
+      const bool dead = !ci.valid || c0 == 0.0 || c1 == 0.0 || c2 == 0.0;
+      if (on && pass == 0) {
+        int st = cstat[(size_t)sd.r0 * ncol + col];
+        st = worst_status(st, cstat[(size_t)sd.r1 * ncol + col]);
+        st = worst_status(st, cstat[(size_t)sd.r2 * ncol + col]);
+        if (!ci.valid) st = ST_NAN_INPUT;
+        else if (dead) st = ST_NO_ROOT;
+        if (status) status[oo] = st;
+      }
+      if (on && !dead) {
+        const double tt = (pass == 0) ? sd.t : (pass == 1) ? sd.t1 : sd.t2;
+        const double cc = (pass == 0) ? c0 : (pass == 1) ? c1 : c2;
+        const double omega = 2.0 * PI_F / tt, wvno = omega / cc;
+        double ugr, norm;
+        for (int i = 0; i < nz; ++i) kp[i] = 0.0;
+        if constexpr (love) love_pass(lay, L, omega, wvno, scr, ugr, norm, sink);
+        else rayleigh_pass(lay, L, omega, wvno, scr, ugr, norm, sink);
+        norms[threadIdx.x] = norm;
+        ugrs[threadIdx.x] = ugr;
+        for (int i = 0; i < nz; ++i) scr.p[(size_t)i * scr.stride] = kp[i];
+      }
+      __syncthreads();
+      if (on && dead) {
+        if (pass == 0) {
+          vc[oo] = 0.0;
+          vout[oo] = 0.0;
+        }
+        for (int i = pass; i < nz; i += 3) kout[(size_t)i * ldo] = 0.0;
+      } else if (on) {
+        const double cp = c0, cg = ugrs[j];
+        const double uc1 = cg / cp;
+        const double dtt = sd.t2 - sd.t1;
+        const double f1 = uc1 * (2.0 - uc1);
+        const double f2 = uc1 * uc1 * sd.t;
+        double tm = 1.0, coef0 = 0.0;
+        if (sphere) {
+          const double om0 = 2.0 * PI_F / sd.t;
+          const double k = love ? 1.5 : 0.5;
+          const double x = (love ? 3.0 : 1.0) * cp / (2. * ar * om0);
+          tm = sqrt(1. + x * x);
+          const double y = k / (ar * om0);
+          const double tm1 = (y * y) / tm;
+          coef0 = cg * cp * tm1;
+        }
+        const double coef1 = tm * (f2 / dtt), coef2 = tm * (f1 - f2 / dtt);
+        const double sc0 = coef0 / norms[j], sc1 = coef1 / norms[j + per], sc2 = coef2 / norms[j + 2 * per];
+        const double* ks = store + j;  // the three threads' node sums
+        for (int i = pass; i < nz; i += 3) {
+          const double* ki = ks + (size_t)i * scr.stride;
+          double v = 0.0;
+          if (coef0 != 0.0) v = v + ki[0] * sc0;
+          if (coef1 != 0.0) v = v + ki[per] * sc1;
+          if (coef2 != 0.0) v = v + ki[2 * per] * sc2;
+          // water / merged fluid nodes carry no kernel (SurfaceWave.cpp:495)
+          kout[(size_t)i * ldo] = (i < ci.nw) ? 0.0 : v;
+        }
+        if (pass == 0) {
+          vc[oo] = cp / tm;
+          vout[oo] = cg * tm;
+        }
+      }
+      __syncthreads();  // the sums are read: the next round's passes write the stores
+    }
+  } else
   for (int s = threadIdx.x; s < gn; s += blockDim.x) {
     const SlotDesc sd = slots[g0 + s];
-    constexpr bool group = (WT == 1 || WT == 3);
     const double c0 = croot[(size_t)sd.r0 * ncol + col];
     int st = cstat[(size_t)sd.r0 * ncol + col];
-    double c1 = 0.0, c2 = 0.0;
-    const bool three = (path == 0) && group;
-    if (three) {
-      c1 = croot[(size_t)sd.r1 * ncol + col];
-      c2 = croot[(size_t)sd.r2 * ncol + col];
-      st = worst_status(st, cstat[(size_t)sd.r1 * ncol + col]);
-      st = worst_status(st, cstat[(size_t)sd.r2 * ncol + col]);
-    }
     const size_t oo = (size_t)sd.oslot * ldo + col;  // outputs: row stride ldo (>= ncol)
-    bool dead = !ci.valid || c0 == 0.0 || (three && (c1 == 0.0 || c2 == 0.0));
+    const bool dead = !ci.valid || c0 == 0.0;
     if (!ci.valid) st = ST_NAN_INPUT;
     else if (dead) st = ST_NO_ROOT;
     if (status) status[oo] = st;
@@ -1203,72 +1279,21 @@ __device__ __noinline__ void eigen_column(int col, int ncol, int nz, int Lmax, c
     } else {
     // ---- get_1d_kernel: kernel1D (SurfaceWave.cpp:266-412) ----
     double* kout = kernel + (size_t)sd.oslot * nz * ldo + col;  // node i at kout[i * ldo]
-    if (!group) {
-      const double omega = 2.0 * PI_F / sd.t, wvno = omega / c0;
-      double ugr, norm;
-      for (int i = 0; i < nz; ++i) kp[i] = 0.0;
-      if constexpr (love) love_pass(lay, L, omega, wvno, scr, ugr, norm, sink);
-      else rayleigh_pass(lay, L, omega, wvno, scr, ugr, norm, sink);
-      double tm = 1.0;
-      if (sphere) {
-        const double x = (love ? 3.0 : 1.0) * c0 / (2. * ar * omega);
-        tm = sqrt(1. + x * x);
-      }
-      const double s1 = 1.0 / (norm * tm * tm * tm);
-      for (int i = 0; i < nz; ++i) kout[(size_t)i * ldo] = kp[i] * s1;
-      const double cs = c0 / tm;
-      vc[oo] = cs;
-      vout[oo] = cs;
-    } else {
-      // sregnpu / slegnpu (sregn96.f90:1737-1878, slegn96.f90:785-918)
-      const double twopi = 2.0 * PI_F;
-      const double cp = c0;
-      double cg = 0.0, f1 = 0.0, f2 = 0.0, dtt = 1.0, tm = 1.0, tm1 = 0.0;
-      for (int pass = 0; pass < 3; ++pass) {
-        const double tt = (pass == 0) ? sd.t : (pass == 1) ? sd.t1 : sd.t2;
-        const double cc = (pass == 0) ? c0 : (pass == 1) ? c1 : c2;
-        const double omega = twopi / tt, wvno = omega / cc;
-        double ugr, norm;
-        for (int i = 0; i < nz; ++i) kp[i] = 0.0;
-        if constexpr (love) love_pass(lay, L, omega, wvno, scr, ugr, norm, sink);
-        else rayleigh_pass(lay, L, omega, wvno, scr, ugr, norm, sink);
-        double coef;
-        if (pass == 0) {
-          cg = ugr;
-          const double uc1 = cg / cp;
-          dtt = sd.t2 - sd.t1;
-          f1 = uc1 * (2.0 - uc1);
-          f2 = uc1 * uc1 * sd.t;
-          if (sphere) {
-            const double om0 = twopi / sd.t;
-            const double k = love ? 1.5 : 0.5;
-            const double x = (love ? 3.0 : 1.0) * cp / (2. * ar * om0);
-            tm = sqrt(1. + x * x);
-            const double y = k / (ar * om0);
-            tm1 = (y * y) / tm;
-            coef = cg * cp * tm1;
-          } else {
-            coef = 0.0;
-          }
-        } else if (pass == 1) {
-          coef = tm * (f2 / dtt);
-        } else {
-          coef = tm * (f1 - f2 / dtt);
-        }
-        // the sum over the passes, from 0, in the output
-        if (coef != 0.0) {
-          const double s1 = coef / norm;
-          for (int i = 0; i < nz; ++i) {
-            const double prev = (pass == 0) ? 0.0 : kout[(size_t)i * ldo];
-            kout[(size_t)i * ldo] = prev + kp[i] * s1;
-          }
-        } else if (pass == 0) {
-          for (int i = 0; i < nz; ++i) kout[(size_t)i * ldo] = 0.0;
-        }
-      }
-      vc[oo] = cp / tm;
-      vout[oo] = cg * tm;
+    const double omega = 2.0 * PI_F / sd.t, wvno = omega / c0;
+    double ugr, norm;
+    for (int i = 0; i < nz; ++i) kp[i] = 0.0;
+    if constexpr (love) love_pass(lay, L, omega, wvno, scr, ugr, norm, sink);
+    else rayleigh_pass(lay, L, omega, wvno, scr, ugr, norm, sink);
+    double tm = 1.0;
+    if (sphere) {
+      const double x = (love ? 3.0 : 1.0) * c0 / (2. * ar * omega);
+      tm = sqrt(1. + x * x);
     }
+    const double s1 = 1.0 / (norm * tm * tm * tm);
+    for (int i = 0; i < nz; ++i) kout[(size_t)i * ldo] = kp[i] * s1;
+    const double cs = c0 / tm;
+    vc[oo] = cs;
+    vout[oo] = cs;
     // water / merged fluid nodes carry no kernel (SurfaceWave.cpp:495)
     for (int i = 0; i < ci.nw; ++i) kout[(size_t)i * ldo] = 0.0;
     }  // get_1d_kernel
@@ -1289,7 +1314,24 @@ int eigen_blocks(int wt, int path, int et, long long n, int nsm) {
 size_t eigen_store(int wt, int path, int et, int Lmax) {
   return eigen_passes(wt, path) ? (size_t)(wt >= 2 ? LOVE_STORE : RAY_STORE) * et * Lmax : 0;
 }
-int eigen_threads(int gn) { return std::min(128, ((gn + 31) / 32) * 32); }
+// Threads of a block for gn slots: a thread per slot, or three where a kernel
+// takes a group slot's three passes; then the width that leaves the fewest
+// lanes idle over the rounds (gn slots in rounds of a third of it), the widest
+// of equals.
+int eigen_threads(int wt, int path, int gn) {
+  if (path != 0 || !(wt == 1 || wt == 3)) return std::min(128, ((gn + 31) / 32) * 32);
+  int best = 32;
+  long long cost = 0;
+  for (int et = 32; et <= 128; et += 32) {
+    const int per = et / 3;
+    const long long c = (long long)((gn + per - 1) / per) * et;
+    if (et == 32 || c <= cost) {
+      best = et;
+      cost = c;
+    }
+  }
+  return best;
+}
 
 template <int WT, int PATH>
 __global__ void __launch_bounds__(128, eigen_minb(WT)) k_eigen(int ncol, int nz, int Lmax, const float4* __restrict__ lay0,
@@ -1837,7 +1879,7 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
   size_t store = 0;  // doubles of the eigen stage's up-pass stores
   if (!roots_only) {
     for (int g = 0; g < P.groups.n; ++g) {
-      const int wt = P.slots[P.groups.start[g]].wtype, et = eigen_threads(P.groups.count[g]);
+      const int wt = P.slots[P.groups.start[g]].wtype, et = eigen_threads(wt, path, P.groups.count[g]);
       store = std::max(store, eigen_blocks(wt, path, et, ncol, ctx->nsm) * eigen_store(wt, path, et, Lmax));
     }
     if (ho) store *= 2;  // its chunks run on two streams
@@ -2016,7 +2058,7 @@ int launch_eigen(swdk_ctx* ctx, const Plan& P, int path, int ncol, int nz, int c
   for (int g = 0; g < P.groups.n; ++g) {
     const int g0 = P.groups.start[g], gn = P.groups.count[g];
     const int wt = P.slots[g0].wtype;
-    const int et = eigen_threads(gn);
+    const int et = eigen_threads(wt, path, gn);
     const size_t smem = (size_t)Lmax * (wt >= 2 ? sizeof(LoveLayer) : sizeof(RayLayer)) + (size_t)nz * sizeof(float2);
     ctx->launches += 1;
     eig[wt][path]<<<eigen_blocks(wt, path, et, c1 - c0, ctx->nsm), et, smem, st>>>(ncol, nz, Lmax, ctx->lay0.as<float4>(), ctx->info.as<ColInfo>(),
@@ -2936,7 +2978,7 @@ int swdk_ragged_create(int n, swdk_ctx* const* ctxs, const swdk_call* calls, swd
       E.pad_ = 0;
       R->eb[wt].push_back(E);
       R->eblocks[wt] += M.ncol;
-      R->et[wt] = std::max(R->et[wt], eigen_threads(E.gn));
+      R->et[wt] = std::max(R->et[wt], eigen_threads(wt, R->path, E.gn));
     }
     if (proposals_on(c)) R->useprop = true;
     // the model's depth vector on the device (k_prep reads it)
