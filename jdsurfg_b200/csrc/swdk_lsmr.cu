@@ -9,15 +9,14 @@
 // with the damping rotation, the second QR factorization that minimizes
 // ||A^T r||, and the paper's estimates of ||r||, ||A^T r||, ||A||, cond(A)
 // for the stopping rules (istop as in the reference's module).  Every
-// scalar of the recurrences lives in device memory and is updated by a
-// one-thread kernel, so an iteration is a fixed sequence of launches with
-// no host round trip; the host reads the state back every LS_CHECK
-// iterations.  Once a stopping rule fires, every kernel of the iteration
+// scalar of the recurrences lives in device memory, so an iteration is a fixed
+// sequence of five launches with no host round trip; the host reads the state
+// back every LS_CHECK iterations.  Once a stopping rule fires, every kernel of the iteration
 // returns at once, so the iterations queued behind it change nothing.
 //
 // A^T y uses the transposed matrix (built by the caller, each row of it a
-// column of A with its entries in row order) and the same row kernel as
-// A x, and the norms are two-stage sums over a fixed grid: the whole solve
+// column of A with its entries in row order) and the same row product as
+// A x, and the norms are two-stage sums in a fixed order: the whole solve
 // is the same bits on every run.
 #include <cuda_runtime.h>
 
@@ -36,7 +35,7 @@ constexpr int LS_CHECK = 16;    // iterations queued between two reads of the st
 
 struct LsmrState {
   // bidiagonalization and the two QR factorizations
-  double alpha, beta, alpha_bar, zeta_bar, rho_prev, rho_bar_prev, c_bar, s_bar;
+  double alpha, beta, udiv, alpha_bar, zeta_bar, rho_prev, rho_bar_prev, c_bar, s_bar;
   // ||r|| estimate
   double beta_dd, beta_dot, rho_dot_prev, tau_tilde_prev, theta_tilde, zeta_prev, damp_sum;
   // ||A||, cond(A)
@@ -47,23 +46,18 @@ struct LsmrState {
   int itn, itnlim, istop, done;
 };
 
-// y = s*y + A x over the rows of A, one warp per row; s = -alpha (which 0),
-// -beta (1) or 1 (2: y += A x).  (s*y) and the sum are rounded separately,
-// as a scaling followed by an accumulating product would be.
+// the start's y += A x over the rows of A, one warp per row
 __global__ void k_ls_spmv(int64_t m, const int64_t* __restrict__ rowptr, const int32_t* __restrict__ idx,
                           const float* __restrict__ val, const double* __restrict__ x, double* __restrict__ y,
-                          const LsmrState* __restrict__ st, int which) {
-  if (st->done || (which == 1 && !(st->beta > 0.0))) return;
+                          const LsmrState* __restrict__ st) {
+  if (st->done) return;
   const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (r >= m) return;
   double acc = 0.0;
   for (int64_t j = rowptr[r] + lane; j < rowptr[r + 1]; j += 32) acc += (double)val[j] * x[idx[j]];
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if (lane == 0) {
-    const double s = which == 0 ? -st->alpha : which == 1 ? -st->beta : 1.0;
-    y[r] = __dadd_rn(which == 2 ? y[r] : __dmul_rn(s, y[r]), acc);
-  }
+  if (lane == 0) y[r] = __dadd_rn(y[r], acc);
 }
 
 // block sum of a fixed-order strided sum of squares: part[blockIdx.x]
@@ -125,6 +119,7 @@ __global__ void k_ls_start(LsmrState* st, double damp, double atol, double btol,
   s.damp = damp; s.atol = atol; s.btol = btol; s.ctol = ctol; s.itnlim = itnlim;
   s.itn = 0; s.istop = 0;
   s.normr = beta; s.normAr = alpha * beta; s.normA = 0.0; s.condA = 1.0; s.normx = 0.0;
+  s.udiv = 1.0;  // the start's u is normalised
   s.done = (alpha * beta == 0.0) ? 1 : 0;
   s.alpha_bar = alpha; s.zeta_bar = alpha * beta;
   s.rho_prev = 1.0; s.rho_bar_prev = 1.0; s.c_bar = 1.0; s.s_bar = 0.0;
@@ -136,9 +131,7 @@ __global__ void k_ls_start(LsmrState* st, double damp, double atol, double btol,
 }
 
 // one iteration's scalar recurrences (after alpha, beta of the step)
-__global__ void k_ls_scalar(LsmrState* st) {
-  LsmrState& s = *st;
-  if (s.done) return;
+__device__ void ls_scalar(LsmrState& s) {
   s.itn += 1;
   const double alpha = s.alpha, beta = s.beta, damp = s.damp;
   // damping rotation on (alpha_bar, damp)
@@ -191,38 +184,8 @@ __global__ void k_ls_scalar(LsmrState* st) {
   s.zeta_prev = zeta;
 }
 
-// h_bar = c_hbar h_bar + h; x += c_x h_bar; h = c_h h + v; partial sums of x^2
-__global__ void k_ls_vec(int64_t n, double* __restrict__ x, double* __restrict__ h, double* __restrict__ hbar,
-                         const double* __restrict__ v, double* __restrict__ part, const LsmrState* __restrict__ st) {
-  if (st->done) return;
-  const double ch = st->c_hbar, cx = st->c_x, chh = st->c_h;
-  double s = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double hb = __dadd_rn(__dmul_rn(hbar[i], ch), h[i]);
-    hbar[i] = hb;
-    const double xi = __dadd_rn(x[i], __dmul_rn(cx, hb));
-    x[i] = xi;
-    h[i] = __dadd_rn(__dmul_rn(h[i], chh), v[i]);
-    s += xi * xi;
-  }
-  block_sum_store(s, part);
-}
-
-// ||x|| and the stopping rules (the reference module's istop)
-__global__ void k_ls_tests(const double* __restrict__ part, LsmrState* st) {
-  if (st->done) return;
-  __shared__ double sh[512];
-  double v = 0.0;
-  for (int i = threadIdx.x; i < LS_PART; i += blockDim.x) v += part[i];
-  sh[threadIdx.x] = v;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x != 0) return;
-  LsmrState& s = *st;
-  s.normx = sqrt(sh[0]);
+// the stopping rules (the reference module's istop), after normx
+__device__ void ls_tests(LsmrState& s) {
   const double test1 = s.normr / s.normb;
   const double test2 = (s.normA * s.normr > 0.0) ? s.normAr / (s.normA * s.normr) : INFINITY;
   const double test3 = 1.0 / s.condA;
@@ -240,6 +203,130 @@ __global__ void k_ls_tests(const double* __restrict__ part, LsmrState* st) {
   s.done = istop > 0;
 }
 
+// ---------------------------------------------------------------------------
+// An iteration is five kernels: the product with A, |u|, the product with A^T,
+// |v| and the scalar recurrences, the vector updates.  The sums leave partial
+// sums in a fixed order; the block that finishes last adds them and does the
+// scalar work that waits for it.
+//
+// The products take 133 (A) and 108 us (A^T) at 20 000 rows of 3137 entries,
+// 502 MB each, 76 us at the copy rate: a warp's gather of x goes line by line,
+// and needs the 64 warps of an SM that 32 registers allow.  Measured slower:
+// eight loads of 32 entries ahead (64 registers, 217 and 122 us), a row from a
+// counter for each resident warp with the next round loaded ahead (138, 112),
+// 16-byte loads of indices and values (more lines per gather, 290), and 224 KB
+// of x in shared memory (192, 173).
+//
+// The other launches, norms, divisions and recurrences of their own, were
+// eight with 2 to 3 us each; they are three.
+// ---------------------------------------------------------------------------
+
+// y = A x - alpha y / udiv (AT false: y is u, held as udiv times the
+// normalised vector) or A^T u / beta - beta y (AT true: y is v; beta = 0
+// leaves it), one warp per row
+template <bool AT>
+__global__ void __launch_bounds__(LS_THREADS, 8)
+    k_ls_product(int64_t m, const int64_t* __restrict__ rowptr, const int32_t* __restrict__ idx,
+                 const float* __restrict__ val, const double* __restrict__ x, double* __restrict__ y,
+                 const LsmrState* __restrict__ st) {
+  if (st->done || (AT && !(st->beta > 0.0))) return;
+  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (r >= m) return;
+  double acc = 0.0;
+  for (int64_t j = rowptr[r] + lane; j < rowptr[r + 1]; j += 32) acc += (double)val[j] * x[idx[j]];
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if (lane == 0)
+    y[r] = AT ? __dadd_rn(__dmul_rn(-st->beta, y[r]), acc / st->beta)
+              : __dadd_rn(__dmul_rn(-st->alpha, y[r] / st->udiv), acc);
+}
+
+// The block's sum of squares sq (one per thread) into part; true in the block
+// that is last to do so, with the total over all blocks in *tot (thread 0).
+__device__ bool ls_last_sum(double sq, double* __restrict__ part, unsigned int* __restrict__ ctr, double* tot) {
+  __shared__ double sh[LS_THREADS];
+  __shared__ bool last;
+  sh[threadIdx.x] = sq;
+  __syncthreads();
+  for (int o = LS_THREADS / 2; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = sh[0];
+    __threadfence();
+    last = atomicAdd(ctr, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  double v = 0.0;
+  for (unsigned int i = threadIdx.x; i < gridDim.x; i += LS_THREADS) v += __ldcg(part + i);
+  sh[threadIdx.x] = v;
+  __syncthreads();
+  for (int o = LS_THREADS / 2; o > 0; o >>= 1) {
+    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    *tot = sh[0];
+    *ctr = 0u;
+  }
+  return true;
+}
+
+// AT false: beta = |u|; AT true: alpha = |v| (v keeps its length, the updates
+// divide; beta = 0 leaves alpha), then the step's recurrences
+template <bool AT>
+__global__ void __launch_bounds__(LS_THREADS) k_ls_length(int64_t n, const double* __restrict__ a,
+                                                          double* __restrict__ part, unsigned int* __restrict__ ctr,
+                                                          LsmrState* __restrict__ st) {
+  if (st->done) return;
+  double s = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * LS_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * LS_THREADS)
+    s += a[i] * a[i];
+  double tot;
+  if (ls_last_sum(s, part, ctr, &tot) && threadIdx.x == 0) {
+    if (!AT) {
+      st->beta = sqrt(tot);
+      st->udiv = st->beta > 0.0 ? st->beta : 1.0;
+    } else {
+      if (st->beta > 0.0) st->alpha = sqrt(tot);
+      ls_scalar(*st);
+    }
+  }
+}
+
+// v /= alpha; h_bar = c_hbar h_bar + h; x += c_x h_bar; h = c_h h + v; |x| and
+// the stopping rules
+__global__ void __launch_bounds__(LS_THREADS) k_ls_vec(int64_t n, double* __restrict__ x, double* __restrict__ h,
+                                                       double* __restrict__ hbar, double* __restrict__ v,
+                                                       double* __restrict__ part, unsigned int* __restrict__ ctr,
+                                                       LsmrState* __restrict__ st) {
+  if (st->done) return;
+  const double ch = st->c_hbar, cx = st->c_x, chh = st->c_h, alpha = st->alpha;
+  const bool div = st->beta > 0.0 && alpha > 0.0;
+  double s = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double vi = v[i];
+    if (div) {
+      vi = vi / alpha;
+      v[i] = vi;
+    }
+    const double hb = __dadd_rn(__dmul_rn(hbar[i], ch), h[i]);
+    hbar[i] = hb;
+    const double xi = __dadd_rn(x[i], __dmul_rn(cx, hb));
+    x[i] = xi;
+    h[i] = __dadd_rn(__dmul_rn(h[i], chh), vi);
+    s += xi * xi;
+  }
+  double tot;
+  if (ls_last_sum(s, part, ctr, &tot) && threadIdx.x == 0) {
+    st->normx = sqrt(tot);
+    ls_tests(*st);
+  }
+}
+
 }  // namespace
 
 struct swdk_lsmr {
@@ -252,6 +339,7 @@ struct swdk_lsmr {
   const int32_t* tidx = nullptr;
   const float* tval = nullptr;
   double *u = nullptr, *v = nullptr, *h = nullptr, *hbar = nullptr, *part = nullptr;
+  unsigned int* ctr = nullptr;  // blocks of the running kernel that have finished
   LsmrState* st = nullptr;
   LsmrState* hst = nullptr;  // pinned copy read back every LS_CHECK iterations
 };
@@ -274,6 +362,7 @@ void ls_free(swdk_lsmr* s) {
   for (double* p : {s->u, s->v, s->h, s->hbar, s->part})
     if (p) cudaFree(p);
   if (s->st) cudaFree(s->st);
+  if (s->ctr) cudaFree(s->ctr);
   if (s->hst) cudaFreeHost(s->hst);
 }
 
@@ -302,6 +391,7 @@ int swdk_lsmr_create(int device, int64_t m, int64_t n, const int64_t* d_rowptr, 
   if (e == cudaSuccess) e = cudaMalloc(&s->h, (size_t)n * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&s->hbar, (size_t)n * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&s->part, LS_PART * sizeof(double));
+  if (e == cudaSuccess) e = cudaMalloc(&s->ctr, sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMalloc(&s->st, sizeof(LsmrState));
   if (e == cudaSuccess) e = cudaMallocHost(&s->hst, sizeof(LsmrState));
   if (e != cudaSuccess) {
@@ -324,6 +414,7 @@ int swdk_lsmr_solve(swdk_lsmr* s, const double* d_b, double* d_x, double damp, d
   const double ctol = conlim > 0.0 ? 1.0 / conlim : 0.0;
   // start: beta u = b, alpha v = A^T u, x = 0, h = v, h_bar = 0
   cudaMemsetAsync(s->st, 0, sizeof(LsmrState), st);
+  cudaMemsetAsync(s->ctr, 0, sizeof(unsigned int), st);
   cudaMemcpyAsync(s->u, d_b, (size_t)m * sizeof(double), cudaMemcpyDeviceToDevice, st);
   cudaMemsetAsync(s->v, 0, (size_t)n * sizeof(double), st);
   cudaMemsetAsync(d_x, 0, (size_t)n * sizeof(double), st);
@@ -331,7 +422,7 @@ int swdk_lsmr_solve(swdk_lsmr* s, const double* d_b, double* d_x, double damp, d
   k_ls_partial<<<LS_PART, LS_THREADS, 0, st>>>(m, s->u, s->part, s->st, 0);
   k_ls_norm<<<1, 512, 0, st>>>(s->part, s->st, 3);
   k_ls_div<<<em, LS_THREADS, 0, st>>>(m, s->u, s->st, 0);
-  k_ls_spmv<<<gn, LS_THREADS, 0, st>>>(n, s->trowptr, s->tidx, s->tval, s->u, s->v, s->st, 2);
+  k_ls_spmv<<<gn, LS_THREADS, 0, st>>>(n, s->trowptr, s->tidx, s->tval, s->u, s->v, s->st);
   k_ls_partial<<<LS_PART, LS_THREADS, 0, st>>>(n, s->v, s->part, s->st, 1);
   k_ls_norm<<<1, 512, 0, st>>>(s->part, s->st, 1);
   k_ls_div<<<en, LS_THREADS, 0, st>>>(n, s->v, s->st, 1);
@@ -345,19 +436,11 @@ int swdk_lsmr_solve(swdk_lsmr* s, const double* d_b, double* d_x, double damp, d
         return SWDK_E_CUDA;
       if (s->hst->done || s->hst->itn >= itnlim) break;
     }
-    // beta u = A v - alpha u
-    k_ls_spmv<<<gm, LS_THREADS, 0, st>>>(m, s->rowptr, s->idx, s->val, s->v, s->u, s->st, 0);
-    k_ls_partial<<<LS_PART, LS_THREADS, 0, st>>>(m, s->u, s->part, s->st, 0);
-    k_ls_norm<<<1, 512, 0, st>>>(s->part, s->st, 0);
-    k_ls_div<<<em, LS_THREADS, 0, st>>>(m, s->u, s->st, 0);
-    // alpha v = A^T u - beta v
-    k_ls_spmv<<<gn, LS_THREADS, 0, st>>>(n, s->trowptr, s->tidx, s->tval, s->u, s->v, s->st, 1);
-    k_ls_partial<<<LS_PART, LS_THREADS, 0, st>>>(n, s->v, s->part, s->st, 1);
-    k_ls_norm<<<1, 512, 0, st>>>(s->part, s->st, 1);
-    k_ls_div<<<en, LS_THREADS, 0, st>>>(n, s->v, s->st, 1);
-    k_ls_scalar<<<1, 1, 0, st>>>(s->st);
-    k_ls_vec<<<LS_PART, LS_THREADS, 0, st>>>(n, d_x, s->h, s->hbar, s->v, s->part, s->st);
-    k_ls_tests<<<1, 512, 0, st>>>(s->part, s->st);
+    k_ls_product<false><<<gm, LS_THREADS, 0, st>>>(m, s->rowptr, s->idx, s->val, s->v, s->u, s->st);
+    k_ls_length<false><<<LS_PART, LS_THREADS, 0, st>>>(m, s->u, s->part, s->ctr, s->st);
+    k_ls_product<true><<<gn, LS_THREADS, 0, st>>>(n, s->trowptr, s->tidx, s->tval, s->u, s->v, s->st);
+    k_ls_length<true><<<LS_PART, LS_THREADS, 0, st>>>(n, s->v, s->part, s->ctr, s->st);
+    k_ls_vec<<<LS_PART, LS_THREADS, 0, st>>>(n, d_x, s->h, s->hbar, s->v, s->part, s->ctr, s->st);
     if (cudaGetLastError() != cudaSuccess) return SWDK_E_CUDA;
   }
   if (info) {
