@@ -341,10 +341,10 @@ int swdk_ragged_launch(swdk_ragged* batch, void* stream);
 int swdk_ragged_stats(swdk_ragged* batch, swdk_stats* out);
 void swdk_ragged_destroy(swdk_ragged* batch);
 
-/* Autotuner of the persistent root-search kernel: times the root search on
- * the given device model for 1..k resident blocks per SM (k = occupancy
- * limit) and one oversubscribed grid, keeps the fastest in the context and
- * returns it in *blocks (may be NULL). */
+/* Autotuner of the root search: times it on the given device model as it is by
+ * default, for 1..k resident blocks per SM of the one-lane kernel (k =
+ * occupancy limit) and one oversubscribed grid, keeps the fastest in the
+ * context and returns its one-lane blocks in *blocks (may be NULL). */
 int swdk_autotune(swdk_ctx* ctx, int nx, int ny, int nz, const float* d_vs, const float* d_vp, const float* d_rho,
                   int* blocks);
 

@@ -56,3 +56,24 @@ def test_group_search_reference_refinement(waves):
     c1, s1 = _roots(case, False, block_roots=592, refine="reference")
     cg, sg = _roots(case, False, refine="reference")
     assert np.array_equal(s1, sg) and np.array_equal(c1, cg)
+
+
+# layered models: 32 lanes per model up to 18 000 of them, 4 up to 26 000, then one
+@pytest.mark.parametrize("iwave,mode,igr,nlayer", [(2, 1, 0, 5), (1, 2, 0, 4), (2, 2, 1, 7)])
+def test_layered_models_are_the_same_in_any_batch(iwave, mode, igr, nlayer):
+    from jdsurfg_b200 import Engine
+    n = 26001
+    rng = np.random.default_rng(nlayer)
+    vs = (np.linspace(2.4, 4.6, nlayer) * (1.0 + 0.05 * rng.standard_normal((n, nlayer)))).astype(np.float32)
+    vs[::7, 0] = 0.0  # a fluid layer on top
+    vp = np.where(vs > 0, 1.76 * vs, 1.5).astype(np.float32)
+    rho = np.where(vs > 0, 0.32 * vp + 0.77, 1.03).astype(np.float32)
+    thk = np.full((n, nlayer), 3.0, np.float32)
+    thk[:, -1] = 0.0
+    t = np.array([3.0, 8.0, 20.0])
+    eng = Engine()
+    cg, ierr = eng.surfdisp96_batch(thk, vp, vs, rho, 1, iwave, mode, igr, t)
+    for a, b in ((0, 1), (1, 130), (130, 18130), (0, 18001)):
+        c, e = eng.surfdisp96_batch(thk[a:b], vp[a:b], vs[a:b], rho[a:b], 1, iwave, mode, igr, t)
+        assert np.array_equal(e, ierr[a:b]) and np.array_equal(c, cg[a:b])
+    eng.close()
