@@ -421,8 +421,8 @@ def run_lsmr(args, torch, dev, rank, world, pg):
                 "gpu_launches": None,
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                              "traffic": None, "bytes_per_iteration": per_it,
-                             "note": "per iteration two SpMV over the 165 M nonzeros, four fixed-grid norm "
-                                     "reductions and the one-thread recurrences; the host reads the state every "
+                             "note": "per iteration two SpMV over the 165 M nonzeros, two norms with the scalar "
+                                     "recurrences and the vector updates; the host reads the state every "
                                      "16 iterations"},
                 "cpu_baseline": cb, "istop": info["istop"], "itn": info["itn"]}
         print(json.dumps(line), flush=True)
