@@ -295,7 +295,11 @@ int swdk_recip_device(const double* d_x, double* d_r, int n, void* stream);
  * networks), then records it on the context's stream; the graph keeps the
  * given device pointers, so a replay recomputes from their current
  * contents.  swdk_set_periods/set_depth/set_proposal and swdk_autotune drop
- * the graph.  Replays update no statistics. */
+ * the graph.  Every other call leaves it usable, host-memory calls and calls
+ * on larger grids included: a scratch buffer that such a call outgrows stays
+ * allocated for the graph until the graph is dropped or the context
+ * destroyed (the same holds for swdk_batch_graph_create).  Replays update no
+ * statistics. */
 int swdk_graph_capture(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_vs, const float* d_vp,
                        const float* d_rho, double* d_vc, double* d_vout, double* d_kernel, int32_t* d_status);
 int swdk_graph_launch(swdk_ctx* ctx, void* stream);

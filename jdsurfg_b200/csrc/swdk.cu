@@ -22,8 +22,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
-#include <mutex>
 #include <cstring>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -1516,6 +1517,14 @@ struct DevBuf {
   template <class T> T* as() const { return (T*)p; }
 };
 
+// What a captured graph holds beside its kernels: buffers whose address it
+// has and that a later, larger call outgrew.  They stay until the graph goes.
+// (A batch graph's contexts may be used from different threads.)
+struct GraphHold {
+  std::mutex mu;
+  std::vector<std::shared_ptr<void>> kept;
+};
+
 struct Plan {
   std::vector<int> order;  // chains queued Rayleigh first
   DevBuf d_order;
@@ -1559,7 +1568,7 @@ struct swdk_ctx {
   bool dirty = true;
   Plan plan[2];  // 0: get_1d_kernel, 1: get_2d_map
   DevBuf layR, layL, lay0, info, chainrule, croot, cstat, nevals, depth_d, ierr, queue;
-  DevBuf store;         // up-pass values of the eigen stage's resident threads
+  DevBuf store, store2;  // up-pass values of the eigen stage's resident threads; the host calls' second stream's
   DevBuf nodes, dltab;  // grid nodes and the depth grid's flattening (node-source root search)
   int roots_blocks = 0, nsm = 148;
   bool coop_ready = false;  // the layered-model call's kernels are opted in to their shared memory
@@ -1591,6 +1600,8 @@ struct swdk_ctx {
   bool capturing = false;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
+  std::shared_ptr<GraphHold> hold;                // of this context's graph
+  std::vector<std::weak_ptr<GraphHold>> holders;  // of every graph that has this context's buffers
   int launches = 0;  // kernels launched by the current call
   // stage marks: 0 start, 1 prep, 5 proposals, 2 roots, 3 eigen, 4 call done
   cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -1612,6 +1623,28 @@ int fail(swdk_ctx* c, int code, const std::string& msg) {
     cudaError_t e_ = (call);                                                                  \
     if (e_ != cudaSuccess) return fail(ctx, SWDK_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
+
+// A buffer that a captured call uses, grown to `bytes`: while a graph has its
+// address the outgrown buffer goes to that graph instead of being freed.
+cudaError_t ensure(swdk_ctx* ctx, DevBuf& b, size_t bytes) {
+  if (bytes > b.n && b.p && !ctx->holders.empty()) {
+    std::shared_ptr<void> old(b.p, [](void* p) { cudaFree(p); });
+    b.p = nullptr;
+    b.n = 0;
+    for (const std::weak_ptr<GraphHold>& w : ctx->holders)
+      if (const std::shared_ptr<GraphHold> h = w.lock()) {
+        std::lock_guard<std::mutex> lk(h->mu);
+        h->kept.push_back(old);
+      }
+  }
+  return b.ensure(bytes);
+}
+
+void add_holder(swdk_ctx* ctx, const std::shared_ptr<GraphHold>& h) {
+  std::vector<std::weak_ptr<GraphHold>>& v = ctx->holders;
+  v.erase(std::remove_if(v.begin(), v.end(), [](const std::weak_ptr<GraphHold>& w) { return w.expired(); }), v.end());
+  v.push_back(h);
+}
 
 int find_chain(Plan& P, std::vector<std::vector<double>>& lists, int iwave, const std::vector<double>& lst, int nmode) {
   for (size_t i = 0; i < P.chains.size(); ++i) {
@@ -1722,12 +1755,12 @@ int build_plan(swdk_ctx* ctx, int path) {
   for (int w = 2; w >= 1; --w)
     for (size_t i = 0; i < P.chains.size(); ++i)
       if (P.chains[i].iwave == w) P.order.push_back((int)i);
-  CK(P.d_order.ensure(P.order.size() * sizeof(int)));
+  CK(ensure(ctx, P.d_order, P.order.size() * sizeof(int)));
   CK(cudaMemcpy(P.d_order.p, P.order.data(), P.order.size() * sizeof(int), cudaMemcpyHostToDevice));
-  CK(P.d_chains.ensure(P.chains.size() * sizeof(ChainDesc)));
-  CK(P.d_periods.ensure(P.periods.size() * sizeof(double)));
-  CK(P.d_slots.ensure(P.slots.size() * sizeof(SlotDesc)));
-  CK(P.d_rootfeat.ensure(P.rootfeat.size() * sizeof(float4)));
+  CK(ensure(ctx, P.d_chains, P.chains.size() * sizeof(ChainDesc)));
+  CK(ensure(ctx, P.d_periods, P.periods.size() * sizeof(double)));
+  CK(ensure(ctx, P.d_slots, P.slots.size() * sizeof(SlotDesc)));
+  CK(ensure(ctx, P.d_rootfeat, P.rootfeat.size() * sizeof(float4)));
   CK(cudaMemcpy(P.d_rootfeat.p, P.rootfeat.data(), P.rootfeat.size() * sizeof(float4), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(P.d_chains.p, P.chains.data(), P.chains.size() * sizeof(ChainDesc), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(P.d_periods.p, P.periods.data(), P.periods.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -1757,11 +1790,11 @@ int run_proposals(swdk_ctx* ctx, const Plan& P, int ncol, cudaStream_t st, const
                   float2* prop = nullptr) {
   const int64_t nrows = (int64_t)P.nroot * ncol;
   if (!prop) {
-    CK(ctx->prop.ensure((size_t)nrows * sizeof(float2)));
+    CK(ensure(ctx, ctx->prop, (size_t)nrows * sizeof(float2)));
     prop = ctx->prop.as<float2>();
   }
   if (!nodefeat) nodefeat = ctx->nodefeat.as<float4>();
-  CK(ctx->pfeat.ensure((size_t)PROP_CHUNK * FEAT_DIM * sizeof(__nv_bfloat16)));
+  CK(ensure(ctx, ctx->pfeat, (size_t)PROP_CHUNK * FEAT_DIM * sizeof(__nv_bfloat16)));
   const int64_t bound[3] = {0, (int64_t)P.nrootR * ncol, nrows};
   for (int w = 0; w < 2; ++w) {
     const int64_t r0 = bound[w], r1 = bound[w + 1];
@@ -1824,17 +1857,17 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
   const int Lmax = 4 * nz - 3;
   const bool useprop = proposals_on(ctx);
   const bool wantfeat = useprop || roots_only;
-  CK(ctx->layR.ensure((size_t)Lmax * ncol * sizeof(float4)));
-  CK(ctx->layL.ensure((size_t)Lmax * ncol * sizeof(float4)));
-  CK(ctx->queue.ensure(sizeof(unsigned int)));
-  CK(ctx->lay0.ensure((size_t)Lmax * ncol * sizeof(float4)));
-  CK(ctx->info.ensure((size_t)ncol * sizeof(ColInfo)));
-  CK(ctx->chainrule.ensure((size_t)nz * ncol * sizeof(float2)));
-  CK(ctx->croot.ensure((size_t)P.nroot * ncol * sizeof(double)));
-  CK(ctx->cstat.ensure((size_t)P.nroot * ncol * sizeof(int32_t)));
-  CK(ctx->nevals.ensure(NCOUNT * sizeof(unsigned long long)));
-  if (wantfeat) CK(ctx->nodefeat.ensure((size_t)ncol * FEAT_NODES * sizeof(float4)));
-  CK(ctx->depth_d.ensure((size_t)nz * sizeof(float)));
+  CK(ensure(ctx, ctx->layR, (size_t)Lmax * ncol * sizeof(float4)));
+  CK(ensure(ctx, ctx->layL, (size_t)Lmax * ncol * sizeof(float4)));
+  CK(ensure(ctx, ctx->queue, sizeof(unsigned int)));
+  CK(ensure(ctx, ctx->lay0, (size_t)Lmax * ncol * sizeof(float4)));
+  CK(ensure(ctx, ctx->info, (size_t)ncol * sizeof(ColInfo)));
+  CK(ensure(ctx, ctx->chainrule, (size_t)nz * ncol * sizeof(float2)));
+  CK(ensure(ctx, ctx->croot, (size_t)P.nroot * ncol * sizeof(double)));
+  CK(ensure(ctx, ctx->cstat, (size_t)P.nroot * ncol * sizeof(int32_t)));
+  CK(ensure(ctx, ctx->nevals, NCOUNT * sizeof(unsigned long long)));
+  if (wantfeat) CK(ensure(ctx, ctx->nodefeat, (size_t)ncol * FEAT_NODES * sizeof(float4)));
+  CK(ensure(ctx, ctx->depth_d, (size_t)nz * sizeof(float)));
   if (ctx->depth_dev != ctx->depth_d.p) {  // first call after swdk_set_depth (never inside a capture)
     if (ctx->capturing) return fail(ctx, SWDK_E_ARG, "depth not on the device before graph capture");
     CK(cudaMemcpyAsync(ctx->depth_d.p, ctx->depth.data(), nz * sizeof(float), cudaMemcpyHostToDevice, st));
@@ -1842,8 +1875,8 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
   }
   const bool use_nodes = ctx->cfg.node_layers != 0;
   if (use_nodes) {
-    CK(ctx->nodes.ensure((size_t)nz * ncol * sizeof(float4)));
-    CK(ctx->dltab.ensure((size_t)Lmax * sizeof(DepthLayer)));
+    CK(ensure(ctx, ctx->nodes, (size_t)nz * ncol * sizeof(float4)));
+    CK(ensure(ctx, ctx->dltab, (size_t)Lmax * sizeof(DepthLayer)));
   }
   CK(cudaMemsetAsync(ctx->nevals.p, 0, NCOUNT * sizeof(unsigned long long), st));
   const bool timing = !ctx->capturing;  // stage events and statistics only on eager calls
@@ -1877,19 +1910,24 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
     ctx->roots_blocks = std::max(1, nsm * std::max(1, per));
   }
   size_t store = 0;  // doubles of the eigen stage's up-pass stores
+  int nch = 1;       // column chunks of a host-memory call, on two streams in turn
   if (!roots_only) {
     for (int g = 0; g < P.groups.n; ++g) {
       const int wt = P.slots[P.groups.start[g]].wtype, et = eigen_threads(wt, path, P.groups.count[g]);
       store = std::max(store, eigen_blocks(wt, path, et, ncol, ctx->nsm) * eigen_store(wt, path, et, Lmax));
     }
-    if (ho) store *= 2;  // its chunks run on two streams
-    CK(ctx->store.ensure(store * sizeof(double)));
+    CK(ensure(ctx, ctx->store, store * sizeof(double)));
+    if (ho) {
+      const size_t bytes = (size_t)ncol * P.kmax * (20 + (path == 0 ? 8 * (size_t)nz : 0));
+      nch = (int)std::min<size_t>(HOST_CHUNKS, std::max<size_t>(1, bytes / HOST_CHUNK_BYTES));
+      if (nch > 1) CK(ctx->store2.ensure(store * sizeof(double)));
+    }
   }
   const int nitems = (int)P.chains.size() * ncol;
   const int rblocks = ctx->cfg.block_roots > 0 ? ctx->cfg.block_roots : ctx->roots_blocks;
   const unsigned int rcap = (unsigned int)std::min<size_t>((size_t)P.nroot * ncol, 0x7fffffffu);
-  CK(ctx->retry_list.ensure((size_t)rcap * sizeof(int2)));
-  CK(ctx->retry_ctr.ensure(2 * sizeof(unsigned int)));
+  CK(ensure(ctx, ctx->retry_list, (size_t)rcap * sizeof(int2)));
+  CK(ensure(ctx, ctx->retry_ctr, 2 * sizeof(unsigned int)));
   CK(cudaMemsetAsync(ctx->queue.p, 0, sizeof(unsigned int), st));
   CK(cudaMemsetAsync(ctx->retry_ctr.p, 0, 2 * sizeof(unsigned int), st));
   unsigned int* rctr = ctx->retry_ctr.as<unsigned int>();
@@ -1939,8 +1977,6 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
       }
       if (!ctx->evefork) CK(cudaEventCreateWithFlags(&ctx->evefork, cudaEventDisableTiming));
       const int kmax = P.kmax;
-      const size_t bytes = (size_t)ncol * kmax * (20 + (path == 0 ? 8 * (size_t)nz : 0));
-      const int nch = (int)std::min<size_t>(HOST_CHUNKS, std::max<size_t>(1, bytes / HOST_CHUNK_BYTES));
       auto chunk = [&](int h, int& a, int& b) {
         a = (int)((long long)ncol * h / nch);
         b = (int)((long long)ncol * (h + 1) / nch);
@@ -1958,7 +1994,7 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
         if (b <= a) continue;
         cudaStream_t es = ctx->estream[h & 1];
         r = launch_eigen(ctx, P, path, ncol, nz, a, b, d_vc, d_vout, d_kernel, d_status, ldo,
-                         ctx->store.as<double>() + (h & 1) * (store / 2), es);
+                         (h & 1 ? ctx->store2 : ctx->store).as<double>(), es);
         if (r) return r;
         CK(cudaEventRecord(ctx->evchunk[h], es));
       }
@@ -2075,6 +2111,7 @@ void drop_graph(swdk_ctx* ctx) {
   if (ctx->graph) cudaGraphDestroy(ctx->graph);
   ctx->gexec = nullptr;
   ctx->graph = nullptr;
+  ctx->hold.reset();
 }
 
 void drop_kids(swdk_ctx* ctx) {
@@ -2284,7 +2321,7 @@ void swdk_destroy(swdk_ctx* ctx) {
   if (!ctx) return;
   cudaSetDevice(ctx->cfg.device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  DevBuf* bufs[] = {&ctx->layR, &ctx->layL, &ctx->lay0, &ctx->info, &ctx->chainrule, &ctx->store, &ctx->croot, &ctx->cstat,
+  DevBuf* bufs[] = {&ctx->layR, &ctx->layL, &ctx->lay0, &ctx->info, &ctx->chainrule, &ctx->store, &ctx->store2, &ctx->croot, &ctx->cstat,
                     &ctx->nodes, &ctx->dltab,
                     &ctx->nevals, &ctx->depth_d, &ctx->ierr, &ctx->in_vs, &ctx->in_vp, &ctx->in_rho,
                     &ctx->out_vc, &ctx->out_vout, &ctx->out_kernel, &ctx->out_status, &ctx->in_misc,
@@ -2410,13 +2447,13 @@ int swdk_surfdisp96_batch(swdk_ctx* ctx, int nmodel, int nlayer, const float* th
   ChainDesc cd;
   cd.t_off = 0; cd.np = kmax; cd.nmode = mode; cd.iwave = iwave; cd.igr = igr; cd.out_off = 0;
   CK(cudaMemcpyAsync(d_ch, &cd, sizeof(cd), cudaMemcpyHostToDevice, st));
-  CK(ctx->layR.ensure(nin * sizeof(float4)));
-  CK(ctx->layL.ensure(nin * sizeof(float4)));
-  CK(ctx->info.ensure(nm * sizeof(ColInfo)));
-  CK(ctx->croot.ensure((size_t)mode * kmax * nm * sizeof(double)));
-  CK(ctx->cstat.ensure((size_t)mode * kmax * nm * sizeof(int32_t)));
+  CK(ensure(ctx, ctx->layR, nin * sizeof(float4)));
+  CK(ensure(ctx, ctx->layL, nin * sizeof(float4)));
+  CK(ensure(ctx, ctx->info, nm * sizeof(ColInfo)));
+  CK(ensure(ctx, ctx->croot, (size_t)mode * kmax * nm * sizeof(double)));
+  CK(ensure(ctx, ctx->cstat, (size_t)mode * kmax * nm * sizeof(int32_t)));
   CK(ctx->ierr.ensure(nm * sizeof(int32_t)));
-  CK(ctx->nevals.ensure(NCOUNT * sizeof(unsigned long long)));
+  CK(ensure(ctx, ctx->nevals, NCOUNT * sizeof(unsigned long long)));
   CK(cudaMemsetAsync(ctx->nevals.p, 0, NCOUNT * sizeof(unsigned long long), st));
   CK(cudaEventRecord(ctx->ev[0], st));
   k_prep_layers<<<(nmodel + 127) / 128, 128, 0, st>>>(nmodel, nlayer, d_in, d_in + nin, d_in + 2 * nin,
@@ -2435,7 +2472,7 @@ int swdk_surfdisp96_batch(swdk_ctx* ctx, int nmodel, int nlayer, const float* th
     ctx->coop_ready = true;
   }
   if (const int G = coop_lanes(nmodel, ctx->nsm, true); G > 1) {
-    CK(ctx->queue.ensure(sizeof(unsigned int)));
+    CK(ensure(ctx, ctx->queue, sizeof(unsigned int)));
     CK(cudaMemsetAsync(ctx->queue.p, 0, sizeof(unsigned int), st));
     const long long need = ((long long)nmodel * G + 127) / 128;
     const CoopArgs A{nmodel, nmodel, G, nullptr, d_ch, d_t, ctx->layR.as<float4>(), ctx->layL.as<float4>(),
@@ -2615,6 +2652,10 @@ int swdk_graph_capture(swdk_ctx* ctx, int path, int nx, int ny, int nz, const fl
   if (e != cudaSuccess) return fail(ctx, SWDK_E_CUDA, std::string("cudaStreamEndCapture: ") + cudaGetErrorString(e));
   ctx->graph = g;
   CK(cudaGraphInstantiate(&ctx->gexec, g, 0));
+  ctx->hold = std::make_shared<GraphHold>();
+  add_holder(ctx, ctx->hold);
+  for (swdk_ctx* k : ctx->kids)
+    if (k) add_holder(k, ctx->hold);
   return SWDK_OK;
 }
 
@@ -2624,6 +2665,7 @@ struct swdk_graph {
   std::vector<cudaEvent_t> events;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+  std::shared_ptr<GraphHold> hold = std::make_shared<GraphHold>();
 };
 
 void swdk_batch_graph_destroy(swdk_graph* g) {
@@ -2699,6 +2741,7 @@ int swdk_batch_graph_create(int n, swdk_ctx* const* ctxs, const swdk_call* calls
   if (e2 != cudaSuccess) return bail(ctx, SWDK_E_CUDA, std::string("cudaStreamEndCapture: ") + cudaGetErrorString(e2));
   e = cudaGraphInstantiate(&g->exec, graph, 0);
   if (e != cudaSuccess) return bail(ctx, SWDK_E_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
+  for (int i = 0; i < n; ++i) add_holder(ctxs[i], g->hold);
   *out = g;
   return SWDK_OK;
 }
@@ -2982,7 +3025,7 @@ int swdk_ragged_create(int n, swdk_ctx* const* ctxs, const swdk_call* calls, swd
     }
     if (proposals_on(c)) R->useprop = true;
     // the model's depth vector on the device (k_prep reads it)
-    CK(c->depth_d.ensure((size_t)k.nz * sizeof(float)));
+    CK(ensure(c, c->depth_d, (size_t)k.nz * sizeof(float)));
     if (c->depth_dev != c->depth_d.p) {
       CK(cudaMemcpy(c->depth_d.p, c->depth.data(), k.nz * sizeof(float), cudaMemcpyHostToDevice));
       c->depth_dev = c->depth_d.p;
