@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(128) k_fmst_travel(Grid G, int npair, int lane
 }
 
 // The same with two pairs per warp (March::march_half), one warp per block;
-// the pairs go round the resident warps.
-template <bool SMEM>
+// the pairs go round the resident warps.  HEAP as march_pair's.
+template <int HEAP>
 __global__ void __launch_bounds__(32) k_fmst_travel_half(Grid G, int npair, const int32_t* __restrict__ cp,
                                                          const float* __restrict__ srcx,
                                                          const float* __restrict__ srcz,
@@ -124,12 +124,12 @@ __global__ void __launch_bounds__(32) k_fmst_travel_half(Grid G, int npair, cons
         const bool mine = p0 + half < npair;
         const int p = mine ? p0 + half : p0;
         const unsigned mask = mine ? 0xffffu << (16 * half) : 0u;
-        if (SMEM)
+        if (HEAP == 1)
             march_pair<1>(G, p, cp[p], srcx, srcz, pslot, slwn, risti_c, risti_r, S, n_overflow,
                           sheap + (size_t)half * ((smem_cap + 2) & ~1), smem_cap, 2, threadIdx.x & 15, mask);
         else
-            march_pair<0>(G, p, cp[p], srcx, srcz, pslot, slwn, risti_c, risti_r, S, n_overflow, nullptr, 0, 2,
-                          threadIdx.x & 15, mask);
+            march_pair<HEAP>(G, p, cp[p], srcx, srcz, pslot, slwn, risti_c, risti_r, S, n_overflow, nullptr, 0, 2,
+                             threadIdx.x & 15, mask);
         __syncwarp();
     }
 }
@@ -242,7 +242,7 @@ extern "C" int swdk_fmst_create(swdk_fmst** out, int device, const swdk_fmst_gri
     if (e != cudaSuccess) { delete f; return SWDK_E_CUDA; }
     cudaDeviceGetAttribute(&f->nsm, cudaDevAttrMultiProcessorCount, device);
     cudaFuncSetAttribute(k_fmst_travel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_fmst_travel_half<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(k_fmst_travel_half<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     // fmst_init (fmst.f90:27-64) and the r*sin(colatitude) tables
     f->G = make_grid(grid->nx, grid->ny, grid->goxd, grid->gozd, grid->dvxd, grid->dvzd);
     make_risti(f->G, f->risti_c, f->risti_r);
@@ -525,7 +525,8 @@ extern "C" int swdk_fmst_pairs(swdk_fmst* f, int npairs, const int32_t* slot, co
                                                           f->d_risti_c, f->d_risti_r, S, f->d_overflow,
                                                           smem ? (int)cap : 0);
                 } else {
-                    const auto k = smem ? k_fmst_travel_half<true> : k_fmst_travel_half<false>;
+                    const auto k = smem ? k_fmst_travel_half<1>
+                                        : cap >= 65536 ? k_fmst_travel_half<2> : k_fmst_travel_half<0>;
                     cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
                     k<<<warps, 32, shm, st>>>(G, np, dcp, d_srcx, d_srcz, d_pslot, slwn, f->d_risti_c, f->d_risti_r, S,
                                               f->d_overflow, smem ? (int)cap : 0);

@@ -26,6 +26,11 @@ inline float __double2float_rn(double x) { return (float)x; }
 inline float __int_as_float(int i) { float x; std::memcpy(&x, &i, 4); return x; }
 struct float4 { float x, y, z, w; };
 #endif
+// The march by half a warp: device code, and host code for a test that
+// defines FM_HOST_WARP and the warp functions for lanes that run in lockstep.
+#if defined(__CUDA_ARCH__) || defined(FM_HOST_WARP)
+#define FM_WARP 1
+#endif
 
 #ifndef SWDK_FMST_SOURCE_OUTSIDE
 #define SWDK_FMST_SOURCE_OUTSIDE 1
@@ -433,7 +438,7 @@ struct March {
         }
     }
 
-#if defined(__CUDA_ARCH__)
+#if defined(FM_WARP)
     // -- the march by half a warp -------------------------------------------
     // Two pairs per warp, 16 lanes each; the lanes of a half hold the same
     // March, and the halves go through the same instructions (`on`: this half
@@ -455,36 +460,49 @@ struct March {
     //     loads its whole path to the root;
     //   * the neighbours' heap positions are loaded together, before the trial
     //     times, and again only after an update that moved other entries.
-    static __device__ __forceinline__ unsigned half_ballot(bool p, int sh) {
+    static FM_HD FM_INLINE unsigned half_ballot(bool p, int sh) {
         return (__ballot_sync(0xffffffffu, p) >> sh) & 0xffffu;
     }
 
     // the entry (key, pk) of node n from free slot tpc up to its place
     // (addtree's and updtree's loop): lane j holds the ancestor tpc >> (j + 1)
-    // and writes slot tpc >> j.  Returns whether other entries moved.
-    __device__ __forceinline__ bool sift_up_half(bool on, int tpc, int pk, int n, float key, int l, int sh) {
-        const int slot = tpc >> l, anc = slot >> 1;
-        FHeap h{0.0f, 0};
-        bool below = false;
-        if (on && anc >= 1) {
-            h = heap[anc];
-            below = key < h.key;
-        }
-        const unsigned up = half_ballot(below, sh);
-        const int moves = __ffs(~up) - 1;  // ancestors from the bottom with key < theirs
-        if (on && l <= moves) {
-            const bool self = l == moves;
-            heap[slot] = self ? FHeap{key, pk} : h;
-            FNode* d = &nd[self ? n : lin(h.node)];
-            d->s = slot;
-            if (self) d->t = key;
+    // and writes slot tpc >> j.  A heap of 65 536 entries or more (DEEP) has
+    // further ancestors, which the next round takes when all 16 moved; the
+    // test for it in every sift costs 6 % of a march (3040 pairs 182.7 ms
+    // without, 194.7 with), so the smaller heaps' code is without it.  Returns
+    // whether other entries moved.
+    template <bool DEEP>
+    FM_HD FM_INLINE bool sift_up_half(bool on, int tpc, int pk, int n, float key, int l, int sh) {
+        bool moved = false;
+        for (;;) {
+            const int slot = tpc >> l, anc = slot >> 1;
+            FHeap h{0.0f, 0};
+            bool below = false;
+            if (on && anc >= 1) {
+                h = heap[anc];
+                below = key < h.key;
+            }
+            const unsigned up = half_ballot(below, sh);
+            const int moves = __ffs(~up) - 1;  // ancestors from the bottom with key < theirs
+            if (on && l <= moves) {
+                const bool self = l == moves;
+                heap[slot] = self ? FHeap{key, pk} : h;
+                FNode* d = &nd[self ? n : lin(h.node)];
+                d->s = slot;
+                if (self) d->t = key;
+            }
+            moved |= on && moves > 0;
+            if (!DEEP) break;
+            on = on && moves == 16;
+            tpc >>= 16;
+            if (!__any_sync(0xffffffffu, on)) break;
         }
         __syncwarp();
-        return on && moves > 0;
+        return moved;
     }
 
     // a node that joins the heap (addtree); false when the heap is full
-    __device__ __forceinline__ bool grow_half(bool on, int n, float key, int l) {
+    FM_HD FM_INLINE bool grow_half(bool on, int n, float key, int l) {
         if (on && ntr >= cap) {
             overflow = true;
             if (l == 0) nd[n].t = key;
@@ -504,7 +522,7 @@ struct March {
     // if all its ancestors move and lead to it (amask: their bits; rmask: the
     // ones that lead right); it writes the child that moves into its node, or
     // the last entry where the path ends.
-    __device__ __forceinline__ void down_half(bool on, int l, int sh, int lv, unsigned amask, unsigned rmask) {
+    FM_HD FM_INLINE void down_half(bool on, int l, int sh, int lv, unsigned amask, unsigned rmask) {
         bool go = on && ntr > 1;
         const FHeap last = go ? heap[ntr] : FHeap{0.0f, 0};
         if (on) ntr = ntr - 1;
@@ -540,7 +558,7 @@ struct March {
     // that are selected here; factors of 1, 2 and the division by 1 are
     // exact, so every case keeps the reference's bits (root2, root1 above).
     // NaN when the quadrant gives none (fminf then takes the other operand).
-    __device__ __forceinline__ float quadrant(int xo, int zo, float tj, float tj2, float tk, float tk2, float slown,
+    FM_HD FM_INLINE float quadrant(int xo, int zo, float tj, float tj2, float tk, float tk2, float slown,
                                               float risti) const {
         const float ri = EARTH;
         const float U = ri * dnx, Z = risti * dnz;
@@ -571,7 +589,8 @@ struct March {
     }
 
     // run: this half has a pair to march
-    __device__ void march_half(bool run, bool refined, const PairGeo& g, int l, int sh) {
+    template <bool DEEP>
+    FM_HD void march_half(bool run, bool refined, const PairGeo& g, int l, int sh) {
         const unsigned FULL = 0xffffffffu;
         const int q = l >> 2, qa = l & 1, qb = (l >> 1) & 1;
         const int dz = q == 2 ? -1 : (q == 3 ? 1 : 0), dx = q == 0 ? -1 : (q == 1 ? 1 : 0);
@@ -678,7 +697,7 @@ struct March {
                 if (ci && stale) tpc = nd[n].s;
                 const bool added = grow_half(fi, n, ti, l);
                 if (added) tpc = ntr;
-                stale |= sift_up_half(ci || added, tpc, pn, n, ti, l, sh);
+                stale |= sift_up_half<DEEP>(ci || added, tpc, pn, n, ti, l, sh);
             }
             prev = pk;
             prev_t = tacc;
@@ -774,7 +793,8 @@ struct Scratch {  // device arrays of one chunk of pairs
 // HEAP: where the pair's heap lies: 0 at hp if given, else in S (either
 // address space); 1 at hp, in shared memory (a device caller that says so gets
 // shared-memory accesses; generic ones return in order behind outstanding
-// global loads, which cost the march 2000 cycles per accepted node).
+// global loads, which cost the march 2000 cycles per accepted node); 2 as 0,
+// for heaps of 65 536 entries or more.
 template <int HEAP = 0>
 FM_HD void march_pair(const Grid& G, int p, int gp, const float* __restrict__ srcx,
                            const float* __restrict__ srcz, const int32_t* __restrict__ pslot,
@@ -793,17 +813,17 @@ FM_HD void march_pair(const Grid& G, int p, int gp, const float* __restrict__ sr
     const bool lead = go && (mode != 2 || lane == 0);
     const int l0 = mode == 2 ? lane : 0, lstep = mode == 2 ? 16 : 1;  // this lane's share of a loop over nodes
     auto group_sync = [&]() {
-#if defined(__CUDA_ARCH__)
+#if defined(FM_WARP)
         if (mode == 2) __syncwarp();
 #endif
     };
     // (iz, ix) joins the heap with time t (on: this half adds one)
     auto add = [&](March& M, bool on, int iz, int ix, float t) {
-#if defined(__CUDA_ARCH__)
+#if defined(FM_WARP)
         if (mode == 2) {
             const int n = M.idx(iz, ix);
             const bool added = M.grow_half(on, n, t, lane);
-            M.sift_up_half(added, M.ntr, March::pack(iz, ix), n, t, lane, threadIdx.x & 16);
+            M.template sift_up_half<HEAP == 2>(added, M.ntr, March::pack(iz, ix), n, t, lane, threadIdx.x & 16);
             return;
         }
 #endif
@@ -811,8 +831,8 @@ FM_HD void march_pair(const Grid& G, int p, int gp, const float* __restrict__ sr
     };
     auto run = [&](March& M, bool refined) {
         if (mode == 1) M.march_nb(refined, g);
-#if defined(__CUDA_ARCH__)
-        else if (mode == 2) M.march_half(go, refined, g, lane, threadIdx.x & 16);
+#if defined(FM_WARP)
+        else if (mode == 2) M.template march_half<HEAP == 2>(go, refined, g, lane, threadIdx.x & 16);
 #endif
         else M.march(refined, g);
     };
@@ -912,7 +932,7 @@ FM_HD void march_pair(const Grid& G, int p, int gp, const float* __restrict__ sr
             const int i = g.vnl + di, j = g.vnt + dj;
             FNode c{0.0f, 0};
             if (go && i <= g.vnr && j <= g.vnb) c = C.nd[C.idx(j, i)];
-#if defined(__CUDA_ARCH__)
+#if defined(FM_WARP)
             if (mode == 2 && !__any_sync(0xffffffffu, c.s > 0)) continue;
 #endif
             add(C, c.s > 0, j, i, c.t);
