@@ -444,14 +444,16 @@ void swdk_fmst_destroy(swdk_fmst* fmst);
 const char* swdk_fmst_last_error(const swdk_fmst* fmst);
 
 /* Scratch budget for the per-pair marching grids (bytes; 0 keeps the
- * current, 16 GiB by default), marching lanes per warp with one lane per pair
- * (1..32, a multiple of lanes_per_pair; default 8), resident marching warps per SM (0..64, default
- * 12; 0 = one warp per group of pairs, all at once), heap entries per pair
- * kept in shared memory (-1 = automatic, the default: 1.5 (nnx + nnz); 0 =
- * heap in global memory; a pair whose band outgrows it is marched again with
- * the full heap) and lanes per pair (1: one lane marches a pair; 4, the
- * default, or 8: half a warp does, the lanes solving the neighbours of the
- * accepted node together, two pairs per warp).  None of them changes a
+ * current, 16 GiB by default), marching lanes per warp (1..32, a multiple of
+ * lanes_per_pair; default 8; with one lane per pair, the pairs of a warp),
+ * resident marching warps per SM (0..64, default 12; 0 = one warp per group of
+ * pairs, all at once), heap entries per pair kept in shared memory (-1 =
+ * automatic, the default: 1.5 (nnx + nnz); 0 = heap in global memory; a pair
+ * whose band outgrows it is marched again with the full heap; refused when
+ * lanes_per_warp / lanes_per_pair such heaps exceed 200 KB) and lanes per pair
+ * (1: one lane marches a pair; 4, the default, or 8: half a warp does, the
+ * lanes solving the neighbours of the accepted node together, two pairs per
+ * warp, or one where two heaps exceed 200 KB).  None of them changes a
  * result. */
 int swdk_fmst_set_options(swdk_fmst* fmst, size_t scratch_budget_bytes, int lanes_per_warp, int warps_per_sm,
                           int smem_heap_entries, int lanes_per_pair);

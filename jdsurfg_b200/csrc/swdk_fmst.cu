@@ -107,10 +107,11 @@ __global__ void __launch_bounds__(128) k_fmst_travel(Grid G, int npair, int lane
     }
 }
 
-// The same with two pairs per warp (March::march_half), one warp per block;
-// the pairs go round the resident warps.  HEAP as march_pair's.
+// The same by half a warp per pair (March::march_half), ppw (1 or 2) pairs per
+// warp, one warp per block; the pairs go round the resident warps.  HEAP as
+// march_pair's.
 template <int HEAP>
-__global__ void __launch_bounds__(32) k_fmst_travel_half(Grid G, int npair, const int32_t* __restrict__ cp,
+__global__ void __launch_bounds__(32) k_fmst_travel_half(Grid G, int npair, int ppw, const int32_t* __restrict__ cp,
                                                          const float* __restrict__ srcx,
                                                          const float* __restrict__ srcz,
                                                          const int32_t* __restrict__ pslot,
@@ -120,8 +121,8 @@ __global__ void __launch_bounds__(32) k_fmst_travel_half(Grid G, int npair, cons
                                                          unsigned int* __restrict__ n_overflow, int smem_cap) {
     extern __shared__ __align__(16) FHeap sheap[];
     const int half = threadIdx.x >> 4;
-    for (int p0 = 2 * blockIdx.x; p0 < npair; p0 += 2 * gridDim.x) {
-        const bool mine = p0 + half < npair;
+    for (int p0 = ppw * blockIdx.x; p0 < npair; p0 += ppw * gridDim.x) {
+        const bool mine = half < ppw && p0 + half < npair;
         const int p = mine ? p0 + half : p0;
         const unsigned mask = mine ? 0xffffu << (16 * half) : 0u;
         if (HEAP == 1)
@@ -227,6 +228,17 @@ struct swdk_fmst {
     cudaEvent_t t0 = nullptr, t1 = nullptr;
 };
 
+constexpr size_t FMST_SMEM = 200 * 1024;  // shared memory of a marching block (one warp)
+
+// Pairs that a warp marches at a time, with hstride entries of heap each in
+// shared memory (0: none).  Two by half a warp each, unless their heaps do not
+// fit together: swdk_fmst_set_options takes heaps of up to all of a block's
+// shared memory.
+static int pairs_per_warp(const swdk_fmst* f, size_t hstride) {
+    if (f->per == 1) return f->lanes;
+    return 2 * hstride * sizeof(FHeap) <= FMST_SMEM ? 2 : 1;
+}
+
 static int fail(swdk_fmst* f, const char* what, cudaError_t e) {
     f->err = std::string(what) + ": " + cudaGetErrorString(e);
     return SWDK_E_CUDA;
@@ -241,8 +253,8 @@ extern "C" int swdk_fmst_create(swdk_fmst** out, int device, const swdk_fmst_gri
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) { delete f; return SWDK_E_CUDA; }
     cudaDeviceGetAttribute(&f->nsm, cudaDevAttrMultiProcessorCount, device);
-    cudaFuncSetAttribute(k_fmst_travel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_fmst_travel_half<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(k_fmst_travel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FMST_SMEM);
+    cudaFuncSetAttribute(k_fmst_travel_half<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FMST_SMEM);
     // fmst_init (fmst.f90:27-64) and the r*sin(colatitude) tables
     f->G = make_grid(grid->nx, grid->ny, grid->goxd, grid->gozd, grid->dvxd, grid->dvzd);
     make_risti(f->G, f->risti_c, f->risti_r);
@@ -288,7 +300,7 @@ extern "C" int swdk_fmst_set_options(swdk_fmst* f, size_t scratch_budget_bytes, 
     if (!f || lanes_per_warp < 1 || lanes_per_warp > 32 || warps_per_sm < 0 || warps_per_sm > 64 ||
         smem_heap_entries < -1 || (lanes_per_pair != 1 && lanes_per_pair != 4 && lanes_per_pair != 8) ||
         lanes_per_warp % lanes_per_pair ||
-        (size_t)(lanes_per_warp / lanes_per_pair) * ((smem_heap_entries + 2) & ~1) * sizeof(FHeap) > 200 * 1024)
+        (size_t)(lanes_per_warp / lanes_per_pair) * ((smem_heap_entries + 2) & ~1) * sizeof(FHeap) > FMST_SMEM)
         return SWDK_E_ARG;
     f->smem_heap = smem_heap_entries;
     f->per = lanes_per_pair;
@@ -433,7 +445,7 @@ extern "C" int swdk_fmst_pairs(swdk_fmst* f, int npairs, const int32_t* slot, co
     // is a front across the grid), within 160 KB of shared memory per SM
     int smem_heap = f->smem_heap;
     if (smem_heap < 0) {
-        const int pairs_per_sm = std::max(1, (f->warps_per_sm > 0 ? f->warps_per_sm : 16) * (f->per == 1 ? f->lanes : 2));
+        const int pairs_per_sm = std::max(1, (f->warps_per_sm > 0 ? f->warps_per_sm : 16) * pairs_per_warp(f, 0));
         smem_heap = (int)std::min<size_t>((size_t)(1.5 * (G.nnx + G.nnz)), (160u << 10) / (8u * pairs_per_sm) - 2);
         if (smem_heap < 256) smem_heap = 0;
     }
@@ -509,7 +521,7 @@ extern "C" int swdk_fmst_pairs(swdk_fmst* f, int npairs, const int32_t* slot, co
             k_fmst_refvel<<<dim3(8, np), 256, 0, st>>>(G, np, dcp, d_srcx, d_srcz, d_pslot, d_used, d_vc, S.rvel,
                                                       S.rslw, S.geo);
             {
-                const int ppw = f->per == 1 ? f->lanes : 2;  // pairs marched by a warp at a time
+                const int ppw = pairs_per_warp(f, smem ? hstride : 0);
                 int warps = (np + ppw - 1) / ppw;
                 if (f->warps_per_sm > 0) warps = std::min(warps, f->warps_per_sm * f->nsm);
                 const size_t shm = smem ? (size_t)ppw * hstride * sizeof(FHeap) : 0;
@@ -528,7 +540,7 @@ extern "C" int swdk_fmst_pairs(swdk_fmst* f, int npairs, const int32_t* slot, co
                     const auto k = smem ? k_fmst_travel_half<1>
                                         : cap >= 65536 ? k_fmst_travel_half<2> : k_fmst_travel_half<0>;
                     cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carve);
-                    k<<<warps, 32, shm, st>>>(G, np, dcp, d_srcx, d_srcz, d_pslot, slwn, f->d_risti_c, f->d_risti_r, S,
+                    k<<<warps, 32, shm, st>>>(G, np, ppw, dcp, d_srcx, d_srcz, d_pslot, slwn, f->d_risti_c, f->d_risti_r, S,
                                               f->d_overflow, smem ? (int)cap : 0);
                 }
             }

@@ -63,3 +63,19 @@ def test_small_grids_and_lone_pairs(nx, ny, npairs):
     for heap in (-1, 0, 40):
         got, _ = _run(grid, pairs, v, smem_heap=heap)
         assert _same(ref, got), heap
+
+
+# shared-memory heaps up to all of a block's 200 KB (25 598 entries, one pair a
+# warp); the largest two of a warp (12 798); the next sizes are refused
+@pytest.mark.parametrize("lanes,per,heap", [(4, 4, 25598), (8, 8, 25598), (4, 4, 12800), (8, 4, 12798), (8, 8, 12798),
+                                            (1, 1, 25598)])
+def test_largest_shared_heaps(lanes, per, heap):
+    from jdsurfg_b200.engine import SwdkError
+    grid = (33, 36, 40.0, 100.0, 0.2, 0.2)  # a full heap of 31 933 entries
+    pairs, v = _pairs(grid, 5, 5, 9), _rough(grid, 2)
+    ref, _ = _run(grid, pairs, v, lanes_per_warp=1, lanes_per_pair=1, smem_heap=0)
+    got, info = _run(grid, pairs, v, lanes_per_warp=lanes, lanes_per_pair=per, smem_heap=heap)
+    assert info["overflow_pairs"] == 0 and _same(ref, got)
+    with pytest.raises(SwdkError, match="set_options"):
+        _run(grid, pairs, v, lanes_per_warp=lanes, lanes_per_pair=per,
+             smem_heap=25600 if lanes == per else 12800)
