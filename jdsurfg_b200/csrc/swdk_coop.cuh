@@ -9,9 +9,9 @@
 // A group of W lanes therefore forms the entries of W layers at once, one
 // per lane, leaves them in shared memory, and runs the W products from
 // there.  The entries and products are the functions that the one-lane
-// evaluation runs (dunkin_entries / dunkin_product, love_coef /
-// love_product), in the same order, so the values are the same bits.
-//
+// evaluation runs (layer_coef, dunkin_entries, dunkin_product; love_coef,
+// love_product; for layered models the _ref ones), every rounding written
+// out, in the same order, so the values are the same bits.
 //
 // What bounds it: the dependent FP64 chain.  With W = 32 and a warp or two per
 // scheduler an evaluation of 161 layers takes 57 000 cycles (entries 19 000,
@@ -62,71 +62,6 @@ __device__ __forceinline__ Dunkin load_dunkin(const double* row) {
   t = q[8]; d.c43 = t.x; d.c51 = t.y;
   d.c53 = row[18];
   return d;
-}
-
-// dltar4's and dltar1's own forms of a layer (surfdisp96.f:712-1095), for
-// layered models: the divisions, square roots and exponentials as dltar4 /
-// dltar1 write them
-__device__ __forceinline__ void vertical_ref(double wvno, double xk, double dpth, double& over, double& times,
-                                             double& cosv, double& ex) {
-  const double r = sqrt((wvno + xk) * fabs(wvno - xk)), p = r * dpth;
-  ex = 0.0;
-  if (wvno < xk) {
-    double s, c;
-    sincos(p, &s, &c);
-    over = s / r; times = -r * s; cosv = c;
-  } else if (wvno == xk) {
-    cosv = 1.0; over = dpth; times = 0.0;
-  } else {
-    ex = p;
-    const double fac = (p < 16.0) ? exp(-2.0 * p) : 0.0;
-    cosv = (1.0 + fac) * 0.5;
-    const double s = (1.0 - fac) * 0.5;
-    over = s / r; times = r * s;
-  }
-}
-
-__device__ __forceinline__ LayerCoef layer_coef_ref(const float4 ly, double wvno, double wvno2, double omega,
-                                                    double iom) {
-  LayerCoef k;
-  k.rho = ly.w;
-  k.irho = 1.0 / k.rho;
-  const double t = (double)ly.z * iom;
-  k.gammk = 2.0 * t * t;
-  k.gam = k.gammk * wvno2;
-  double w, x, cosp, pex, y, z, cosq, sex;
-  vertical_ref(wvno, omega / (double)ly.y, ly.x, w, x, cosp, pex);
-  vertical_ref(wvno, omega / (double)ly.z, ly.x, y, z, cosq, sex);
-  const double exa = pex + sex;
-  k.a0 = (exa < 60.0) ? exp(-exa) : 0.0;
-  k.cpcq = cosp * cosq; k.cpy = cosp * y; k.cpz = cosp * z; k.cqw = cosq * w; k.cqx = cosq * x;
-  k.xy = x * y; k.xz = x * z; k.wy = w * y; k.wz = w * z;
-  return k;
-}
-
-__device__ __forceinline__ RayVec rayleigh_start_ref(const float4 h, double wvno, double wvno2, double omega,
-                                                     double iom) {
-  const double a = h.y, b = h.z, rho1 = h.w;
-  const double xka = omega / a, xkb = omega / b;
-  const double ra = sqrt((wvno + xka) * fabs(wvno - xka)), rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
-  const double t = b * iom, gammk = 2.0 * t * t, gam = gammk * wvno2, gamm1 = gam - 1.0;
-  RayVec e;
-  e.e0 = rho1 * rho1 * (gamm1 * gamm1 - gam * gammk * ra * rb);
-  e.e1 = -rho1 * ra;
-  e.e2 = rho1 * (gamm1 - gammk * ra * rb);
-  e.e3 = rho1 * rb;
-  e.e4 = wvno2 - ra * rb;
-  return e;
-}
-
-__device__ __forceinline__ LoveCoef love_coef_ref(const float4 ly, double wvno, double omega) {
-  const double beta1 = ly.z, rho1 = ly.w;
-  LoveCoef k;
-  double ex;
-  k.xmu = rho1 * beta1 * beta1;
-  k.ixmu = 1.0 / k.xmu;
-  vertical_ref(wvno, omega / beta1, ly.x, k.y, k.z, k.cosq, ex);
-  return k;
 }
 
 // NORM 0: dltar4 as written (normalised at every layer by the reciprocal)
@@ -189,13 +124,7 @@ __device__ double coop_rayleigh(bool on, const LayerView& V, double wvno, double
     __syncwarp();
   }
   if (on && V.llw != 1) {
-    if (NORM == 0) {
-      const float4 ly = V.get(0);
-      double w, x, cosp, ex;
-      vertical_ref(wvno, omega / (double)ly.y, ly.x, w, x, cosp, ex);
-      const double w0 = -(double)ly.w * w;
-      return cosp * e0 + w0 * e1;
-    }
+    if (NORM == 0) return rayleigh_fluid_top_ref(V.get(0), wvno, omega, e0, e1);
     return rayleigh_fluid_top(V.layer(0), wvno, omega, e0, e1);
   }
   return e0;
@@ -206,10 +135,7 @@ __device__ double coop_love(bool on, const LayerView& V, double wvno, double ome
   const int hs = on ? V.L - 1 : 0, mlo = on ? V.llw - 1 : 0;
   double e1 = 0.0, e2 = 0.0;
   if (on && NORM == 0) {
-    const float4 h = V.get(hs);
-    const double beta1 = h.z, xkb = omega / beta1;
-    e1 = (double)h.w * sqrt((wvno + xkb) * fabs(wvno - xkb));
-    e2 = 1.0 / (beta1 * beta1);
+    love_start_ref(V.get(hs), wvno, omega, e1, e2);
   } else if (on) {
     love_start(V.layer(hs), wvno, omega, e1, e2);
   }
@@ -237,7 +163,7 @@ __device__ double coop_love(bool on, const LayerView& V, double wvno, double ome
       t = q[2]; k.ixmu = t.x;
       const bool norm = ++since >= NORM || a + i == n - 1;
       if (norm) since = 0;
-      love_product<NORM == 0 ? 4 : NORM>(k, norm, e1, e2);
+      love_product<NORM>(k, norm, e1, e2);
     }
     __syncwarp();
   }

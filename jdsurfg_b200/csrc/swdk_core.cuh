@@ -236,172 +236,6 @@ struct LayerView {
   }
 };
 
-// dltar4 (surfdisp96.f:798-898)
-SWDK_HDI double dltar4(const LayerView& V, double wvno, double omga) {
-  double omega = omga;
-  if (omega < 1.0e-4) omega = 1.0e-4;
-  const double wvno2 = wvno * wvno;
-  const double iom = 1.0 / omega;
-  float4 h = V.get(V.L - 1);
-  double a = h.y, b = h.z, rho1 = h.w;
-  double xka = omega / a, xkb = omega / b;
-  double ra = sqrt((wvno + xka) * fabs(wvno - xka));
-  double rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
-  double t = b * iom;
-  double gammk = 2.0 * t * t;
-  double gam = gammk * wvno2;
-  double gamm1 = gam - 1.0;
-  double e0 = rho1 * rho1 * (gamm1 * gamm1 - gam * gammk * ra * rb);
-  double e1 = -rho1 * ra;
-  double e2 = rho1 * (gamm1 - gammk * ra * rb);
-  double e3 = rho1 * rb;
-  double e4 = wvno2 - ra * rb;
-  for (int m = V.L - 2; m >= V.llw - 1; --m) {
-    float4 ly = V.get(m);
-    const double dpth = ly.x;
-    a = ly.y;
-    b = ly.z;
-    const double rho = ly.w;
-    xka = omega / a;
-    xkb = omega / b;
-    t = b * iom;
-    gammk = 2.0 * t * t;
-    gam = gammk * wvno2;
-    ra = sqrt((wvno + xka) * fabs(wvno - xka));
-    rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
-    const double p = ra * dpth, q = rb * dpth;
-    // var (surfdisp96.f:901-1018)
-    double w, x, cosp, y, z, cosq, pex = 0.0, sex = 0.0;
-    if (wvno < xka) {
-      double sp, cp;
-      sincos(p, &sp, &cp);
-      w = sp / ra; x = -ra * sp; cosp = cp;
-    } else if (wvno == xka) {
-      cosp = 1.0; w = dpth; x = 0.0;
-    } else {
-      pex = p;
-      double fac = (p < 16.0) ? exp(-2.0 * p) : 0.0;
-      cosp = (1.0 + fac) * 0.5;
-      double sp = (1.0 - fac) * 0.5;
-      w = sp / ra; x = ra * sp;
-    }
-    if (wvno < xkb) {
-      double sq, cq;
-      sincos(q, &sq, &cq);
-      y = sq / rb; z = -rb * sq; cosq = cq;
-    } else if (wvno == xkb) {
-      cosq = 1.0; y = dpth; z = 0.0;
-    } else {
-      sex = q;
-      double fac = (q < 16.0) ? exp(-2.0 * q) : 0.0;
-      cosq = (1.0 + fac) * 0.5;
-      double sq = (1.0 - fac) * 0.5;
-      y = sq / rb; z = rb * sq;
-    }
-    const double exa = pex + sex;
-    const double a0 = (exa < 60.0) ? exp(-exa) : 0.0;
-    const double cpcq = cosp * cosq, cpy = cosp * y, cpz = cosp * z, cqw = cosq * w, cqx = cosq * x;
-    const double xy = x * y, xz = x * z, wy = w * y, wz = w * z;
-    // dnka (surfdisp96.f:1051-1095)
-    const double irho = 1.0 / rho;
-    gamm1 = gam - 1.0;
-    const double twgm1 = gam + gamm1, gmgmk = gam * gammk, gmgm1 = gam * gamm1, gm1sq = gamm1 * gamm1;
-    const double rho2 = rho * rho, irho2 = irho * irho;
-    const double a0pq = a0 - cpcq;
-    const double c11 = cpcq - 2.0 * gmgm1 * a0pq - gmgmk * xz - wvno2 * gm1sq * wy;
-    const double c12 = (wvno2 * cpy - cqx) * irho;
-    const double c13 = -(twgm1 * a0pq + gammk * xz + wvno2 * gamm1 * wy) * irho;
-    const double c14 = (cpz - wvno2 * cqw) * irho;
-    const double c15 = -(2.0 * wvno2 * a0pq + xz + wvno2 * wvno2 * wy) * irho2;
-    const double c21 = (gmgmk * cpz - gm1sq * cqw) * rho;
-    const double c22 = cpcq;
-    const double c23 = gammk * cpz - gamm1 * cqw;
-    const double c24 = -wz;
-    const double c41 = (gm1sq * cpy - gmgmk * cqx) * rho;
-    const double c42 = -xy;
-    const double c43 = gamm1 * cpy - gammk * cqx;
-    const double c51 = -(2.0 * gmgmk * gm1sq * a0pq + gmgmk * gmgmk * xz + gm1sq * gm1sq * wy) * rho2;
-    const double c53 = -(gammk * gamm1 * twgm1 * a0pq + gam * gammk * gammk * xz + gamm1 * gm1sq * wy) * rho;
-    const double tt = -2.0 * wvno2;
-    const double c31 = tt * c53, c32 = tt * c43, c33 = a0 + 2.0 * (cpcq - c11), c34 = tt * c23, c35 = tt * c13;
-    // ee(i) = sum_j e(j) ca(j,i); ca rows: 1:(c11..c15) 2:(c21,c22,c23,c24,c14)
-    // 3:(c31..c35) 4:(c41,c42,c43,c22,c12) 5:(c51,c41,c53,c21,c11)
-    double f0 = e0 * c11 + e1 * c21 + e2 * c31 + e3 * c41 + e4 * c51;
-    double f1 = e0 * c12 + e1 * c22 + e2 * c32 + e3 * c42 + e4 * c41;
-    double f2 = e0 * c13 + e1 * c23 + e2 * c33 + e3 * c43 + e4 * c53;
-    double f3 = e0 * c14 + e1 * c24 + e2 * c34 + e3 * c22 + e4 * c21;
-    double f4 = e0 * c15 + e1 * c14 + e2 * c35 + e3 * c12 + e4 * c11;
-    // normc (surfdisp96.f:1022-1047): divide by the largest magnitude
-    double t1 = fmax(fmax(fmax(fabs(f0), fabs(f1)), fmax(fabs(f2), fabs(f3))), fabs(f4));
-    if (t1 < 1.e-40) t1 = 1.0;
-    const double it1 = 1.0 / t1;
-    e0 = f0 * it1; e1 = f1 * it1; e2 = f2 * it1; e3 = f3 * it1; e4 = f4 * it1;
-  }
-  if (V.llw != 1) {
-    float4 ly = V.get(0);
-    const double a0l = ly.y, dpth = ly.x, rho = ly.w;
-    xka = omega / a0l;
-    ra = sqrt((wvno + xka) * fabs(wvno - xka));
-    const double p = ra * dpth;
-    double w, cosp;
-    if (wvno < xka) {
-      double sp, cp;
-      sincos(p, &sp, &cp);
-      w = sp / ra; cosp = cp;
-    } else if (wvno == xka) {
-      cosp = 1.0; w = dpth;
-    } else {
-      double fac = (p < 16.0) ? exp(-2.0 * p) : 0.0;
-      cosp = (1.0 + fac) * 0.5;
-      w = ((1.0 - fac) * 0.5) / ra;
-    }
-    const double w0 = -rho * w;
-    return cosp * e0 + w0 * e1;
-  }
-  return e0;
-}
-
-// dltar1 (surfdisp96.f:734-794)
-SWDK_HDI double dltar1(const LayerView& V, double wvno, double omega) {
-  float4 h = V.get(V.L - 1);
-  double beta1 = h.z, rho1 = h.w;
-  double xkb = omega / beta1;
-  double rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
-  double e1 = rho1 * rb;
-  double e2 = 1.0 / (beta1 * beta1);
-  for (int m = V.L - 2; m >= V.llw - 1; --m) {
-    float4 ly = V.get(m);
-    beta1 = ly.z;
-    rho1 = ly.w;
-    const double dpth = ly.x;
-    const double xmu = rho1 * beta1 * beta1;
-    xkb = omega / beta1;
-    rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
-    const double q = dpth * rb;
-    double cosq, y, z;
-    if (wvno < xkb) {
-      double sq, cq;
-      sincos(q, &sq, &cq);
-      y = sq / rb; z = -rb * sq; cosq = cq;
-    } else if (wvno == xkb) {
-      cosq = 1.0; y = dpth; z = 0.0;
-    } else {
-      double fac = (q < 16.0) ? exp(-2.0 * q) : 0.0;
-      cosq = (1.0 + fac) * 0.5;
-      double sq = (1.0 - fac) * 0.5;
-      y = sq / rb; z = rb * sq;
-    }
-    const double e10 = e1 * cosq + e2 * xmu * z;
-    const double e20 = e1 * y / xmu + e2 * cosq;
-    double xnor = fmax(fabs(e10), fabs(e20));
-    if (xnor < 1.e-40) xnor = 1.0;
-    const double ix = 1.0 / xnor;
-    e1 = e10 * ix;
-    e2 = e20 * ix;
-  }
-  return e1;
-}
-
 // 1/x for the positive, normal layer parameters: the hardware estimate
 // (PTX rcp.approx.ftz.f64) refined by two Newton-Raphson steps
 // r <- r + r (1 - x r), each with fused multiply-adds; the relative error
@@ -431,7 +265,7 @@ struct LayerCoef {
   double a0, cpcq, cpy, cpz, cqw, cqx, xy, xz, wy, wz, gam, gammk, rho, irho;
 };
 
-// Sums of products in the Rayleigh evaluation are written with the rounding
+// Sums of products in the period equations are written with the rounding
 // they have: xmul / xadd round, xfma rounds once.  Left to the compiler, the
 // same expressions were contracted differently in the one-lane loop and in
 // the group kernel, and unrounded roots differed by 1e-15 km/s; written out,
@@ -591,24 +425,22 @@ SWDK_HD void rayleigh_norm(double& e0, double& e1, double& e2, double& e3, doubl
 
 SWDK_HD double rayleigh_fluid_top(const float4 ly, double wvno, double omega, double e0, double e1) {
   const double dpth = ly.x, rho = ly.w;
-  const double xka = omega * recip((double)ly.y);
-  const double Xa = (wvno + xka) * fabs(wvno - xka);
+  const double xka = xmul(omega, recip((double)ly.y));
+  const double Xa = xmul(xadd(wvno, xka), fabs(xadd(wvno, -xka)));
+  const double ir = rsqrt(Xa), r = xmul(Xa, ir), p = xmul(r, dpth);  // not used where X = 0
   double w, cosp;
   if (wvno < xka) {
-    const double ir = rsqrt(Xa), r = Xa * ir;
     double sp, cp;
-    sincos(r * dpth, &sp, &cp);
-    w = sp * ir; cosp = cp;
+    sincos(p, &sp, &cp);
+    w = xmul(sp, ir); cosp = cp;
   } else if (wvno == xka) {
     cosp = 1.0; w = dpth;
   } else {
-    const double ir = rsqrt(Xa), r = Xa * ir, p = r * dpth;
-    const double fac = (p < 16.0) ? exp(-2.0 * p) : 0.0;
-    cosp = (1.0 + fac) * 0.5;
-    w = ((1.0 - fac) * 0.5) * ir;
+    const double fac = (p < 16.0) ? exp(xmul(-2.0, p)) : 0.0;
+    cosp = xmul(xadd(1.0, fac), 0.5);
+    w = xmul(xmul(xadd(1.0, -fac), 0.5), ir);
   }
-  const double w0 = -rho * w;
-  return cosp * e0 + w0 * e1;
+  return xfma(cosp, e0, xmul(xmul(-rho, w), e1));
 }
 
 template <int NORM, bool NODES>
@@ -658,44 +490,44 @@ SWDK_HD LoveCoef love_coef(const float4 ly, double wvno, double omega) {
   const double beta1 = ly.z, rho1 = ly.w;
   const double dpth = ly.x;
   LoveCoef k;
-  k.xmu = rho1 * beta1 * beta1;
+  k.xmu = xmul(xmul(rho1, beta1), beta1);
   k.ixmu = recip(k.xmu);
-  const double xkb = omega * recip(beta1);
-  const double Xb = (wvno + xkb) * fabs(wvno - xkb);
+  const double xkb = xmul(omega, recip(beta1));
+  const double Xb = xmul(xadd(wvno, xkb), fabs(xadd(wvno, -xkb)));
+  const double ir = rsqrt(Xb), r = xmul(Xb, ir), q = xmul(dpth, r);  // not used where X = 0
   if (wvno < xkb) {
-    const double ir = rsqrt(Xb), r = Xb * ir;
     double sq, cq;
-    sincos(dpth * r, &sq, &cq);
-    k.y = sq * ir; k.z = -r * sq; k.cosq = cq;
+    sincos(q, &sq, &cq);
+    k.y = xmul(sq, ir); k.z = xmul(-r, sq); k.cosq = cq;
   } else if (wvno == xkb) {
     k.cosq = 1.0; k.y = dpth; k.z = 0.0;
   } else {
-    const double ir = rsqrt(Xb), r = Xb * ir, q = dpth * r;
-    const double fac = (q < 16.0) ? exp(-2.0 * q) : 0.0;
-    k.cosq = (1.0 + fac) * 0.5;
-    const double sq = (1.0 - fac) * 0.5;
-    k.y = sq * ir; k.z = r * sq;
+    const double fac = (q < 16.0) ? exp(xmul(-2.0, q)) : 0.0;
+    k.cosq = xmul(xadd(1.0, fac), 0.5);
+    const double sq = xmul(xadd(1.0, -fac), 0.5);
+    k.y = xmul(sq, ir); k.z = xmul(r, sq);
   }
   return k;
 }
 
 SWDK_HD void love_start(const float4 h, double wvno, double omega, double& e1, double& e2) {
-  const double beta1 = h.z, rho1 = h.w;
-  const double xkb = omega * recip(beta1);
-  const double rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
-  e1 = rho1 * rb;
-  e2 = 1.0 / (beta1 * beta1);
+  const double beta1 = h.z, rho1 = h.w, ib = recip(beta1);
+  e1 = xmul(rho1, sqrt(xmul(xfma(omega, ib, wvno), fabs(xfma(-omega, ib, wvno)))));
+  e2 = 1.0 / xmul(beta1, beta1);
 }
 
+// NORM as rayleigh_norm's; 0: dltar1 as written (divides by xmu, normalises
+// by the reciprocal)
 template <int NORM>
 SWDK_HD void love_product(const LoveCoef& k, bool norm, double& e1, double& e2) {
-  const double e10 = e1 * k.cosq + e2 * k.xmu * k.z;
-  const double e20 = e1 * k.y * k.ixmu + e2 * k.cosq;
+  const double e1y = xmul(e1, k.y);
+  const double e10 = xfma(e1, k.cosq, xmul(xmul(e2, k.xmu), k.z));
+  const double e20 = xfma(e2, k.cosq, NORM == 0 ? e1y / k.xmu : xmul(e1y, k.ixmu));
   if (norm) {
     double xnor = fmax(fabs(e10), fabs(e20));
     if (xnor < 1.e-40) xnor = 1.0;
     if (NORM == 1) { e1 = e10 / xnor; e2 = e20 / xnor; }
-    else { const double ix2 = 1.0 / xnor; e1 = e10 * ix2; e2 = e20 * ix2; }
+    else { const double ix2 = 1.0 / xnor; e1 = xmul(e10, ix2); e2 = xmul(e20, ix2); }
   } else {
     e1 = e10; e2 = e20;
   }
@@ -705,52 +537,120 @@ SWDK_HD void love_product(const LoveCoef& k, bool norm, double& e1, double& e2) 
 template <int NORM, bool NODES>
 SWDK_HDI double dltar1_fast(const LayerView& V, double wvno, double omega) {
   const int hs = V.L - 1;  // the half-space
-  float4 h = V.layer(hs);
-  double beta1 = h.z, rho1 = h.w;
-  double xkb = omega * recip(beta1);
-  double rb = sqrt((wvno + xkb) * fabs(wvno - xkb));
-  double e1 = rho1 * rb;
-  double e2 = 1.0 / (beta1 * beta1);
+  double e1, e2;
+  love_start(V.layer(hs), wvno, omega, e1, e2);
   int since = 0;
   const int mlo = V.llw - 1;
   LayerView::Walk wk;
   if (hs - 1 >= mlo) V.walk_start<-1, NODES>(wk, hs - 1);
   for (int m = hs - 1; m >= mlo; --m) {
-    const float4 ly = V.walk_layer<-1, NODES>(wk, m);
-    beta1 = ly.z;
-    rho1 = ly.w;
-    const double dpth = ly.x;
-    const double xmu = rho1 * beta1 * beta1;
-    const double ixmu = recip(xmu);
-    xkb = omega * recip(beta1);
-    const double Xb = (wvno + xkb) * fabs(wvno - xkb);
-    double cosq, y, z;
-    if (wvno < xkb) {
-      const double ir = rsqrt(Xb), r = Xb * ir;
-      double sq, cq;
-      sincos(dpth * r, &sq, &cq);
-      y = sq * ir; z = -r * sq; cosq = cq;
-    } else if (wvno == xkb) {
-      cosq = 1.0; y = dpth; z = 0.0;
-    } else {
-      const double ir = rsqrt(Xb), r = Xb * ir, q = dpth * r;
-      const double fac = (q < 16.0) ? exp(-2.0 * q) : 0.0;
-      cosq = (1.0 + fac) * 0.5;
-      const double sq = (1.0 - fac) * 0.5;
-      y = sq * ir; z = r * sq;
-    }
-    const double e10 = e1 * cosq + e2 * xmu * z;
-    const double e20 = e1 * y * ixmu + e2 * cosq;
-    if (++since >= NORM || m == V.llw - 1) {
-      since = 0;
-      double xnor = fmax(fabs(e10), fabs(e20));
-      if (xnor < 1.e-40) xnor = 1.0;
-      if (NORM == 1) { e1 = e10 / xnor; e2 = e20 / xnor; }
-      else { const double ix2 = 1.0 / xnor; e1 = e10 * ix2; e2 = e20 * ix2; }
-    } else {
-      e1 = e10; e2 = e20;
-    }
+    const LoveCoef k = love_coef(V.walk_layer<-1, NODES>(wk, m), wvno, omega);
+    const bool norm = ++since >= NORM || m == mlo;
+    if (norm) since = 0;
+    love_product<NORM>(k, norm, e1, e2);
   }
+  return e1;
+}
+
+// ---------------------------------------------------------------------------
+// dltar4 and dltar1 as written (surfdisp96.f:712-1095), for layered models:
+// their divisions, square roots and exponentials, normalised at every layer by
+// the reciprocal.  The roundings of the sums are those that the compiler gave
+// these expressions in the one-lane kernel (the group kernel forms the same
+// values layer by layer).
+// ---------------------------------------------------------------------------
+SWDK_HD void vertical_ref(double wvno, double xk, double dpth, double& over, double& times, double& cosv,
+                          double& ex) {
+  const double r = sqrt(xmul(xadd(wvno, xk), fabs(xadd(wvno, -xk)))), p = xmul(r, dpth);
+  ex = 0.0;
+  if (wvno < xk) {
+    double s, c;
+    sincos(p, &s, &c);
+    over = s / r; times = xmul(-r, s); cosv = c;
+  } else if (wvno == xk) {
+    cosv = 1.0; over = dpth; times = 0.0;
+  } else {
+    ex = p;
+    const double fac = (p < 16.0) ? exp(xmul(-2.0, p)) : 0.0;
+    cosv = xmul(xadd(1.0, fac), 0.5);
+    const double s = xmul(xadd(1.0, -fac), 0.5);
+    over = s / r; times = xmul(r, s);
+  }
+}
+
+SWDK_HD LayerCoef layer_coef_ref(const float4 ly, double wvno, double wvno2, double omega, double iom) {
+  LayerCoef k;
+  k.rho = ly.w;
+  k.irho = 1.0 / k.rho;
+  const double t = xmul((double)ly.z, iom);
+  k.gammk = xmul(2.0 * t, t);
+  k.gam = xmul(k.gammk, wvno2);
+  double w, x, cosp, pex, y, z, cosq, sex;
+  vertical_ref(wvno, omega / (double)ly.y, ly.x, w, x, cosp, pex);
+  vertical_ref(wvno, omega / (double)ly.z, ly.x, y, z, cosq, sex);
+  const double exa = xadd(pex, sex);
+  k.a0 = (exa < 60.0) ? exp(-exa) : 0.0;
+  k.cpcq = xmul(cosp, cosq); k.cpy = xmul(cosp, y); k.cpz = xmul(cosp, z);
+  k.cqw = xmul(cosq, w); k.cqx = xmul(cosq, x);
+  k.xy = xmul(x, y); k.xz = xmul(x, z); k.wy = xmul(w, y); k.wz = xmul(w, z);
+  return k;
+}
+
+SWDK_HD RayVec rayleigh_start_ref(const float4 h, double wvno, double wvno2, double omega, double iom) {
+  const double a = h.y, b = h.z, rho1 = h.w;
+  const double xka = omega / a, xkb = omega / b;
+  const double ra = sqrt(xmul(xadd(wvno, xka), fabs(xadd(wvno, -xka))));
+  const double rb = sqrt(xmul(xadd(wvno, xkb), fabs(xadd(wvno, -xkb))));
+  const double t = xmul(b, iom), gammk = xmul(2.0 * t, t), gam = xmul(gammk, wvno2), gamm1 = xadd(gam, -1.0);
+  RayVec e;
+  e.e0 = xmul(xmul(rho1, rho1), xfma(gamm1, gamm1, -xmul(xmul(xmul(gam, gammk), ra), rb)));
+  e.e1 = xmul(-rho1, ra);
+  e.e2 = xmul(rho1, xfma(-xmul(gammk, ra), rb, gamm1));
+  e.e3 = xmul(rho1, rb);
+  e.e4 = xadd(wvno2, -xmul(ra, rb));
+  return e;
+}
+
+SWDK_HD double rayleigh_fluid_top_ref(const float4 ly, double wvno, double omega, double e0, double e1) {
+  double w, x, cosp, ex;
+  vertical_ref(wvno, omega / (double)ly.y, ly.x, w, x, cosp, ex);
+  return xfma(cosp, e0, xmul(xmul(-(double)ly.w, w), e1));
+}
+
+SWDK_HD LoveCoef love_coef_ref(const float4 ly, double wvno, double omega) {
+  const double beta1 = ly.z, rho1 = ly.w;
+  LoveCoef k;
+  double ex;
+  k.xmu = xmul(xmul(rho1, beta1), beta1);
+  k.ixmu = 0.0;  // love_product<0> divides
+  vertical_ref(wvno, omega / beta1, ly.x, k.y, k.z, k.cosq, ex);
+  return k;
+}
+
+SWDK_HD void love_start_ref(const float4 h, double wvno, double omega, double& e1, double& e2) {
+  const double beta1 = h.z, xkb = omega / beta1;
+  e1 = xmul((double)h.w, sqrt(xmul(xadd(wvno, xkb), fabs(xadd(wvno, -xkb)))));
+  e2 = 1.0 / xmul(beta1, beta1);
+}
+
+SWDK_HDI double dltar4(const LayerView& V, double wvno, double omga) {
+  double omega = omga;
+  if (omega < 1.0e-4) omega = 1.0e-4;
+  const double wvno2 = wvno * wvno, iom = 1.0 / omega;
+  const RayVec st = rayleigh_start_ref(V.get(V.L - 1), wvno, wvno2, omega, iom);
+  double e0 = st.e0, e1 = st.e1, e2 = st.e2, e3 = st.e3, e4 = st.e4;
+  for (int m = V.L - 2; m >= V.llw - 1; --m) {
+    apply_dunkin(layer_coef_ref(V.get(m), wvno, wvno2, omega, iom), wvno2, e0, e1, e2, e3, e4);
+    rayleigh_norm<4>(e0, e1, e2, e3, e4);
+  }
+  if (V.llw != 1) return rayleigh_fluid_top_ref(V.get(0), wvno, omega, e0, e1);
+  return e0;
+}
+
+SWDK_HDI double dltar1(const LayerView& V, double wvno, double omega) {
+  double e1, e2;
+  love_start_ref(V.get(V.L - 1), wvno, omega, e1, e2);
+  for (int m = V.L - 2; m >= V.llw - 1; --m) love_product<0>(love_coef_ref(V.get(m), wvno, omega), true, e1, e2);
   return e1;
 }
 
