@@ -44,8 +44,9 @@ constexpr double FEAT_C0 = 3.5;                  // phase velocity offset of the
 // [0] secular evaluations, [1]/[2] Rayleigh/Love layer-evaluations,
 // [3]/[4] learned cells used / dropped, [5..10] evaluations by phase
 // (EV_* below)
-constexpr int NCOUNT = 11;
+constexpr int NCOUNT = 12;
 constexpr int EV_BASE = 5;
+constexpr int EV_WET = 11;  // not 0: some column has fluid nodes on top
 
 struct ColInfo {
   double cc;    // surfdisp96 start value cc (surfdisp96.f:222)
@@ -239,7 +240,8 @@ __global__ void __launch_bounds__(32 * PREP_COLS) k_prep(int ncol, int ldi, int 
                                               float4* __restrict__ lay0,
                                               ColInfo* __restrict__ info, float2* __restrict__ chainrule,
                                               float4* __restrict__ nodefeat, float4* __restrict__ nodes,
-                                              const DepthLayer* __restrict__ dl) {
+                                              const DepthLayer* __restrict__ dl,
+                                              unsigned long long* __restrict__ wet) {
   const unsigned FULL = 0xffffffffu;
   __shared__ float sv[PREP_COLS][NZMAX], sp[PREP_COLS][NZMAX], sr[PREP_COLS][NZMAX], dep[NZMAX];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -357,6 +359,7 @@ __global__ void __launch_bounds__(32 * PREP_COLS) k_prep(int ncol, int ldi, int 
     ci.betmx = betmx;
     ci.pad_ = 0.0f;
     info[col] = ci;
+    if (nw > 0) *wet = 1ull;
   }
 }
 
@@ -677,7 +680,9 @@ __global__ void __launch_bounds__(128, SWDK_ROOTS_MINB) k_roots_queue(int ncol, 
                                                      unsigned int retry_cap,
                                                      unsigned long long* __restrict__ nevals, RaggedMap rg,
                                                      const float4* __restrict__ nodes,
-                                                     const DepthLayer* __restrict__ dl) {
+                                                     const DepthLayer* __restrict__ dl,
+                                                     const unsigned long long* __restrict__ gate, int gate_on) {
+  if (gate && (*gate != 0ull) != (gate_on != 0)) return;  // the other kernel's call (launch_roots)
   double cbuf[KMAX_CHAIN];
   double cbbuf[KMAX_CHAIN + 24];
   // dynamic shared memory (ROOTS_SMEM): the chain states, and the chains'
@@ -981,33 +986,95 @@ cudaError_t roots_occupancy(int* per) {
   return e;
 }
 
-// Lanes per chain (1: k_roots_queue) for a root search of nitems chains.  One
-// lane each needs about 75 000 chains to fill the GPU; a call's time is then
-// the longest chain's, about 30 ms whatever the size.  More lanes shorten the
-// chain and cost throughput (the products run in every lane of a group; groups
-// of one warp that evaluate different numbers of velocities take turns).
-// Chains that walk the scan grid (no proposals, or higher modes, whose scans
-// the proposals leave) gain most from many lanes, which take eight points of
-// it at a time.  ms of the search with 1 / 4 / 32 lanes, 20 periods of 41
-// nodes, one mode:
-//   Rayleigh, proposals                    Rayleigh and Love, plain scan
-//   1500   28.7 / 17.7 /  5.1              11834  86.5 / 48.5 / 42.4 (30 periods)
-//   5200   28.9 / 12.7 / 15.8              16384  65.2 / 51.5 / 51.8
-//   12800  28.2 / 16.2 / 38.9              23040  69.8 / 56.7 / 71.6
-//   16384  28.4 / 26.9 / 48.3              32768  71.4 / 85.8 / 101.9
-// and two modes with coast columns 10240: 186.9 / 106.3 / 66.1, 20000: 257 /
-// 157 / 125 (8 and 16 lanes lie between and lead nowhere).  The lines are a
-// device's of 148 SMs and move with its size.
-int coop_lanes(long long nitems, int nsm, bool scans) {
-  const long long n = nitems * 148 / std::max(1, nsm);
-  if (scans) return n <= 18000 ? 32 : n <= 26000 ? 4 : 1;
-  return n <= 4500 ? 32 : n <= 16000 ? 4 : 1;
+// A root search's chains, for the choice of their kernel.
+struct RootsLoad {
+  long long items = 0;   // (chain, column) pairs
+  double work = 0.0;     // sum over them of periods x modes x layers, Love's evaluations counted less
+  double longest = 0.0;  // the largest of these terms, and of that chain:
+  int layers = 0;
+  double step = 0.4;     // log of the ratio of adjacent periods
+  bool love = false;
+  bool modes = false;    // chains of several modes
+  bool scans = false;    // chains without proposals
+  bool reference = false, layered = false;  // surfdisp96's refinement; swdk_surfdisp96_batch
+  void add(const ChainDesc& d, const double* t, long long ncol, int L) {
+    const double wave = d.iwave == 2 ? 1.0 : (0.25 * L + 20.0) / (L + 20.0);
+    const double w = (double)d.np * d.nmode * L * wave;
+    items += ncol;
+    work += w * ncol;
+    modes |= d.nmode > 1;
+    if (w <= longest) return;
+    longest = w;
+    layers = L;
+    love = d.iwave != 2;
+    const auto mm = std::minmax_element(t, t + d.np);
+    step = d.np > 1 ? std::log(*mm.second / *mm.first) / (d.np - 1) : 0.4;
+  }
+};
+
+// Lanes per chain, 1 (k_roots_queue, k_roots), 4 or 32.  One lane each needs
+// about 75 000 chains to fill the GPU; below that a call's time is the longest
+// chain's, whatever the number.  Groups shorten the chain and cost throughput
+// (the products run in every lane of a group, and trial velocities evaluated
+// ahead of need are partly wasted), so their time grows with the work.  Hence
+// the rule: how often the one-lane time holds the group kernel's, as a constant
+// over the number of longest chains that the work makes up; for 4 lanes no more
+// than a chain gains while every group is resident, and less where a few groups
+// are left for a second turn.  The constants fall with the layers (a round
+// between evaluations costs a group 4000 to 8000 cycles, whatever their number)
+// and for closely spaced periods, where a scan ends within the first of the
+// points that 32 lanes take at a time.  With a column under water (wet) the
+// longest chain is about twice as long.  ms of the search with 1 / 4 / 32 lanes,
+// Rayleigh, one mode, by the number of chains:
+//                                           6000              12000              20000
+//   161 layers, proposals, 9 periods   37 / 17 / 15       38 / 21 / 30       40 / 40 / 50
+//                          40 periods  52 / 25 / 38       52 / 31 / 75       56 / 58 / 123
+//               plain scan, 9 periods  50 / 21 / 17       49 / 27 / 34       53 / 51 / 57
+//               reference refinement   81 / 52 / 59       81 / 59 / 110      89 / 114 / 176
+//   13 layers, plain scan             6.2 / 3.5 / 5.0    6.2 / 4.6 / 10.0   6.8 / 9.9 / 17.6
+//   layered models, 9 layers          7.6 / 5.7 / 7.0    7.7 / 7.1 / 13.4   8.7 / 13.9 / 22.6
+//   129 layers, proposals, 2 % wet     96 / 31 / 20       96 / 39 / 39       97 / 51 / 57
+// The choice over 980 searches (ten kinds of 5 to 317 layers, four of layered
+// models of 2 to 200, 300 to 26 000 chains): 2.04 times as fast as one lane on
+// average, 0.95 at worst; the best of the three each time 2.07.  Over 588 more
+// (fluid columns, both waves): 1.99, 0.76 (five layers' nodes, two modes); 2.07.
+// The lines are a device's of 148 SMs and move with its size.
+int coop_lanes(const RootsLoad& l, int nsm, bool wet) {
+  if (l.items <= 0 || !(l.longest > 0.0)) return 1;
+  const double chains = l.work / l.longest * 148.0 / std::max(1, nsm);
+  const long long per = 32LL * std::max(1, nsm);       // chains of 4 lanes in one block per SM
+  const long long rounds = (l.items + per - 1) / per;  // blocks per SM that they take; three are resident
+  const double wide = std::min(1.0, std::max(0.0, std::log(l.step / 0.075) / std::log(0.4 / 0.075)));
+  const double L = l.layers;
+  double n32, n4, r4 = 3.0 - 0.45 * (double)rounds, fit = rounds <= 3 ? 1.0 : rounds == 4 ? 0.65 : 0.88;
+  if (l.layered) {
+    const double k = l.love ? 0.85 : 1.0;
+    n32 = k * (18000.0 + 12000.0 * wide) * (L + 3.0) / (L + 40.0);
+    n4 = k * 31000.0 * (L + 1.0) / (L + 20.0);
+    r4 *= L / (L + 6.0);
+  } else if (l.reference) {
+    n32 = (6500.0 + 4000.0 * wide) * (L + 25.0) / (L + 50.0);
+    n4 = 15500.0;
+    r4 *= 0.65;
+  } else {
+    const double k = l.love ? 1.4 : 1.0;
+    n32 = k * (l.scans && !l.modes ? 16000.0 + 6000.0 * wide : 11000.0 + 6500.0 * wide) * (L + 10.0) / (L + 45.0);
+    n4 = k * (19500.0 + 4000.0 * wide) * (L + 15.0) / (L + 45.0);
+  }
+  if (wet) {
+    n32 *= 1.3 + 0.5 * L / (L + 30.0);
+    n4 *= 1.0 + 0.9 * L / (L + 60.0);
+    r4 *= 1.2;
+  }
+  const double g32 = n32 / chains, g4 = rounds <= 3 ? std::min(r4, n4 / chains) : fit * n4 / chains;
+  if (g32 >= std::max(g4, 1.1)) return 32;
+  return g4 >= 1.0 ? 4 : 1;
 }
 
 struct RootsCall {
   int ncol;
   long long nitems;
-  bool scans;  // chains without proposals or of several modes
+  RootsLoad load;
   const int* order;
   const ChainDesc* chains;
   const double* periods;
@@ -1027,28 +1094,37 @@ struct RootsCall {
   RaggedMap rg;
   const float4* nodes;
   const DepthLayer* dl;
+  const unsigned long long* wet;  // the call's columns with fluid nodes on top, 0 or not (set by k_prep)
 };
 
 // the root search and the retries of its failed periods; rblocks: blocks of
 // k_roots_queue; tuned: that count was asked for (swdk_autotune, or the
 // caller's configuration), so the one-lane kernel runs
-cudaError_t launch_roots(const RootsCall& c, int rblocks, int nsm, bool tuned, cudaStream_t st) {
-  const int G = tuned ? 1 : coop_lanes(c.nitems, nsm, c.scans);
-  if (G > 1) {
-    const long long need = (c.nitems * G + 127) / 128;
-    const auto k = c.refine == 0 ? k_roots_coop<1> : k_roots_coop<4>;
-    const CoopArgs A{c.ncol,  (int)c.nitems,  G,       c.order,      c.chains, c.periods, c.layR,  c.layL, c.info,
-                     c.refine, c.rtol,        c.sngl,  RETRY_DEFERRED, c.croot, c.cstat,  c.queue, c.prop, c.retry_list,
-                     c.rctr,  c.rcap,         c.nevals, c.rg,          c.nodes, c.dl,     nullptr};
-    k<<<(unsigned)std::max(1LL, std::min<long long>(need, 3LL * nsm)), 128, coop_smem(G), st>>>(A);
-  } else {
-    k_roots_queue<<<(unsigned)std::max(1LL, std::min<long long>(rblocks, (c.nitems + 127) / 128)), 128, ROOTS_SMEM,
-                    st>>>(c.ncol, (int)c.nitems, c.order, c.chains, c.periods, c.layR, c.layL, c.info, c.refine,
-                          c.rtol, c.sngl, RETRY_DEFERRED, c.croot, c.cstat, c.queue, c.prop, c.retry_list, c.rctr,
-                          c.rcap, c.nevals, c.rg, c.nodes, c.dl);
+// Whether there are fluid columns is known on the device alone: where the
+// choice depends on it, both kernels are launched and one returns at once.
+cudaError_t launch_roots(const RootsCall& c, int rblocks, int nsm, bool tuned, int* launches, cudaStream_t st) {
+  const int dry = tuned ? 1 : coop_lanes(c.load, nsm, false), wet = tuned ? 1 : coop_lanes(c.load, nsm, true);
+  for (int pass = 0; pass < (dry == wet ? 1 : 2); ++pass) {
+    const int G = pass ? wet : dry;
+    const unsigned long long* gate = dry == wet ? nullptr : c.wet;
+    if (G > 1) {
+      const long long need = (c.nitems * G + 127) / 128;
+      const auto k = c.refine == 0 ? k_roots_coop<1> : k_roots_coop<4>;
+      const CoopArgs A{c.ncol,  (int)c.nitems,  G,       c.order,      c.chains, c.periods, c.layR,  c.layL, c.info,
+                       c.refine, c.rtol,        c.sngl,  RETRY_DEFERRED, c.croot, c.cstat,  c.queue, c.prop, c.retry_list,
+                       c.rctr,  c.rcap,         c.nevals, c.rg,          c.nodes, c.dl,     nullptr, gate, pass};
+      k<<<(unsigned)std::max(1LL, std::min<long long>(need, 3LL * nsm)), 128, coop_smem(G), st>>>(A);
+    } else {
+      k_roots_queue<<<(unsigned)std::max(1LL, std::min<long long>(rblocks, (c.nitems + 127) / 128)), 128, ROOTS_SMEM,
+                      st>>>(c.ncol, (int)c.nitems, c.order, c.chains, c.periods, c.layR, c.layL, c.info, c.refine,
+                            c.rtol, c.sngl, RETRY_DEFERRED, c.croot, c.cstat, c.queue, c.prop, c.retry_list, c.rctr,
+                            c.rcap, c.nevals, c.rg, c.nodes, c.dl, gate, pass);
+    }
+    *launches += 1;
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  *launches += 1;
   k_retry<<<(unsigned)rblocks, 128, RETRY_SMEM, st>>>(c.ncol, c.order, c.chains, c.periods, c.layR, c.layL, c.info,
                                                       c.refine, c.rtol, c.sngl, c.croot, c.cstat, c.retry_list, c.rctr,
                                                       c.rcap, c.rctr + 1, c.nevals, c.rg, c.nodes, c.dl);
@@ -1893,7 +1969,8 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
                                              ctx->lay0.as<float4>(), ctx->info.as<ColInfo>(),
                                              ctx->chainrule.as<float2>(), wantfeat ? ctx->nodefeat.as<float4>() : nullptr,
                                              use_nodes ? ctx->nodes.as<float4>() : nullptr,
-                                             use_nodes ? ctx->dltab.as<DepthLayer>() : nullptr);
+                                             use_nodes ? ctx->dltab.as<DepthLayer>() : nullptr,
+                                             ctx->nevals.as<unsigned long long>() + EV_WET);
   CK(cudaGetLastError());
   if (timing) CK(cudaEventRecord(ctx->ev[1], st));
   if (useprop) {
@@ -1931,12 +2008,12 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
   CK(cudaMemsetAsync(ctx->queue.p, 0, sizeof(unsigned int), st));
   CK(cudaMemsetAsync(ctx->retry_ctr.p, 0, 2 * sizeof(unsigned int), st));
   unsigned int* rctr = ctx->retry_ctr.as<unsigned int>();
-  ctx->launches += 2;
   RootsCall rc;
   rc.ncol = ncol;
   rc.nitems = nitems;
-  rc.scans = !useprop;
-  for (const ChainDesc& d : P.chains) rc.scans |= d.nmode > 1;
+  rc.load.scans = !useprop;
+  rc.load.reference = ctx->cfg.refine == 0;
+  for (const ChainDesc& d : P.chains) rc.load.add(d, P.periods.data() + d.t_off, ncol, Lmax);
   rc.order = P.d_order.as<int>();
   rc.chains = P.d_chains.as<ChainDesc>();
   rc.periods = P.d_periods.as<double>();
@@ -1957,7 +2034,8 @@ int run_device(swdk_ctx* ctx, int path, int nx, int ny, int nz, const float* d_v
   rc.rg = RaggedMap{nullptr, nullptr, 0, Lmax};
   rc.nodes = use_nodes ? ctx->nodes.as<float4>() : nullptr;
   rc.dl = ctx->dltab.as<DepthLayer>();
-  CK(launch_roots(rc, rblocks, ctx->nsm, ctx->cfg.block_roots > 0, st));
+  rc.wet = ctx->nevals.as<unsigned long long>() + EV_WET;
+  CK(launch_roots(rc, rblocks, ctx->nsm, ctx->cfg.block_roots > 0, &ctx->launches, st));
   if (timing) CK(cudaEventRecord(ctx->ev[2], st));
   if (!roots_only) {
     if (!ho) {
@@ -2471,7 +2549,10 @@ int swdk_surfdisp96_batch(swdk_ctx* ctx, int nmodel, int nlayer, const float* th
     CK(roots_occupancy(&per));
     ctx->coop_ready = true;
   }
-  if (const int G = coop_lanes(nmodel, ctx->nsm, true); G > 1) {
+  RootsLoad load;
+  load.layered = true;
+  load.add(cd, t, nmodel, nlayer);
+  if (const int G = coop_lanes(load, ctx->nsm, false); G > 1) {
     CK(ensure(ctx, ctx->queue, sizeof(unsigned int)));
     CK(cudaMemsetAsync(ctx->queue.p, 0, sizeof(unsigned int), st));
     const long long need = ((long long)nmodel * G + 127) / 128;
@@ -2817,7 +2898,7 @@ int ragged_enqueue(swdk_ragged* R, cudaStream_t st, bool timing) {
         R->info.as<ColInfo>() + M.col0, R->chainrule.as<float2>() + M.crs0,
         R->useprop ? R->nodefeat.as<float4>() + M.col0 * FEAT_NODES : nullptr,
         use_nodes ? R->nodes.as<float4>() + M.node0 : nullptr,
-        use_nodes ? R->dltab.as<DepthLayer>() + M.dl0 : nullptr);
+        use_nodes ? R->dltab.as<DepthLayer>() + M.dl0 : nullptr, R->nevals.as<unsigned long long>() + EV_WET);
     CK(cudaGetLastError());
   }
   if (timing) CK(cudaEventRecord(R->ev[1], st));
@@ -2841,12 +2922,15 @@ int ragged_enqueue(swdk_ragged* R, cudaStream_t st, bool timing) {
   const RaggedMap rg{R->d_blocks.as<RBlock>(), R->d_models.as<RModel>(), (int)R->blocks.size(), 0};
   const unsigned int rcap = (unsigned int)std::min<long long>(R->root_tot, 0x7fffffffLL);
   unsigned int* rctr = R->retry_ctr.as<unsigned int>();
-  R->launches += 2;
   RootsCall rc;
   rc.ncol = 0;
   rc.nitems = R->nitems;
-  rc.scans = !R->useprop;
-  for (const ChainDesc& d : R->chains) rc.scans |= d.nmode > 1;
+  rc.load.scans = !R->useprop;
+  rc.load.reference = cfg.refine == 0;
+  for (const RBlock& B : R->blocks) {
+    const ChainDesc& d = R->chains[B.chain];
+    rc.load.add(d, R->periods.data() + d.t_off, R->models[B.model].ncol, R->models[B.model].Lmax);
+  }
   rc.order = nullptr;
   rc.chains = R->d_chains.as<ChainDesc>();
   rc.periods = R->d_periods.as<double>();
@@ -2867,7 +2951,8 @@ int ragged_enqueue(swdk_ragged* R, cudaStream_t st, bool timing) {
   rc.rg = rg;
   rc.nodes = use_nodes ? R->nodes.as<float4>() : nullptr;
   rc.dl = R->dltab.as<DepthLayer>();
-  CK(launch_roots(rc, R->roots_blocks, R->nsm, cfg.block_roots > 0, st));
+  rc.wet = R->nevals.as<unsigned long long>() + EV_WET;
+  CK(launch_roots(rc, R->roots_blocks, R->nsm, cfg.block_roots > 0, &R->launches, st));
   if (timing) CK(cudaEventRecord(R->ev[2], st));
   if (R->path != 2) {
     using EigR = void (*)(const REBlock*, int, const RModel*, const float4*, const ColInfo*, const float2*,

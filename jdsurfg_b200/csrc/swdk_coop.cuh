@@ -272,6 +272,8 @@ struct CoopArgs {
   const float4* nodes;
   const DepthLayer* dl;
   int32_t* ierr_out;  // REF: the chains' ierr
+  const unsigned long long* gate;  // if given, the launch is for calls where (*gate != 0) == gate_on
+  int gate_on;
 };
 
 // The group's first lane: gives the chain its value, runs its state machine
@@ -410,6 +412,7 @@ __device__ __noinline__ int coop_step(CoopGroup& g, const CoopArgs& A, unsigned 
 template <int NORM>
 __global__ void __launch_bounds__(128, 3) k_roots_coop(const __grid_constant__ CoopArgs A) {
   const unsigned FULL = 0xffffffffu;
+  if (A.gate && (*A.gate != 0ull) != (A.gate_on != 0)) return;
   extern __shared__ __align__(16) unsigned char coop_sm[];
   __shared__ unsigned long long phase_ev[NPHASE_EV];
   __shared__ unsigned long long blk_ev[5];
