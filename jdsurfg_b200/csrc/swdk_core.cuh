@@ -427,15 +427,16 @@ SWDK_HD double rayleigh_fluid_top(const float4 ly, double wvno, double omega, do
   const double dpth = ly.x, rho = ly.w;
   const double xka = xmul(omega, recip((double)ly.y));
   const double Xa = xmul(xadd(wvno, xka), fabs(xadd(wvno, -xka)));
-  const double ir = rsqrt(Xa), r = xmul(Xa, ir), p = xmul(r, dpth);  // not used where X = 0
   double w, cosp;
   if (wvno < xka) {
+    const double ir = rsqrt(Xa), r = xmul(Xa, ir);
     double sp, cp;
-    sincos(p, &sp, &cp);
+    sincos(xmul(r, dpth), &sp, &cp);
     w = xmul(sp, ir); cosp = cp;
   } else if (wvno == xka) {
     cosp = 1.0; w = dpth;
   } else {
+    const double ir = rsqrt(Xa), r = xmul(Xa, ir), p = xmul(r, dpth);
     const double fac = (p < 16.0) ? exp(xmul(-2.0, p)) : 0.0;
     cosp = xmul(xadd(1.0, fac), 0.5);
     w = xmul(xmul(xadd(1.0, -fac), 0.5), ir);
