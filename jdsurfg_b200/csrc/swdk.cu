@@ -654,9 +654,8 @@ __device__ __forceinline__ int ragged_find(const T* tab, int n, long long key, l
 // (chains in `order`, Rayleigh first, columns consecutive) whenever their
 // current chain is finished, so lanes stay busy while long chains run.
 // queue[0] is the next item; the launch covers the GPU once.
-// Dynamic shared memory of k_roots_queue (128 threads): 55 KB,
-// above the 48 KB a launch gets without opting in; four blocks fit an SM's
-// 228 KB.
+// Dynamic shared memory of k_roots_queue (128 threads, 352 bytes each): 45 KB;
+// four blocks fit an SM's 228 KB.
 constexpr size_t ROOTS_SMEM = 128 * (sizeof(ChainState) + sizeof(ChainParams) + sizeof(ChainIO));
 
 #ifndef SWDK_ROOTS_MINB

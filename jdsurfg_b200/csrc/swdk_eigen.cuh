@@ -581,7 +581,8 @@ struct PassStore {
   }
 };
 constexpr int RAY_STORE = 6, LOVE_STORE = 3;
-// the same within the caller's frame
+// the same within the caller's frame (the host tests' passes; the kernels'
+// stores are PassStore)
 template <int N>
 struct LocalStore {
   double v[LMAX][N];

@@ -416,7 +416,8 @@ struct March {
     }
 
     // The same march as march() with the neighbours solved one by one from
-    // their own stencils (the per-lane work of march_coop), sequentially.
+    // their own stencils: the plain form that the host tests hold march()'s
+    // shared window against.  No kernel runs it.
     FM_HD void march_nb(bool refined, const PairGeo& g) {
         while (ntr > 0 && !overflow) {
             const FHeap root = heap[1];
@@ -444,11 +445,11 @@ struct March {
     // March, and the halves go through the same instructions (`on`: this half
     // takes part), so one instruction stream serves both.
     //
-    // An accepted node is a dependent chain of some hundred instructions at
-    // four cycles or more each, which is what bounds the march (a pair alone
-    // and 3040 pairs together take nearly the same time): the root, the
-    // stencils' loads, the sift-down, the trial times, up to four heap
-    // updates.  So the chain is kept short:
+    // An accepted node is a dependent chain, 1.7 us or 3300 cycles of a pair
+    // alone, which is what bounds the march (131 ms for one pair, 183 ms for
+    // 3040 together): the root, the sift-down, the trial times, up to four
+    // heap updates one after another, and the loads between them.  So the
+    // chain is kept short:
     //   * lane 4q + (a + 2b) of a half solves quadrant (a, b) of neighbour q
     //     with straight-line code;
     //   * the loads of the next root's stencils start one node ahead: the next
@@ -801,7 +802,7 @@ FM_HD void march_pair(const Grid& G, int p, int gp, const float* __restrict__ sr
                            const float* __restrict__ slwn, const float* __restrict__ risti_c,
                            const float* __restrict__ risti_r, const Scratch& S, unsigned int* __restrict__ n_overflow,
                            FHeap* hp, int smem_cap, int mode, int lane, unsigned mask) {
-    // mode 0: one lane, window march; 1: one lane, neighbours one by one;
+    // mode 0: one lane, window march; 1 (host tests): one lane, neighbours one by one;
     // 2 (device): half a warp (lane 0 .. 15, mask its lanes) marches the pair,
     // every lane holding the same state; the other half marches another pair
     // or none (mask 0: this half has none) and takes part in every step.

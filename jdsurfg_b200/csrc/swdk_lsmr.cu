@@ -82,8 +82,8 @@ __global__ void k_ls_partial(int64_t n, const double* __restrict__ a, double* __
   block_sum_store(s, part);
 }
 
-// the norm from the partial sums: which 0 -> beta, 1 -> alpha (only after a
-// step with beta > 0), 3 -> beta of the start (normb as well)
+// the start's norms from the partial sums: which 0 -> beta (normb as well),
+// 1 -> alpha (with beta > 0)
 __global__ void k_ls_norm(const double* __restrict__ part, LsmrState* __restrict__ st, int which) {
   if (st->done || (which == 1 && !(st->beta > 0.0))) return;
   __shared__ double sh[512];
@@ -98,8 +98,7 @@ __global__ void k_ls_norm(const double* __restrict__ part, LsmrState* __restrict
   if (threadIdx.x == 0) {
     const double nrm = sqrt(sh[0]);
     if (which == 1) st->alpha = nrm;
-    else st->beta = nrm;
-    if (which == 3) st->normb = nrm;
+    else st->beta = st->normb = nrm;
   }
 }
 
@@ -420,7 +419,7 @@ int swdk_lsmr_solve(swdk_lsmr* s, const double* d_b, double* d_x, double damp, d
   cudaMemsetAsync(d_x, 0, (size_t)n * sizeof(double), st);
   cudaMemsetAsync(s->hbar, 0, (size_t)n * sizeof(double), st);
   k_ls_partial<<<LS_PART, LS_THREADS, 0, st>>>(m, s->u, s->part, s->st, 0);
-  k_ls_norm<<<1, 512, 0, st>>>(s->part, s->st, 3);
+  k_ls_norm<<<1, 512, 0, st>>>(s->part, s->st, 0);
   k_ls_div<<<em, LS_THREADS, 0, st>>>(m, s->u, s->st, 0);
   k_ls_spmv<<<gn, LS_THREADS, 0, st>>>(n, s->trowptr, s->tidx, s->tval, s->u, s->v, s->st);
   k_ls_partial<<<LS_PART, LS_THREADS, 0, st>>>(n, s->v, s->part, s->st, 1);
