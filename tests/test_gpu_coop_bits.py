@@ -34,22 +34,27 @@ def test_layered_models_unrounded(iwave, mode, igr, nlayer, refine):
     eng.close()
 
 
-# 26 000 chains without proposals and 16 000 with: the last that groups of lanes search
-@pytest.mark.parametrize("ncol,waves,learned", [(13000, ("Lc", "Rc"), False), (8000, ("Rc", "Lc"), True),
-                                                (16001, ("Lc",), True)])
+# 32 lanes (6000 chains), 4 (9000), and 32 where the launch rule finds the
+# columns under water (6000); 592 blocks: one lane
+@pytest.mark.parametrize("ncol,waves,learned", [(3000, ("Lc", "Rc"), False), (4500, ("Rc", "Lc"), True),
+                                                (6000, ("Lc",), True)])
 def test_grid_chains_unrounded(ncol, waves, learned):
     import torch
+    from torch.profiler import ProfilerActivity, profile
     from jdsurfg_b200 import Engine, learn
     case = synth.make_case(ncol, 1, np.arange(6, dtype=np.float32) * 3.0, 2.5, 4.6, 0.08,
                            np.array([2.0, 6.0, 15.0, 40.0]), waves, 1, ncol, lvz_frac=0.2, water_frac=0.3)
     out = []
-    for kw in (dict(), dict(block_roots=592)):
+    for kw, kernel in ((dict(), "k_roots_coop"), (dict(block_roots=592), "k_roots_queue")):
         eng = Engine(sngl=False, **kw)
         nets = learn.load_proposals(eng) if learned else None
         eng.setup(case)
         dev = [None if case[k] is None else torch.from_numpy(case[k]).cuda() for k in ("vs", "vp", "rho")]
-        eng.roots_device(ncol, 1, case["nz"], *dev)
-        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+            eng.roots_device(ncol, 1, case["nz"], *dev)
+            torch.cuda.synchronize()
+        ran = {k for e in prof.events() for k in ("k_roots_coop", "k_roots_queue") if k in e.name}
+        assert ran == {kernel}
         out.append(eng.last_roots(ncol))
         del nets
         eng.close()
